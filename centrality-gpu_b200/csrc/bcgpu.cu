@@ -64,8 +64,15 @@ struct bc_plan {
   unsigned long long *counter = nullptr;
   // PLAIN
   unsigned long long *acc = nullptr;  // [n_packed][kAccDigits] fixed-point BC counters (folded into bc per launch)
-  bcg::PlainItem *items = nullptr;
+  bcg::PlainItem *items = nullptr;  // those of the per-source kernel
   int64_t n_items = 0;
+  // PLAIN plans: items of BCCs that fit shared memory run on the small-BCC
+  // kernels, the others on the per-source kernel. Before item j lie
+  // item_at[j] of the per-source kernel's items and src_at[j] entries of the
+  // small-BCC source list. Empty in other plans (every item per-source).
+  std::vector<int64_t> item_at, src_at;
+  int32_t *tsrc = nullptr;
+  int slots = 0;  // workspace slots of the per-source kernel; slot `slots` is the row export's
   int32_t *ws_i = nullptr, *epochs = nullptr;
   double *ws_f = nullptr;
   int64_t ws_n = 0;
@@ -297,7 +304,8 @@ constexpr int kBatchedMaxLevels = 96;
 // and so the eccentricity, are those of the sequential BFS.
 constexpr int32_t kParallelBfs = 1 << 16;
 
-int bcc_ecc0(const bc_bccs *B, int32_t b, std::vector<int32_t> &dist, std::vector<int32_t> &queue, bool parallel) {
+int bcc_ecc0(const bc_bccs *B, int32_t b, std::vector<int32_t> &dist, std::vector<int32_t> &queue, bool parallel,
+             bool *connected = nullptr) {
   const int64_t vo = B->vtx_off[b];
   const int32_t nb = (int32_t)(B->vtx_off[b + 1] - vo);
   dist.assign((size_t)nb, -1);
@@ -337,6 +345,7 @@ int bcc_ecc0(const bc_bccs *B, int32_t b, std::vector<int32_t> &dist, std::vecto
       if (dist[y] < 0) { dist[y] = dist[x] + 1; queue[tail++] = y; }
     }
   }
+  if (connected) *connected = tail == nb;
   return ecc;
 }
 
@@ -381,6 +390,41 @@ constexpr int64_t kTileItemsPerCta = 4;
 // eight per CTA); larger ones the CTA class (the CTA on one source).
 constexpr int64_t kTileWarpMaxVertices = 640;
 
+// Whether BCC b's arcs come in mirrored pairs, by a sum over the arcs of a
+// mixed (u, v) that pairs cancel: an undirected BCC always passes.
+bool mirrored(const bc_bccs *B, int32_t b) {
+  const int64_t vo = B->vtx_off[b], nb = B->vtx_off[b + 1] - vo;
+  uint64_t sum = 0;
+  for (int64_t u = 0; u < nb; ++u)
+    for (int64_t e = B->row[vo + u]; e < B->row[vo + u + 1]; ++e) {
+      const uint64_t v = (uint64_t)B->col[e], lo = std::min<uint64_t>(u, v), hi = std::max<uint64_t>(u, v);
+      uint64_t h = (lo << 32 | hi) * 0x9e3779b97f4a7c15ull;  // the splitmix64 finaliser
+      h = (h ^ (h >> 30)) * 0xbf58476d1ce4e5b9ull;
+      h = (h ^ (h >> 27)) * 0x94d049bb133111ebull;
+      h ^= h >> 31;
+      sum += (uint64_t)u < v ? h : (uint64_t)u > v ? 0 - h : 0;
+    }
+  return sum == 0;
+}
+
+// Whether the chains of BCC b are paths of the BCC: every chain vertex has
+// just its two chain neighbours. With mirrored arcs a BFS from a chain vertex
+// then gives the rows that the merge of the chain's ends gives.
+bool chains_are_paths(const bc_bccs *B, int32_t b) {
+  const int64_t vo = B->vtx_off[b];
+  for (int64_t c = B->chain_off[b]; c < B->chain_off[b + 1]; ++c) {
+    const int32_t st = B->chain_start[c], k = B->chain_len[c];
+    for (int32_t j = 0; j < k; ++j) {
+      const int32_t prev = j == 0 ? B->chain_l[c] : st + j - 1, next = j == k - 1 ? B->chain_r[c] : st + j + 1;
+      const int64_t e0 = B->row[vo + st + j], e1 = B->row[vo + st + j + 1];
+      if (e1 - e0 != 2) return false;
+      const int32_t x = B->col[e0], y = B->col[e0 + 1];
+      if (!((x == prev && y == next) || (x == next && y == prev))) return false;
+    }
+  }
+  return true;
+}
+
 // Small-BCC class of each BCC (-1: not in the schedule): BCCs off the
 // multi-source passes with at most opts.tile_max vertices whose CTA fits the
 // device's shared memory and whose path counts cannot overflow FP64 without
@@ -389,18 +433,22 @@ constexpr int64_t kTileWarpMaxVertices = 640;
 // (2 ecc(0) + 1) log2(maxdeg) <= 1000 keeps every count below 2^1000 (and the
 // levels below the CTA class's level table). Within a class, candidates are
 // taken smallest first while the launch's shared memory (sized by the class's
-// largest BCC and largest slice) still fits.
+// largest BCC and largest slice) still fits. PLAIN plans (strict) take no
+// limit from tile_max, and check what the bounds rest on -- a connected BCC,
+// mirrored arcs, chains that are paths of it -- since they must give what the
+// per-source kernel gives on any input.
 // The variant whose shared memory bounds a class's (the CTA class's largest
 // block has the largest work queue).
 int fit_cls(int c) { return c == bcg::kTileWarp ? c : bcg::kTileCta1024; }
 
 void route_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<char> &on, std::vector<int8_t> &cls,
-                 std::vector<int32_t> &ecc_of) {
+                 std::vector<int32_t> &ecc_of, bool strict = false) {
   cls.assign((size_t)B->n_bcc, -1);
   ecc_of.assign((size_t)B->n_bcc, -1);
   const size_t lim = bcg::tile_smem_limit(ctx->device);
   if (lim == 0) return;
-  const int64_t cap = std::min<int64_t>(ctx->opts.tile_max > 0 ? ctx->opts.tile_max : INT32_MAX, bcg::kTileMaxVertices);
+  const int64_t cap = std::min<int64_t>(ctx->opts.tile_max > 0 && !strict ? ctx->opts.tile_max : INT32_MAX,
+                                        bcg::kTileMaxVertices);
   std::vector<int64_t> bytes((size_t)B->n_bcc, 0);
   std::vector<int8_t> want((size_t)B->n_bcc, -1);
 #pragma omp parallel
@@ -417,8 +465,11 @@ void route_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<char> &on, std
       if (bcg::tile_smem_bytes(fit_cls(c), nb, bytes[b]) > lim) continue;
       int64_t maxdeg = 1;
       for (int64_t k = vo; k < vo + nb; ++k) maxdeg = std::max(maxdeg, B->row[k + 1] - B->row[k]);
-      const int ecc = bcc_ecc0(B, b, dist, queue, false);
+      if (strict && !(mirrored(B, b) && chains_are_paths(B, b))) continue;
+      bool connected = true;
+      const int ecc = bcc_ecc0(B, b, dist, queue, false, &connected);
       ecc_of[b] = ecc;
+      if (strict && !connected) continue;
       if ((2.0 * ecc + 1.0) * std::log2((double)std::max<int64_t>(maxdeg, 2)) <= 1000.0) want[b] = (int8_t)c;
     }
   }
@@ -447,9 +498,17 @@ void route_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<char> &on, std
 // groups' arrays and the slice fit, and the BCC fits that class's level
 // table); 512-thread CTAs at 2 per SM; a 1024-thread CTA of two groups; one
 // 1024-thread CTA per SM. Each bucket's items are contiguous.
+// With a source list (PLAIN plans: src, each BCC's sources from list[b] on)
+// the items hold places in it, and contributions go straight into the
+// fixed-point counters, so that BC is bit for bit what the per-source kernel
+// gives.
 int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, const std::vector<int32_t> &ecc_of,
-                bc_plan *p) {
+                bc_plan *p, const std::vector<int32_t> *src = nullptr, const std::vector<int64_t> *list = nullptr) {
   int rc = BCGPU_OK;
+  auto first_of = [&](int32_t b) { return src ? (*list)[(size_t)b] : 0; };
+  auto sources_of = [&](int32_t b) {
+    return src ? (*list)[(size_t)b + 1] - (*list)[(size_t)b] : B->vtx_off[b + 1] - B->vtx_off[b];
+  };
   std::vector<int64_t> off((size_t)B->n_bcc, -1);
   std::vector<int32_t> size((size_t)B->n_bcc, 0);
   std::vector<int8_t> bucket((size_t)B->n_bcc, -1);
@@ -504,7 +563,7 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
       const int64_t nb = B->vtx_off[b + 1] - B->vtx_off[b];
       nmax = std::max(nmax, nb);
       smax = std::max<int64_t>(smax, size[b]);
-      sources += nb;
+      sources += sources_of(b);
     }
     if (sources == 0) continue;
     T.nmax = (int32_t)nmax;
@@ -521,11 +580,11 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
         floor_items, std::min<int64_t>(kTileItemSources, sources / ((int64_t)T.grid * kTileItemsPerCta)));
     for (int32_t b = 0; b < B->n_bcc; ++b) {
       if (bucket[b] != k) continue;
-      const int64_t nb = B->vtx_off[b + 1] - B->vtx_off[b];
+      const int64_t l0 = first_of(b), l1 = l0 + sources_of(b);
       off[b] = total;
       total += size[b];
-      for (int32_t s0 = 0; s0 < nb; s0 += per_item)
-        p->h_titems.push_back({b, s0, (int32_t)std::min<int64_t>(nb, s0 + per_item), 0});
+      for (int64_t s0 = l0; s0 < l1; s0 += per_item)
+        p->h_titems.push_back({b, (int32_t)s0, (int32_t)std::min<int64_t>(l1, s0 + per_item), 0});
     }
     T.i1 = (int64_t)p->h_titems.size();
     if (T.cls == bcg::kTileWarp) p->tcap = nmax + 2;
@@ -534,9 +593,9 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
   // slices: local row offsets (uint16 when narrow, else int32), neighbours
   // (uint16), 16-byte aligned parts; bit 0 of a narrow slice's offset set
   std::vector<unsigned char> blob((size_t)std::max<int64_t>(total, 16), 0);
-#pragma omp parallel for schedule(dynamic, 16)
+#pragma omp parallel for schedule(dynamic, 16) if (B->n_bcc > 16)
   for (int32_t b = 0; b < B->n_bcc; ++b) {
-    if (cls[b] < 0) continue;
+    if (off[b] < 0) continue;  // no item
     const int64_t vo = B->vtx_off[b], nb = B->vtx_off[b + 1] - vo, e0 = B->row[vo];
     const int64_t arcs = B->row[vo + nb] - e0;
     const bool narrow = bcg::TileSlice::narrow(arcs);
@@ -550,7 +609,7 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
   }
   std::vector<int64_t> off_flag(off);  // what the kernels read: offset | narrow
   for (int32_t b = 0; b < B->n_bcc; ++b) {
-    if (cls[b] < 0) continue;
+    if (off[b] < 0) continue;
     const int64_t vo = B->vtx_off[b], nb = B->vtx_off[b + 1] - vo;
     if (bcg::TileSlice::narrow(B->row[vo + nb] - B->row[vo])) off_flag[b] |= 1;
   }
@@ -566,9 +625,11 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
       (rc = upload(p, &p->slice_off, off_flag.data(), B->n_bcc)) ||
       (rc = upload(p, &p->slice_bytes, size.data(), B->n_bcc)) ||
       (rc = upload(p, &p->titems, p->h_titems.data(), p->n_titems)) || (rc = dalloc(p, &p->tws_lv, slots * p->tcap)) ||
-      (rc = dalloc(p, &p->tws_P, p_rows * std::max<int64_t>(p->tcap_P, 1))) ||
+      (rc = src ? upload(p, &p->tsrc, src->data(), (int64_t)src->size())
+                : dalloc(p, &p->tws_P, p_rows * std::max<int64_t>(p->tcap_P, 1))) ||
       (rc = alloc_acc(p, B->n_packed)))
     return rc;
+  if (src) return BCGPU_OK;  // the plan's units are its per-source items
   for (const auto &it : p->h_titems) {
     const int64_t vo = B->vtx_off[it.bcc], nb = B->vtx_off[it.bcc + 1] - vo;
     const int64_t arcs = B->row[vo + nb] - B->row[vo];
@@ -770,8 +831,41 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
       p->unit_aux.push_back(p->unit_aux.back() + aux);
       p->unit_visits.push_back(p->unit_visits.back() + src * nb);
     }
+    // PLAIN: items of the BCCs that fit shared memory go to the small-BCC
+    // kernels (sources of an item: its own vertex, then its chains'), unless
+    // the caller asked for a rescaling threshold, which only the per-source
+    // kernel applies. Rows in shared memory instead of L2, and a BFS per chain
+    // vertex instead of a merge and a double listing: a chain-endpoint call on
+    // a BCC of 1,494 vertices went from 1.95 to 0.66 ms, 1,194 sources.
+    if (p->mode == BCGPU_MODE_PLAIN && ctx->opts.rescale_exp == 0 && p->n_items > 0 &&
+        p->unit_sources.back() < INT32_MAX) {
+      std::vector<int32_t> plain_ecc;
+      route_tiles(ctx, B, std::vector<char>((size_t)B->n_bcc, 0), tile, plain_ecc, true);
+      std::vector<int32_t> src;
+      std::vector<int64_t> list((size_t)B->n_bcc + 1, 0);
+      std::vector<bcg::PlainItem> rest;
+      for (const auto &it : items) {
+        p->item_at.push_back((int64_t)rest.size());
+        p->src_at.push_back((int64_t)src.size());
+        if (tile[it.bcc] < 0) {
+          rest.push_back(it);
+          continue;
+        }
+        if (it.own) src.push_back(it.src);
+        for (int32_t c = it.c0; c < it.c1; ++c)
+          for (int32_t k = 0; k < B->chain_len[c]; ++k) src.push_back(B->chain_start[c] + k);
+        list[(size_t)it.bcc + 1] = (int64_t)src.size();
+      }
+      p->item_at.push_back((int64_t)rest.size());
+      p->src_at.push_back((int64_t)src.size());
+      for (int32_t b = 0; b < B->n_bcc; ++b) list[(size_t)b + 1] = std::max(list[(size_t)b + 1], list[(size_t)b]);
+      if (!src.empty() && (rc = build_tiles(ctx, B, tile, plain_ecc, p, &src, &list))) return bail(rc);
+      p->h_items = std::move(items);
+      items = std::move(rest);
+    } else {
+      p->h_items = items;
+    }
     if ((rc = upload(p, &p->items, items.data(), (int64_t)items.size()))) return bail(rc);
-    p->h_items = items;
     p->ws_n = (p->mode == BCGPU_MODE_PLAIN ? nb_max : nb_plain) + 2;
     if ((rc = alloc_acc(p, B->n_packed))) return bail(rc);
     const int64_t per_slot = p->ws_n * (bcg::kWsIntRows * 4 + bcg::kWsDblRows * 8);
@@ -790,7 +884,8 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
       if (grid == want) break;
     }
     p->grid = std::max(1, grid);
-    const int64_t slots = p->grid + 1;  // + the row-export slot
+    p->slots = (int)std::min<int64_t>(p->grid, (int64_t)items.size());  // items take a slot each
+    const int64_t slots = p->slots + 1;  // + the row-export slot
     if ((rc = dalloc(p, &p->ws_i, slots * bcg::kWsIntRows * p->ws_n)) ||
         (rc = dalloc(p, &p->ws_f, slots * bcg::kWsDblRows * p->ws_n)) || (rc = dalloc(p, &p->epochs, 2 * slots)))
       return bail(rc);
@@ -1111,19 +1206,45 @@ bcg::PlainArgs plain_args(const bc_plan *p) {
   a.row = p->row; a.col = p->col; a.reach = p->reach; a.vtx_off = p->vtx_off;
   a.chain_start = p->chain_start; a.chain_len = p->chain_len; a.chain_l = p->chain_l; a.chain_r = p->chain_r;
   a.items = p->items; a.next_item = p->counter; a.acc = p->acc;
-  a.ws_i = p->ws_i; a.ws_f = p->ws_f; a.ws_n = p->ws_n; a.epochs = p->epochs; a.rows_slot = p->grid;
+  a.ws_i = p->ws_i; a.ws_f = p->ws_f; a.ws_n = p->ws_n; a.epochs = p->epochs; a.rows_slot = p->slots;
   a.rescale_exp = p->ctx->opts.rescale_exp > 0 ? p->ctx->opts.rescale_exp : 900;
   a.err = p->err;
   return a;
+}
+
+// The small-BCC launches of items [t0, t1), of which those that hold places
+// of the source list only run [lo, hi).
+int enqueue_tiles(bc_plan *p, int64_t t0, int64_t t1, int32_t lo, int32_t hi, int *launches) {
+  bc_ctx *ctx = p->ctx;
+  for (const bc_plan::TileLaunch &T : p->tl) {
+    int64_t j0 = std::max(t0, T.i0), j1 = std::min(t1, T.i1);
+    if (p->tsrc) {  // a launch's items hold rising places
+      while (j0 < j1 && p->h_titems[(size_t)j0].s1 <= lo) ++j0;
+      while (j1 > j0 && p->h_titems[(size_t)j1 - 1].s0 >= hi) --j1;
+    }
+    if (j1 <= j0) continue;
+    CK(ctx, cudaMemsetAsync(p->counter, 0, sizeof(unsigned long long), ctx->stream));
+    bcg::TileArgs a{};
+    a.vtx_off = p->vtx_off; a.reach = p->reach; a.slices = p->slices; a.slice_off = p->slice_off;
+    a.slice_bytes = p->slice_bytes; a.items = p->titems; a.item_begin = j0; a.item_end = j1;
+    a.src = p->tsrc; a.src_lo = lo; a.src_hi = hi;
+    a.next_item = p->counter; a.acc = p->acc; a.ws_lv = p->tws_lv; a.cap = p->tcap; a.nmax = T.nmax;
+    a.ws_P = p->tws_P; a.cap_P = p->tcap_P;
+    a.slice_max = T.slice_max; a.wait_ns = wait_ns(ctx); a.err = p->err;
+    CK(ctx, bcg::launch_tile(T.cls, a, (int)std::min<int64_t>(T.grid, j1 - j0), T.smem, ctx->stream));
+    ++*launches;
+  }
+  return BCGPU_OK;
 }
 
 // The device work of units [begin, end) (range already checked), enqueued on
 // the context's stream: the multi-source passes, then the per-source items.
 int enqueue_units(bc_plan *p, int64_t begin, int64_t end, int *launches) {
   bc_ctx *ctx = p->ctx;
+  int rc = BCGPU_OK;
   if (p->bp && begin < p->n_bat) {  // multi-source passes
     std::string msg;
-    int rc = bcg::batched_run(p->bp, begin, std::min(end, p->n_bat), ctx->stream, launches, &msg);
+    rc = bcg::batched_run(p->bp, begin, std::min(end, p->n_bat), ctx->stream, launches, &msg);
     if (rc) return fail(ctx, rc, "batched run: " + msg);
   }
   const int64_t i0 = std::max(begin, p->n_bat) - p->n_bat, i1 = std::min(end - p->n_bat, p->n_items);
@@ -1139,15 +1260,24 @@ int enqueue_units(bc_plan *p, int64_t begin, int64_t end, int *launches) {
       b0 = std::min(b0, p->h_items[j].bcc);
       b1 = std::max(b1, p->h_items[j].bcc);
     }
-    CK(ctx, cudaMemsetAsync(p->counter, 0, sizeof(unsigned long long), ctx->stream));
-    bcg::PlainArgs a = plain_args(p);
-    a.item_begin = j0; a.item_end = j1;
-    const int grid = (int)std::min<int64_t>(p->grid, j1 - j0);
-    CK(ctx, bcg::launch_plain(a, p->block, grid, ctx->stream));
+    const bool split = !p->item_at.empty();  // a PLAIN plan with small BCCs among its items
+    const int64_t k0 = split ? p->item_at[(size_t)j0] : j0, k1 = split ? p->item_at[(size_t)j1] : j1;
+    if (k1 > k0) {
+      CK(ctx, cudaMemsetAsync(p->counter, 0, sizeof(unsigned long long), ctx->stream));
+      bcg::PlainArgs a = plain_args(p);
+      a.item_begin = k0; a.item_end = k1;
+      const int grid = (int)std::min<int64_t>(p->slots, k1 - k0);
+      CK(ctx, bcg::launch_plain(a, p->block, grid, ctx->stream));
+      ++*launches;
+    }
+    if (split && p->src_at[(size_t)j1] > p->src_at[(size_t)j0] &&
+        (rc = enqueue_tiles(p, 0, p->n_titems, (int32_t)p->src_at[(size_t)j0], (int32_t)p->src_at[(size_t)j1], launches)))
+      return rc;
     CK(ctx, bcg::launch_fold(p->acc, p->bc, p->h_vtx_off[b0], p->h_vtx_off[b1 + 1], ctx->stream));
-    *launches += 2;
+    ++*launches;
     j0 = j1;
   }
+  if (p->tsrc) return BCGPU_OK;
   // small-BCC items: one launch per class (each BCC's sources are far fewer
   // than kAccMaxAdds), then one fold over the BCCs they touched
   const int64_t t0 = std::max(begin, p->n_bat + p->n_items) - p->n_bat - p->n_items;
@@ -1158,19 +1288,7 @@ int enqueue_units(bc_plan *p, int64_t begin, int64_t end, int *launches) {
       b0 = std::min(b0, p->h_titems[j].bcc);
       b1 = std::max(b1, p->h_titems[j].bcc);
     }
-    for (const bc_plan::TileLaunch &T : p->tl) {
-      const int64_t j0 = std::max(t0, T.i0), j1 = std::min(t1, T.i1);
-      if (j1 <= j0) continue;
-      CK(ctx, cudaMemsetAsync(p->counter, 0, sizeof(unsigned long long), ctx->stream));
-      bcg::TileArgs a{};
-      a.vtx_off = p->vtx_off; a.reach = p->reach; a.slices = p->slices; a.slice_off = p->slice_off;
-      a.slice_bytes = p->slice_bytes; a.items = p->titems; a.item_begin = j0; a.item_end = j1;
-      a.next_item = p->counter; a.acc = p->acc; a.ws_lv = p->tws_lv; a.cap = p->tcap; a.nmax = T.nmax;
-      a.ws_P = p->tws_P; a.cap_P = p->tcap_P;
-      a.slice_max = T.slice_max; a.wait_ns = wait_ns(ctx); a.err = p->err;
-      CK(ctx, bcg::launch_tile(T.cls, a, (int)std::min<int64_t>(T.grid, j1 - j0), T.smem, ctx->stream));
-      ++*launches;
-    }
+    if ((rc = enqueue_tiles(p, t0, t1, 0, 0, launches))) return rc;
     CK(ctx, bcg::launch_fold(p->acc, p->bc, p->h_vtx_off[b0], p->h_vtx_off[b1 + 1], ctx->stream));
     ++*launches;
   }

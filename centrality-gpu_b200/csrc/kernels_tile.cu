@@ -163,7 +163,11 @@ __device__ bool next_item(const TileArgs &a, Ctl &ctl, unsigned char *slice, uns
   vo = a.vtx_off[it.bcc];
   nb = (int32_t)(a.vtx_off[it.bcc + 1] - vo);
   const int64_t soff = a.slice_off[it.bcc] & ~int64_t(15);
-  if (nb > a.nmax || a.slice_off[it.bcc] < 0 || it.s0 < 0 || it.s1 > nb) {  // uniform over the CTA
+  if (a.src) {  // places in the source list, clipped to the launch's range
+    it.s0 = max(it.s0, a.src_lo);
+    it.s1 = min(it.s1, a.src_hi);
+  }
+  if (nb > a.nmax || a.slice_off[it.bcc] < 0 || it.s0 < 0 || (!a.src && it.s1 > nb)) {  // uniform over the CTA
     if (tid == 0) set_err(a.err, kDevBadItem);
     return false;
   }
@@ -184,6 +188,9 @@ __device__ bool next_item(const TileArgs &a, Ctl &ctl, unsigned char *slice, uns
   }
   return true;
 }
+
+// Local id of source k of an item.
+__device__ __forceinline__ int32_t source_of(const TileArgs &a, int32_t k) { return a.src ? __ldg(a.src + k) : k; }
 
 __device__ __forceinline__ View view_of(const TileArgs &a, const unsigned char *slice, int32_t nb, int64_t vo,
                                         int32_t bcc) {
@@ -406,8 +413,8 @@ __global__ void __launch_bounds__(kThreads, 1) tile_warp_kernel(TileArgs a) {
       int k = 0;
       if (lane == 0) k = atomicAdd(&ctl.next, 1);
       k = __shfl_sync(0xffffffffu, k, 0);
-      const int32_t s = it.s0 + k;
-      if (s >= it.s1) break;
+      if (it.s0 + k >= it.s1) break;
+      const int32_t s = source_of(a, it.s0 + k);
       const int nlev = warp_bfs(g, nb, s, d, sq, S, lv, &ctl.tails[warp], lane);
       warp_sweep(g, nlev, d, sq, S, lv, (double)__ldg(g.rch + s) + 1.0, cnt, lane, a.err);
     }
@@ -510,12 +517,20 @@ __device__ int cta_bfs(const View &g, int32_t nb, int32_t s, int16_t *d, double 
   return lev + 1;
 }
 
+// One source's contribution c to vertex w: to the group's FP64 row P (one
+// writer per vertex and source), or straight into the BCC's fixed-point
+// counters when there is no row.
+__device__ __forceinline__ void contribute(double *P, unsigned long long *acc, int32_t w, double c, int *err) {
+  if (P) P[w] += c;
+  else if (c != 0.0) acc_add(acc + (int64_t)kAccDigits * w, c, err);
+}
+
 // Dependency sweep of one group, two group barriers per level as in cta_bfs;
-// contributions go to the group's FP64 row P, each vertex written by one
-// thread.
+// each vertex's contribution is made by one thread.
 template <int kBlock, int kGroup>
 __device__ void cta_sweep(const View &g, int nlev, const int16_t *d, double *sq, const uint16_t *S, const int32_t *lv,
-                          int32_t *q, int *nq, double wsrc, double *P, int *err, int grp, int tid) {
+                          int32_t *q, int *nq, double wsrc, double *P, unsigned long long *acc, int *err, int grp,
+                          int tid) {
   using L = CtaLayout<kBlock, kGroup>;
   constexpr int kWarps = kGroup / 32;
   const int lane = tid & 31, warp = tid >> 5;
@@ -537,7 +552,7 @@ __device__ void cta_sweep(const View &g, int nlev, const int16_t *d, double *sq,
         e1 = g.row(w + 1);
       }
       const bool big = e1 - e0 > kLaneDeg;
-      if (w >= 0 && !big) P[w] += finish(g, w, push_row(g, e0, e1, d, sq, dsucc), sq, err) * wsrc;
+      if (w >= 0 && !big) contribute(P, acc, w, finish(g, w, push_row(g, e0, e1, d, sq, dsucc), sq, err) * wsrc, err);
       bool mine = false;
       if (w >= 0 && big) {
         const int pos = atomicAdd(nql, 1);
@@ -550,7 +565,7 @@ __device__ void cta_sweep(const View &g, int nlev, const int16_t *d, double *sq,
         over &= over - 1;
         const int32_t wj = __shfl_sync(0xffffffffu, w, j);
         const double sum = push_row_warp(g, g.row(wj), g.row(wj + 1), d, sq, dsucc, lane);
-        if (lane == 0) P[wj] += finish(g, wj, sum, sq, err) * wsrc;
+        if (lane == 0) contribute(P, acc, wj, finish(g, wj, sum, sq, err) * wsrc, err);
       }
     }
     L::sync(grp);
@@ -558,7 +573,7 @@ __device__ void cta_sweep(const View &g, int nlev, const int16_t *d, double *sq,
     for (int k = warp; k < nlong; k += kWarps) {
       const int32_t w = q[k];
       const double sum = push_row_warp(g, g.row(w), g.row(w + 1), d, sq, dsucc, lane);
-      if (lane == 0) P[w] += finish(g, w, sum, sq, err) * wsrc;
+      if (lane == 0) contribute(P, acc, w, finish(g, w, sum, sq, err) * wsrc, err);
     }
     L::sync(grp);
   }
@@ -577,7 +592,8 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) tile_cta_kernel(TileArg
   Ctl &ctl = *reinterpret_cast<Ctl *>(s_raw);
   const int grp = threadIdx.x / kGroup, gtid = threadIdx.x % kGroup;
   unsigned char *mine = s_raw + L::group(grp, nmax);
-  double *P = a.ws_P + ((int64_t)blockIdx.x * L::kG + grp) * a.cap_P;  // the group's FP64 row (global, L2-resident)
+  // the group's FP64 row (global, L2-resident), if the launch has them
+  double *P = a.ws_P ? a.ws_P + ((int64_t)blockIdx.x * L::kG + grp) * a.cap_P : nullptr;
   double *sq = reinterpret_cast<double *>(mine);
   int16_t *d = reinterpret_cast<int16_t *>(mine + L::d(nmax));
   uint16_t *S = reinterpret_cast<uint16_t *>(mine + L::S(nmax));
@@ -596,17 +612,21 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) tile_cta_kernel(TileArg
   int64_t vo;
   int32_t nb;
   while (next_item(a, ctl, slice, phase, it, vo, nb)) {
-    for (int v = gtid; v < nb; v += kGroup) P[v] = 0.0;
+    if (P)
+      for (int v = gtid; v < nb; v += kGroup) P[v] = 0.0;
     __syncthreads();
     if (tid == 0) ctl.bcc = it.bcc;  // read again only after the next barrier
     const View g = view_of(a, slice, nb, vo, it.bcc);
-    for (int32_t s = it.s0 + grp; s < it.s1; s += L::kG) {  // the group's sources in order: P's sums are fixed
+    unsigned long long *acc = a.acc + (int64_t)kAccDigits * vo;
+    for (int32_t k = it.s0 + grp; k < it.s1; k += L::kG) {  // the group's sources in order: P's sums are fixed
+      const int32_t s = source_of(a, k);
       const int nlev = cta_bfs<kBlock, kGroup>(g, nb, s, d, sq, S, lv, q, cnt, nq, a.err, grp, gtid);
       if (nlev < 0) break;
-      cta_sweep<kBlock, kGroup>(g, nlev, d, sq, S, lv, q, nq, (double)__ldg(g.rch + s) + 1.0, P, a.err, grp, gtid);
+      cta_sweep<kBlock, kGroup>(g, nlev, d, sq, S, lv, q, nq, (double)__ldg(g.rch + s) + 1.0, P, acc, a.err, grp,
+                                gtid);
     }
     __syncthreads();
-    unsigned long long *acc = a.acc + (int64_t)kAccDigits * vo;
+    if (!P) continue;  // uniform over the grid
     for (int v = gtid; v < nb; v += kGroup)
       if (P[v] != 0.0) acc_add(acc + (int64_t)kAccDigits * v, P[v], a.err);
   }

@@ -13,7 +13,8 @@
 
 namespace bcg {
 
-// Sources [s0, s1) (local ids) of BCC bcc.
+// Sources [s0, s1) of BCC bcc: local ids, or places in the plan's source list
+// (TileArgs::src).
 struct TileItem {
   int32_t bcc, s0, s1, pad;
 };
@@ -56,11 +57,14 @@ struct TileArgs {
   const int32_t *slice_bytes;    // [n_bcc] its size (TileSlice::bytes)
   const TileItem *items;
   int64_t item_begin, item_end;
+  const int32_t *src;             // source list (local ids) the items index, or null: items hold local ids
+  int32_t src_lo, src_hi;         // with a list: only its places in [src_lo, src_hi) run (items are clipped to it)
   unsigned long long *next_item;  // zeroed before each launch
   unsigned long long *acc;        // [n_packed][kAccDigits] fixed-point BC counters (plain.h)
   int32_t *ws_lv;                 // warp class: level offsets per warp slot ([slots][cap])
   int64_t cap;                    // per-slot row capacity (>= largest BCC of the class + 2)
-  double *ws_P;                   // CTA class: FP64 partial BC row per source group ([grid * groups][cap_P])
+  double *ws_P;                   // CTA class: FP64 partial BC row per source group ([grid * groups][cap_P]); null:
+                                  // every contribution goes straight into the counters (PLAIN plans)
   int64_t cap_P;
   int32_t nmax;                   // largest BCC of the launch (shared-memory rows are sized for it)
   int32_t slice_max;              // largest slice in bytes
