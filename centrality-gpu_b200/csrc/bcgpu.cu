@@ -9,6 +9,7 @@
 #include "bcgpu.h"
 #include "batched.h"
 #include "common.cuh"
+#include "core.h"
 #include "internal.h"
 #include "plain.h"
 #include "tile.h"
@@ -66,12 +67,16 @@ struct bc_plan {
   unsigned long long *acc = nullptr;  // [n_packed][kAccDigits] fixed-point BC counters (folded into bc per launch)
   bcg::PlainItem *items = nullptr;  // those of the per-source kernel
   int64_t n_items = 0;
-  // PLAIN plans: items of BCCs that fit shared memory run on the small-BCC
-  // kernels, the others on the per-source kernel. Before item j lie
-  // item_at[j] of the per-source kernel's items and src_at[j] entries of the
-  // small-BCC source list. Empty in other plans (every item per-source).
-  std::vector<int64_t> item_at, src_at;
+  // Per-source items run on one of three kernels, by BCC: in PLAIN plans the
+  // small-BCC kernels where the BCC fits shared memory; else the contracted
+  // per-source kernel (core.h); else, for what that one does not take, the
+  // whole-BCC per-source kernel. Before item j lie src_at[j] entries of the
+  // small-BCC source list, core_at[j] of the contracted kernel's and
+  // item_at[j] items of the whole-BCC kernel.
+  std::vector<int64_t> src_at, core_at, item_at;
   int32_t *tsrc = nullptr;
+  bcg::CoreArgs core{};
+  int core_slots = 0, core_block = 256, core_grid = 0;
   int slots = 0;  // workspace slots of the per-source kernel; slot `slots` is the row export's
   int32_t *ws_i = nullptr, *epochs = nullptr;
   double *ws_f = nullptr;
@@ -305,7 +310,7 @@ constexpr int kBatchedMaxLevels = 96;
 constexpr int32_t kParallelBfs = 1 << 16;
 
 int bcc_ecc0(const bc_bccs *B, int32_t b, std::vector<int32_t> &dist, std::vector<int32_t> &queue, bool parallel,
-             bool *connected = nullptr) {
+             bool *connected) {
   const int64_t vo = B->vtx_off[b];
   const int32_t nb = (int32_t)(B->vtx_off[b + 1] - vo);
   dist.assign((size_t)nb, -1);
@@ -313,6 +318,7 @@ int bcc_ecc0(const bc_bccs *B, int32_t b, std::vector<int32_t> &dist, std::vecto
   if (parallel) {
     std::vector<int32_t> frontier{0}, next;
     int lev = 0;
+    size_t reached = 1;
     while (true) {
       next.clear();
 #pragma omp parallel
@@ -329,7 +335,11 @@ int bcc_ecc0(const bc_bccs *B, int32_t b, std::vector<int32_t> &dist, std::vecto
 #pragma omp critical
         next.insert(next.end(), mine.begin(), mine.end());
       }
-      if (next.empty()) return lev;
+      if (next.empty()) {
+        *connected = reached == (size_t)nb;
+        return lev;
+      }
+      reached += next.size();
       frontier.swap(next);
       ++lev;
     }
@@ -345,7 +355,7 @@ int bcc_ecc0(const bc_bccs *B, int32_t b, std::vector<int32_t> &dist, std::vecto
       if (dist[y] < 0) { dist[y] = dist[x] + 1; queue[tail++] = y; }
     }
   }
-  if (connected) *connected = tail == nb;
+  *connected = tail == nb;
   return ecc;
 }
 
@@ -395,6 +405,7 @@ constexpr int64_t kTileWarpMaxVertices = 640;
 bool mirrored(const bc_bccs *B, int32_t b) {
   const int64_t vo = B->vtx_off[b], nb = B->vtx_off[b + 1] - vo;
   uint64_t sum = 0;
+#pragma omp parallel for schedule(static) reduction(+ : sum) if (nb >= kParallelBfs)
   for (int64_t u = 0; u < nb; ++u)
     for (int64_t e = B->row[vo + u]; e < B->row[vo + u + 1]; ++e) {
       const uint64_t v = (uint64_t)B->col[e], lo = std::min<uint64_t>(u, v), hi = std::max<uint64_t>(u, v);
@@ -407,17 +418,20 @@ bool mirrored(const bc_bccs *B, int32_t b) {
   return sum == 0;
 }
 
-// Whether the chains of BCC b are paths of the BCC: every chain vertex has
+// Whether the chains of BCC b are paths of the BCC between different ends:
+// every chain vertex is on one chain (validate() has counted them) and has
 // just its two chain neighbours. With mirrored arcs a BFS from a chain vertex
 // then gives the rows that the merge of the chain's ends gives.
 bool chains_are_paths(const bc_bccs *B, int32_t b) {
   const int64_t vo = B->vtx_off[b];
+  std::vector<char> held((size_t)(B->vtx_off[b + 1] - vo), 0);
   for (int64_t c = B->chain_off[b]; c < B->chain_off[b + 1]; ++c) {
     const int32_t st = B->chain_start[c], k = B->chain_len[c];
+    if (B->chain_l[c] == B->chain_r[c]) return false;
     for (int32_t j = 0; j < k; ++j) {
       const int32_t prev = j == 0 ? B->chain_l[c] : st + j - 1, next = j == k - 1 ? B->chain_r[c] : st + j + 1;
       const int64_t e0 = B->row[vo + st + j], e1 = B->row[vo + st + j + 1];
-      if (e1 - e0 != 2) return false;
+      if (e1 - e0 != 2 || held[(size_t)(st + j)]++) return false;
       const int32_t x = B->col[e0], y = B->col[e0 + 1];
       if (!((x == prev && y == next) || (x == next && y == prev))) return false;
     }
@@ -489,6 +503,25 @@ void route_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<char> &on, std
       cls[b] = (int8_t)c;
     }
   }
+}
+
+// Shared memory for a bit per core vertex at most (a CTA of 512 threads needs
+// 28 KB more): cores of up to 1.5 million vertices.
+constexpr int64_t kCoreBits = 190 * 1024;
+
+// Whether the contracted per-source kernel takes BCC b, by its shape: what
+// mirrored(), chains_are_paths() and a BFS say (the kernel's level tables, its
+// closed forms and a chain source's two ways into the core rest on them), and
+// chains short enough for its ring of buckets. *ecc: as known, or -1.
+bool core_takes(const bc_bccs *B, int32_t b, std::vector<int32_t> &dist, std::vector<int32_t> &queue, int32_t *ecc,
+                bool connected) {
+  const int64_t vo = B->vtx_off[b], nb = B->vtx_off[b + 1] - vo;
+  if (B->row[vo + nb] - B->row[vo] > INT32_MAX || B->n_chains >= 1 << 29) return false;
+  for (int64_t c = B->chain_off[b]; c < B->chain_off[b + 1]; ++c)
+    if (B->chain_len[c] > bcg::kCoreMaxChain) return false;
+  if (!mirrored(B, b) || !chains_are_paths(B, b)) return false;
+  if (*ecc < 0) *ecc = bcc_ecc0(B, b, dist, queue, nb >= kParallelBfs, &connected);
+  return connected;
 }
 
 // Work items, staged slices and warp workspace of the small-BCC schedule.
@@ -643,6 +676,48 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
   return BCGPU_OK;
 }
 
+// The contracted per-source kernel's tables (filled on the device), source
+// list and workspace, for the BCCs with on[b] set.
+int build_core(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &on, const std::vector<bcg::CoreSource> &src,
+               bc_plan *p) {
+  int rc = BCGPU_OK;
+  bcg::CoreArgs &a = p->core;
+  bcg::CoreRow *rows = nullptr;
+  int32_t *n_plain = nullptr, *xcol = nullptr, *xk = nullptr, *xcid = nullptr, *vchain = nullptr;
+  int64_t *chain_off = nullptr, *row_off = nullptr;
+  std::vector<int64_t> off((size_t)B->n_bcc, 0);
+  int64_t ncore = 0;
+  for (int32_t b = 0; b < B->n_bcc; ++b) {
+    off[(size_t)b] = ncore;
+    if (on[(size_t)b]) ncore += B->n_plain[b];
+  }
+  int8_t *d_on = nullptr;
+  int4 *ctab = nullptr;
+  bcg::CoreSource *list = nullptr;
+  if ((rc = upload(p, &n_plain, B->n_plain, B->n_bcc)) || (rc = upload(p, &chain_off, B->chain_off, B->n_bcc + 1)) ||
+      (rc = upload(p, &d_on, on.data(), B->n_bcc)) || (rc = upload(p, &list, src.data(), (int64_t)src.size())) ||
+      (rc = upload(p, &row_off, off.data(), B->n_bcc)) || (rc = dalloc(p, &rows, ncore)) || (rc = dalloc(p, &xcol, B->n_arcs)) || (rc = dalloc(p, &xk, B->n_arcs)) ||
+      (rc = dalloc(p, &xcid, B->n_arcs)) || (rc = dalloc(p, &ctab, B->n_chains)) ||
+      (rc = dalloc(p, &vchain, B->n_packed)))
+    return rc;
+  CK(ctx, bcg::core_contract(p->row, p->col, p->vtx_off, n_plain, p->reach, chain_off, p->chain_start, p->chain_len,
+                             p->chain_l, p->chain_r, d_on, B->n_bcc, B->n_packed, row_off, rows, xcol, xk, xcid, ctab, vchain,
+                             ctx->stream));
+  p->core_slots = (int)std::min<int64_t>(p->core_grid, (int64_t)src.size());
+  const int64_t n = p->core_slots, rec = a.shape.rec_bytes();
+  std::vector<int32_t> ep((size_t)n, 1);
+  if ((rc = dalloc(p, &a.rec, n * rec)) || (rc = dalloc(p, &a.ws, n * a.shape.rest_bytes())) ||
+      (rc = upload(p, &a.epochs, ep.data(), n)))
+    return rc;
+  CK(ctx, cudaMemsetAsync(a.rec, 0, (size_t)(n * rec), ctx->stream));  // key 0: unvisited
+  CK(ctx, cudaStreamSynchronize(ctx->stream));                         // ep goes out of scope
+  a.row = p->row; a.vtx_off = p->vtx_off; a.n_plain = n_plain; a.reach = p->reach; a.chain_off = chain_off;
+  a.rows = rows; a.row_off = row_off; a.xcol = xcol; a.xk = xk; a.xcid = xcid; a.ctab = ctab; a.vchain = vchain; a.src = list;
+  a.next = p->counter; a.acc = p->acc; a.err = p->err;
+  a.rescale_exp = ctx->opts.rescale_exp > 0 ? ctx->opts.rescale_exp : 900;
+  return BCGPU_OK;
+}
+
 // Source orders of the BCCs in multi-source passes, computed on one host
 // thread (each BCC up to the passes the plan fills, as batched_create would).
 // get() waits for the thread; a host allocation that failed there is
@@ -710,18 +785,22 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
 
   // BATCHED: which BCCs take multi-source passes (the others: per-source items)
   std::vector<char> on;
-  std::vector<int32_t> ecc0;  // eccentricity of each BCC's local vertex 0 (the batched plan reuses it)
+  std::vector<int32_t> ecc0;  // eccentricity of each BCC's local vertex 0, -1 unknown (the batched plan reuses it)
+  std::vector<char> conn0;    // where it is known: the BCC is connected
   int64_t n_on = 0;
   if (p->mode == BCGPU_MODE_BATCHED) {
     on.assign((size_t)B->n_bcc, 1);
     ecc0.assign((size_t)B->n_bcc, -1);
+    conn0.assign((size_t)B->n_bcc, 0);
     if (ctx->opts.plain_core >= 0) {
       const int32_t min_core = ctx->opts.plain_core > 0 ? ctx->opts.plain_core : kBatchedMinCore;
       auto route = [&](int32_t b, std::vector<int32_t> &dist, std::vector<int32_t> &queue, bool parallel) {
         if (B->n_plain[b] < min_core) { on[b] = 0; return; }
         int kmax = 0;
         for (int64_t c = B->chain_off[b]; c < B->chain_off[b + 1]; ++c) kmax = std::max(kmax, B->chain_len[c]);
-        ecc0[b] = bcc_ecc0(B, b, dist, queue, parallel);
+        bool connected = false;
+        ecc0[b] = bcc_ecc0(B, b, dist, queue, parallel, &connected);
+        conn0[b] = connected;
         on[b] = 2 * ecc0[b] + kmax <= kBatchedMaxLevels;
       };
       auto big = [&](int32_t b) { return B->vtx_off[b + 1] - B->vtx_off[b] >= kParallelBfs; };
@@ -832,42 +911,19 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
       p->unit_visits.push_back(p->unit_visits.back() + src * nb);
     }
     // PLAIN: items of the BCCs that fit shared memory go to the small-BCC
-    // kernels (sources of an item: its own vertex, then its chains'), unless
-    // the caller asked for a rescaling threshold, which only the per-source
-    // kernel applies. Rows in shared memory instead of L2, and a BFS per chain
+    // kernels (sources of an item: its own vertex, then its chains'). With a
+    // rescaling threshold of the caller's, which those do not apply, they go
+    // to the whole-BCC kernel, whose sums are the same bit for bit, so that a
+    // threshold never changes BC. Rows in shared memory instead of L2, and a BFS per chain
     // vertex instead of a merge and a double listing: a chain-endpoint call on
     // a BCC of 1,494 vertices went from 1.95 to 0.66 ms, 1,194 sources.
-    if (p->mode == BCGPU_MODE_PLAIN && ctx->opts.rescale_exp == 0 && p->n_items > 0 &&
-        p->unit_sources.back() < INT32_MAX) {
-      std::vector<int32_t> plain_ecc;
-      route_tiles(ctx, B, std::vector<char>((size_t)B->n_bcc, 0), tile, plain_ecc, true);
-      std::vector<int32_t> src;
-      std::vector<int64_t> list((size_t)B->n_bcc + 1, 0);
-      std::vector<bcg::PlainItem> rest;
-      for (const auto &it : items) {
-        p->item_at.push_back((int64_t)rest.size());
-        p->src_at.push_back((int64_t)src.size());
-        if (tile[it.bcc] < 0) {
-          rest.push_back(it);
-          continue;
-        }
-        if (it.own) src.push_back(it.src);
-        for (int32_t c = it.c0; c < it.c1; ++c)
-          for (int32_t k = 0; k < B->chain_len[c]; ++k) src.push_back(B->chain_start[c] + k);
-        list[(size_t)it.bcc + 1] = (int64_t)src.size();
-      }
-      p->item_at.push_back((int64_t)rest.size());
-      p->src_at.push_back((int64_t)src.size());
-      for (int32_t b = 0; b < B->n_bcc; ++b) list[(size_t)b + 1] = std::max(list[(size_t)b + 1], list[(size_t)b]);
-      if (!src.empty() && (rc = build_tiles(ctx, B, tile, plain_ecc, p, &src, &list))) return bail(rc);
-      p->h_items = std::move(items);
-      items = std::move(rest);
-    } else {
-      p->h_items = items;
-    }
-    if ((rc = upload(p, &p->items, items.data(), (int64_t)items.size()))) return bail(rc);
+    const bool listed = p->unit_sources.back() - p->unit_sources[(size_t)p->n_bat] < INT32_MAX;
+    std::vector<int8_t> small((size_t)B->n_bcc, -1), core((size_t)B->n_bcc, 0);
+    std::vector<int32_t> small_ecc;
+    const bool scaled = ctx->opts.rescale_exp != 0;
+    if (p->mode == BCGPU_MODE_PLAIN && p->n_items > 0 && listed)
+      route_tiles(ctx, B, std::vector<char>((size_t)B->n_bcc, 0), small, small_ecc, true);
     p->ws_n = (p->mode == BCGPU_MODE_PLAIN ? nb_max : nb_plain) + 2;
-    if ((rc = alloc_acc(p, B->n_packed))) return bail(rc);
     const int64_t per_slot = p->ws_n * (bcg::kWsIntRows * 4 + bcg::kWsDblRows * 8);
     // Four 256-thread CTAs per SM (four sources in flight) when their rows
     // fit the budget, else two of 512, else one of 1024 per SM; with
@@ -884,17 +940,99 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
       if (grid == want) break;
     }
     p->grid = std::max(1, grid);
-    p->slots = (int)std::min<int64_t>(p->grid, (int64_t)items.size());  // items take a slot each
-    const int64_t slots = p->slots + 1;  // + the row-export slot
-    if ((rc = dalloc(p, &p->ws_i, slots * bcg::kWsIntRows * p->ws_n)) ||
-        (rc = dalloc(p, &p->ws_f, slots * bcg::kWsDblRows * p->ws_n)) || (rc = dalloc(p, &p->epochs, 2 * slots)))
-      return bail(rc);
-    if (cudaMemsetAsync(p->ws_f, 0, sizeof(double) * (size_t)(slots * bcg::kWsDblRows * p->ws_n), ctx->stream) !=
-        cudaSuccess)  // row records: stamp 0, unvisited
-      return bail(cuda_fail(ctx, cudaGetLastError(), "cudaMemsetAsync"));
-    std::vector<int32_t> ep((size_t)(2 * slots), 1);
-    CK(ctx, cudaMemcpyAsync(p->epochs, ep.data(), sizeof(int32_t) * ep.size(), cudaMemcpyHostToDevice, ctx->stream));
-    p->h2d_bytes += (int64_t)(sizeof(int32_t) * ep.size());
+    // the others: the contracted kernel, if its slot is no larger than the
+    // whole-BCC kernel's (long chains in a BCC of few chain vertices are not
+    // worth their buckets)
+    bcg::CoreArgs::CoreShape &shape = p->core.shape;
+    shape = {4, 2, 0, 2, 3};
+    int levels = 1;  // the deepest core's
+    if (listed && p->n_items > 0) {
+      std::vector<int32_t> dist, queue;
+      std::vector<char> seen((size_t)B->n_bcc, 0);
+      for (const auto &it : items) {
+        const int32_t b = it.bcc;
+        if (seen[b] || small[b] >= 0) continue;
+        seen[b] = 1;
+        int32_t ecc = ecc0.empty() ? -1 : ecc0[b];
+        if (!core_takes(B, b, dist, queue, &ecc, !conn0.empty() && conn0[b])) continue;
+        int kmax = 0;
+        for (int64_t c = B->chain_off[b]; c < B->chain_off[b + 1]; ++c) kmax = std::max(kmax, B->chain_len[c]);
+        bcg::CoreArgs::CoreShape h = shape;
+        levels = std::max(levels, ecc);
+        h.cap = std::max<int64_t>(h.cap, (B->n_plain[b] + 3) / 4 * 4);  // 16-byte parts of shared memory
+        h.bcap = std::max<int64_t>(h.bcap, 2 * (B->chain_off[b + 1] - B->chain_off[b]) + 2);
+        h.ccap = std::max(h.ccap, B->chain_off[b + 1] - B->chain_off[b]);
+        h.tcap = std::max(h.tcap, 2 * ecc + kmax + 3);
+        h.ring = std::max(h.ring, kmax + 3);
+        if (h.rec_bytes() + h.rest_bytes() > std::max<int64_t>(per_slot, 1 << 16) ||
+            h.smem_bytes() > kCoreBits)
+          continue;
+        shape = h;
+        core[b] = 1;
+      }
+    }
+    // Its CTAs: as wide as its levels are (core vertices over the depth seen
+    // from local vertex 0, and half as much again), between 64 and 512 threads,
+    // as many as fit. Narrow levels leave a wide CTA's warps idle, and wide
+    // ones make more sources in flight miss L2 more often: kernel ms for 64 /
+    // 128 / 256 / 512 threads, 80x80 grid (width 37) 14.9 / 17.1 / 24.3 / -,
+    // 512x512 grid (241) 320 / 171 / 143 / 123, R-MAT 14 (1,009) 135 / 114 / 107
+    // / 91. plain_ctas_per_sm 4, 8 or 16 asks for 256, 128 or 64 threads.
+    if (ctx->opts.plain_ctas_per_sm) {
+      p->core_block = 1024 / ctx->opts.plain_ctas_per_sm;
+    } else {
+      p->core_block = 64;
+      while (p->core_block < 512 && 2 * p->core_block * (int64_t)levels < 3 * shape.cap) p->core_block *= 2;
+    }
+    p->core_grid = (int)std::min<int64_t>((int64_t)ctx->sms * bcg::core_ctas_per_sm(p->core_block, shape),
+                                          avail / (shape.rec_bytes() + shape.rest_bytes()));
+    if (p->core_grid < 1) std::fill(core.begin(), core.end(), 0);
+    std::vector<int32_t> src;
+    std::vector<bcg::CoreSource> csrc;
+    std::vector<int64_t> list((size_t)B->n_bcc + 1, 0);
+    std::vector<bcg::PlainItem> rest;
+    for (const auto &it : items) {
+      p->src_at.push_back((int64_t)src.size());
+      p->core_at.push_back((int64_t)csrc.size());
+      p->item_at.push_back((int64_t)rest.size());
+      const bool t = small[it.bcc] >= 0 && !scaled;
+      if (!t && !core[it.bcc]) {
+        rest.push_back(it);
+        continue;
+      }
+      auto add = [&](int32_t s) {
+        if (t) src.push_back(s);
+        else csrc.push_back({it.bcc, s});
+      };
+      if (it.own) add(it.src);
+      for (int32_t c = it.c0; c < it.c1; ++c)
+        for (int32_t k = 0; k < B->chain_len[c]; ++k) add(B->chain_start[c] + k);
+      if (t) list[(size_t)it.bcc + 1] = (int64_t)src.size();
+    }
+    p->src_at.push_back((int64_t)src.size());
+    p->core_at.push_back((int64_t)csrc.size());
+    p->item_at.push_back((int64_t)rest.size());
+    for (int32_t b = 0; b < B->n_bcc; ++b) list[(size_t)b + 1] = std::max(list[(size_t)b + 1], list[(size_t)b]);
+    if (!src.empty() && (rc = build_tiles(ctx, B, small, small_ecc, p, &src, &list))) return bail(rc);
+    p->h_items = std::move(items);
+    if ((rc = upload(p, &p->items, rest.data(), (int64_t)rest.size()))) return bail(rc);
+    if ((rc = alloc_acc(p, B->n_packed))) return bail(rc);
+    if (!csrc.empty() && (rc = build_core(ctx, B, core, csrc, p))) return bail(rc);
+    p->slots = (int)std::min<int64_t>(p->grid, (int64_t)rest.size());  // items take a slot each
+    if (p->slots || p->mode == BCGPU_MODE_PLAIN) {
+      const int64_t slots = p->slots + 1;  // + the row-export slot
+      if ((rc = dalloc(p, &p->ws_i, slots * bcg::kWsIntRows * p->ws_n)) ||
+          (rc = dalloc(p, &p->ws_f, slots * bcg::kWsDblRows * p->ws_n)) || (rc = dalloc(p, &p->epochs, 2 * slots)))
+        return bail(rc);
+      if (cudaMemsetAsync(p->ws_f, 0, sizeof(double) * (size_t)(slots * bcg::kWsDblRows * p->ws_n), ctx->stream) !=
+          cudaSuccess)  // row records: stamp 0, unvisited
+        return bail(cuda_fail(ctx, cudaGetLastError(), "cudaMemsetAsync"));
+      std::vector<int32_t> ep((size_t)(2 * slots), 1);
+      CK(ctx, cudaMemcpyAsync(p->epochs, ep.data(), sizeof(int32_t) * ep.size(), cudaMemcpyHostToDevice, ctx->stream));
+      p->h2d_bytes += (int64_t)(sizeof(int32_t) * ep.size());
+    }
+    // the tables above are copied before they go out of scope
+    CK(ctx, cudaStreamSynchronize(ctx->stream));
   }
   HOST_MARK("plain items+ws");
   if (n_tile && (rc = build_tiles(ctx, B, tile, tile_ecc, p))) return bail(rc);
@@ -1260,8 +1398,16 @@ int enqueue_units(bc_plan *p, int64_t begin, int64_t end, int *launches) {
       b0 = std::min(b0, p->h_items[j].bcc);
       b1 = std::max(b1, p->h_items[j].bcc);
     }
-    const bool split = !p->item_at.empty();  // a PLAIN plan with small BCCs among its items
-    const int64_t k0 = split ? p->item_at[(size_t)j0] : j0, k1 = split ? p->item_at[(size_t)j1] : j1;
+    const int64_t k0 = p->item_at[(size_t)j0], k1 = p->item_at[(size_t)j1];
+    const int64_t c0 = p->core_at[(size_t)j0], c1 = p->core_at[(size_t)j1];
+    const int64_t t0 = p->src_at[(size_t)j0], t1 = p->src_at[(size_t)j1];
+    if (c1 > c0) {
+      CK(ctx, cudaMemsetAsync(p->counter, 0, sizeof(unsigned long long), ctx->stream));
+      bcg::CoreArgs a = p->core;
+      a.lo = c0; a.hi = c1;
+      CK(ctx, bcg::launch_core(a, p->core_block, (int)std::min<int64_t>(p->core_slots, c1 - c0), ctx->stream));
+      ++*launches;
+    }
     if (k1 > k0) {
       CK(ctx, cudaMemsetAsync(p->counter, 0, sizeof(unsigned long long), ctx->stream));
       bcg::PlainArgs a = plain_args(p);
@@ -1270,9 +1416,7 @@ int enqueue_units(bc_plan *p, int64_t begin, int64_t end, int *launches) {
       CK(ctx, bcg::launch_plain(a, p->block, grid, ctx->stream));
       ++*launches;
     }
-    if (split && p->src_at[(size_t)j1] > p->src_at[(size_t)j0] &&
-        (rc = enqueue_tiles(p, 0, p->n_titems, (int32_t)p->src_at[(size_t)j0], (int32_t)p->src_at[(size_t)j1], launches)))
-      return rc;
+    if (t1 > t0 && (rc = enqueue_tiles(p, 0, p->n_titems, (int32_t)t0, (int32_t)t1, launches))) return rc;
     CK(ctx, bcg::launch_fold(p->acc, p->bc, p->h_vtx_off[b0], p->h_vtx_off[b1 + 1], ctx->stream));
     ++*launches;
     j0 = j1;
