@@ -390,16 +390,6 @@ int alloc_acc(bc_plan *p, int64_t n_packed) {
   return BCGPU_OK;
 }
 
-// Sources per small-BCC work item, at most: the CTA runs them (a warp each,
-// or one after another) from one staged slice; larger BCCs are split so that
-// many CTAs share them, and a class with few sources in all gets smaller
-// items, so that it still has several items per resident CTA.
-constexpr int32_t kTileItemSources = 128;
-constexpr int64_t kTileItemsPerCta = 4;
-// BCCs of up to this many vertices take the warp class (a warp per source,
-// eight per CTA); larger ones the CTA class (the CTA on one source).
-constexpr int64_t kTileWarpMaxVertices = 640;
-
 // Whether BCC b's arcs come in mirrored pairs, by a sum over the arcs of a
 // mixed (u, v) that pairs cancel: an undirected BCC always passes.
 bool mirrored(const bc_bccs *B, int32_t b) {
@@ -475,7 +465,7 @@ void route_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<char> &on, std
       const int64_t arcs = B->row[vo + nb] - B->row[vo];
       bytes[b] = bcg::TileSlice::bytes(nb, arcs);
       if (nb > cap) continue;
-      const int c = nb <= kTileWarpMaxVertices ? bcg::kTileWarp : bcg::kTileCta;
+      const int c = nb <= bcg::kTileWarpMaxVertices ? bcg::kTileWarp : bcg::kTileCta;
       if (bcg::tile_smem_bytes(fit_cls(c), nb, bytes[b]) > lim) continue;
       int64_t maxdeg = 1;
       for (int64_t k = vo; k < vo + nb; ++k) maxdeg = std::max(maxdeg, B->row[k + 1] - B->row[k]);
@@ -545,7 +535,6 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
   std::vector<int64_t> off((size_t)B->n_bcc, -1);
   std::vector<int32_t> size((size_t)B->n_bcc, 0);
   std::vector<int8_t> bucket((size_t)B->n_bcc, -1);
-  constexpr int64_t kSmPerSm = 228 * 1024, kReserved = 1024;  // shared memory per SM, per-CTA reserve
   // bucket k -> class: 0 warp, 1 / 2 CTA (4+ / 3 per SM), 3 four groups, 4 CTA-512, 5 two groups, 6 CTA-1024
   constexpr int kBucketCls[7] = {bcg::kTileWarp,    bcg::kTileCta,       bcg::kTileCta,      bcg::kTileCta1024x4,
                                  bcg::kTileCta512, bcg::kTileCta1024x2, bcg::kTileCta1024};
@@ -556,7 +545,7 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
     const int64_t vo = B->vtx_off[b], nb = B->vtx_off[b + 1] - vo;
     size[b] = (int32_t)bcg::TileSlice::bytes(nb, B->row[vo + nb] - B->row[vo]);
     if (cls[b] == bcg::kTileWarp) { bucket[b] = 0; continue; }
-    per[b] = kSmPerSm / ((int64_t)bcg::tile_smem_bytes(bcg::kTileCta, nb, size[b]) + kReserved);
+    per[b] = bcg::kTileSmPerSm / ((int64_t)bcg::tile_smem_bytes(bcg::kTileCta, nb, size[b]) + bcg::kTileReserved);
     bucket[b] = (int8_t)(per[b] >= 4 ? 1 : per[b] == 3 ? 2 : per[b] == 2 ? 4 : 6);
   }
   // the grouped classes: a BCC moves up when its groups fit and the bucket's
@@ -607,10 +596,7 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
     T.grid = ctx->sms * per_sm;
     const int groups = bcg::tile_groups(T.cls);
     if (T.cls != bcg::kTileWarp) p_rows = std::max<int64_t>(p_rows, (int64_t)T.grid * groups);
-    // a warp-class item feeds 8 warps, a grouped CTA's item its groups
-    const int64_t floor_items = T.cls == bcg::kTileWarp ? bcg::kTileWarps : groups;
-    const int32_t per_item = (int32_t)std::max<int64_t>(
-        floor_items, std::min<int64_t>(kTileItemSources, sources / ((int64_t)T.grid * kTileItemsPerCta)));
+    const int32_t per_item = bcg::tile_item_sources(T.cls, T.grid, sources);
     for (int32_t b = 0; b < B->n_bcc; ++b) {
       if (bucket[b] != k) continue;
       const int64_t l0 = first_of(b), l1 = l0 + sources_of(b);

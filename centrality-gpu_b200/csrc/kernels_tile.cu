@@ -35,11 +35,13 @@
 //    global fixed-point counters.
 // Path counts are FP64 without per-level scaling: the plan routes a BCC here
 // only when no path count can pass 2^1000 ((2 ecc + 1) levels of at most
-// maxdeg predecessors each); a non-finite value still flags kDevOverflow.
+// maxdeg predecessors each); one that does, or a non-finite value, flags
+// kDevOverflow.
 #include "accum.cuh"
 #include "common.cuh"
 #include "tile.h"
 
+#include <algorithm>
 #include <cooperative_groups.h>
 
 namespace cg = cooperative_groups;
@@ -292,7 +294,9 @@ __device__ __forceinline__ double finish(const View &g, int32_t w, double sum, d
   const double sw = sq[w];
   const double delta = sw * sum;
   const double qw = ((double)__ldg(g.rch + w) + 1.0 + delta) / sw;
-  if (exp_bits(qw) == 0x7ff || exp_bits(delta) == 0x7ff || exp_bits(sw) == 0) set_err(err, kDevOverflow);
+  // counts past 2^1000 too: their q would lose bits below FP64's normal range
+  if (exp_bits(qw) == 0x7ff || exp_bits(delta) == 0x7ff || (unsigned)(exp_bits(sw) - 1) >= 1023 + 1000)
+    set_err(err, kDevOverflow);
   sq[w] = qw;
   return delta;
 }
@@ -647,6 +651,30 @@ size_t tile_smem_bytes(int cls, int64_t nmax, int64_t slice_max) {
 }
 
 int tile_groups(int cls) { return cls == kTileCta1024x2 ? 2 : cls == kTileCta1024x4 ? 4 : 1; }
+
+// At most kItemSources: the CTA runs them (a warp each, or one after another)
+// from one staged slice; larger BCCs are split so that many CTAs share them, and
+// a class with few sources in all gets smaller items, so that it still has
+// several per resident CTA -- but an item feeds every warp of the warp class and
+// every group of a grouped CTA.
+int32_t tile_item_sources(int cls, int64_t grid, int64_t sources) {
+  constexpr int64_t kItemSources = 128, kItemsPerCta = 4;
+  const int64_t least = cls == kTileWarp ? kTileWarps : tile_groups(cls);
+  return (int32_t)std::max<int64_t>(least, std::min<int64_t>(kItemSources, sources / (grid * kItemsPerCta)));
+}
+
+int tile_class(int64_t n, int64_t slice_bytes, size_t lim) {
+  auto fits = [&](int cls) { return tile_smem_bytes(cls, n, slice_bytes) <= lim; };
+  if (n > kTileMaxVertices) return -1;
+  if (n <= kTileWarpMaxVertices) return fits(kTileWarp) ? kTileWarp : -1;
+  const int64_t per = kTileSmPerSm / ((int64_t)tile_smem_bytes(kTileCta, n, slice_bytes) + kTileReserved);
+  if (per >= 4) return kTileCta;
+  if (fits(kTileCta1024x4)) return kTileCta1024x4;
+  if (per == 3) return kTileCta;
+  if (per == 2) return kTileCta512;
+  if (fits(kTileCta1024x2)) return kTileCta1024x2;
+  return fits(kTileCta1024) ? kTileCta1024 : -1;
+}
 
 size_t tile_smem_limit(int device) {
   int v = 0;

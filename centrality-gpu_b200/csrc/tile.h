@@ -32,6 +32,8 @@ constexpr int kTileWarps = 8;          // warps per CTA
 constexpr int kTileMaxLevels = 1024;   // BFS levels the CTA class records (routing keeps BCCs below)
 constexpr int kTileGroupMaxLevels = 256;  // the same for the grouped classes
 constexpr int kGroupLongQueue = 256;      // long-row queue of a group in the grouped classes
+constexpr int64_t kTileWarpMaxVertices = 640;  // BCCs of up to this many vertices take the warp class
+constexpr int64_t kTileSmPerSm = 228 * 1024, kTileReserved = 1024;  // shared memory per SM, per-CTA reserve
 constexpr int32_t kTileMaxVertices = 65535;  // neighbour ids are 16-bit in the slice
 
 // Byte layout of one BCC's staged slice, each part starting on a 16-byte
@@ -72,6 +74,13 @@ struct TileArgs {
   int *err;
 };
 
+// Class of a lone BCC of n vertices with a slice of slice_bytes, as the plan's
+// buckets (bcgpu.cu build_tiles) would have it, or -1 if none fits lim bytes of
+// shared memory. The classes of several groups hold fewer levels than the others.
+int tile_class(int64_t n, int64_t slice_bytes, size_t lim);
+// Sources per work item of a launch of class cls with `grid` resident CTAs and
+// `sources` in all.
+int32_t tile_item_sources(int cls, int64_t grid, int64_t sources);
 // Dynamic shared memory of a launch of class cls for BCCs of up to nmax
 // vertices and slices of up to slice_max bytes.
 size_t tile_smem_bytes(int cls, int64_t nmax, int64_t slice_max);

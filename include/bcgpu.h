@@ -167,8 +167,10 @@ int bc_begin_free(bc_ctx *ctx, const int32_t *R, const int32_t *C, int32_t n, in
 /* Variant of bc_begin_free that allocates nothing (no reference counterpart).
  * BC is accumulated like the per-source schedule's (fixed-point counters
  * folded to FP64: the same result on every call, whatever the order in which
- * the CTAs finish their sources); the first call on a device clears the
- * array's rows and counters, later calls reuse what the previous call left.
+ * the CTAs finish their sources). A BCC that fits shared memory runs on the
+ * small-BCC kernels, a larger one (or one too deep for them) on the per-source
+ * kernel with its rows in the array; the first call on a device clears what it
+ * uses of the array, later calls reuse what the previous call left.
  * For callers that cannot create device allocations of their own -- their
  * device memory belongs to another allocator (a framework's caching pool, an
  * arena budgeted up front), so a cudaMalloc/cudaFree here would break that
