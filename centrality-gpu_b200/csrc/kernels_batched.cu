@@ -10,7 +10,8 @@
 // (the reference's ear postprocessing, Codes/postprocesses.cu:205-351, done
 // here for every source of the pass at once).
 //
-// Slots. One pass ("batch") covers up to B = 32*W sources of one BCC:
+// Slots. One pass ("batch") covers up to B = 32*W sources of one BCC (on small
+// cores the kernel runs several passes as one, see merge_passes):
 //   core source     level 0 at the vertex;
 //   chain source    the vertex at position p (0-based from L) of a chain of
 //                   k vertices: seeded at L on level p+1 and at R on level
@@ -71,7 +72,10 @@ constexpr int kWarpsPerCta = kThreads / 32;
 #define BCGPU_BATCHED_HEAVY_DEG 1024
 #endif
 constexpr int kHeavyDeg = BCGPU_BATCHED_HEAVY_DEG;
-constexpr int kHeavyDegSmall = 32; // ... or than this, on cores small enough that one row is a level's critical path
+// ... or than this, on cores small enough that one row is a level's critical path
+// (R-MAT 14, 16 passes of 512 one by one / by 8: 61.9 / 39.2 ms for 32, 54.9 /
+// 32.1 for 128, 55.8 / 31.3 for 512).
+constexpr int kHeavyDegSmall = 512;
 constexpr int kSmallCore = 16384;  // cores below this many vertices use kHeavyDegSmall
 #ifndef BCGPU_BATCHED_CHUNK
 #define BCGPU_BATCHED_CHUNK 2048
@@ -113,10 +117,10 @@ struct Slot {
   int32_t src, chain, pos, pad;
 };
 
-// Where a chain source enters the core: slot reaches core vertex v on `level`
-// with one path along its chain.
+// Where a chain source enters the core: slot of pass `pass` reaches core vertex
+// v on `level` with one path along its chain.
 struct Seed {
-  int32_t v, level, slot, pad;
+  int32_t v, level, slot, pass;
 };
 
 struct Batch {
@@ -187,7 +191,9 @@ struct Args {
   int32_t *X;       // [B][tcap+2]
   int32_t *rexp;    // [B] per-level max exponent (rescale)
   int64_t n_cap;    // core rows allocated (>= largest core)
-  int32_t W;        // words per row (row stride)
+  int32_t W;        // words per row (row stride): those of `merge` passes
+  int32_t width;    // slots of a pass
+  int32_t merge;    // passes run as one, at most
   int32_t tcap;     // levels allocated
   int32_t rescale_exp;
   unsigned long long wait_ns;  // limit of one grid-barrier wait
@@ -709,9 +715,21 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
   constexpr bool kComp = sizeof(QT) == 4;
   PHASE_INIT();
 
-  for (int64_t bi = a.b0; bi < a.b1; ++bi) {
+  int npass = 1;
+  for (int64_t bi = a.b0; bi < a.b1; bi += npass) {
     if (cta_failed(a)) return;
-    const Batch bt = a.batches[bi];
+    // the next passes of the same BCC as one: their slots, seeds and arming
+    // lists follow each other, and all but a BCC's last pass are full
+    Batch bt = a.batches[bi];
+    for (npass = 1; npass < a.merge && bi + npass < a.b1; ++npass) {
+      const Batch &nx = a.batches[bi + npass];
+      if (nx.bcc != bt.bcc) break;
+      bt.nslots += nx.nslots;
+      bt.nseeds += nx.nseeds;
+      bt.narm += nx.narm;
+      bt.max_seed = max(bt.max_seed, nx.max_seed);
+    }
+    bt.words = (bt.nslots + 31) / 32;
     const Slot *slots = a.slots + bt.slot_off;
     const Seed *seeds = a.seeds + bt.seed_off;
     const int words = bt.words;
@@ -917,7 +935,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
         for (int64_t i = gtid; i < bt.nseeds; i += gthreads) {
           const Seed s = seeds[i];
           if (s.level != t + 1) continue;
-          const int b = s.slot, w = b >> 5;
+          const int b = s.slot + (int)(s.pass - bi) * a.width, w = b >> 5;
           const uint32_t bit = 1u << (b & 31);
           const int64_t idx = ((int64_t)s.v * W + w) * 32 + (b & 31);
           const double one = scale2(1.0, -a.X[(int64_t)b * (a.tcap + 2) + t]);
@@ -1220,7 +1238,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
     // ---- fold the batch into BC (fixed word order), unless FP32 range failed
     const int bad = *(volatile int *)&a.ctrl->range_err;
     if (bad) {
-      if (gtid == 0) a.redo[bi] = 1;
+      if (gtid < npass) a.redo[bi + gtid] = 1;
     } else {
       for (int64_t v = gtid; v < n; v += gthreads) {  // core vertices (chain vertices were added above)
         double s = 0.0;
@@ -1263,6 +1281,7 @@ using HostBuf = std::vector<T, NoInit<T>>;
 struct BatchedPlan {
   int width = 0;       // B
   int W = 0;           // words
+  int merge = 1;       // passes run as one, at most
   int tcap = 0;
   int64_t n_cap = 0;
   bool f32 = true;
@@ -1313,6 +1332,20 @@ int batched_width(int requested) {
   const int width = requested > 0 ? requested : 512;
   return std::max(32, std::min(1024, (width + 31) / 32 * 32));
 }
+
+namespace {
+
+// Passes of `width` slots run as one on a core of n vertices: a level of a pass
+// costs its slowest row whatever else there is to do, so a small core gets more
+// slots per level, up to 80 million (vertex, slot) pairs (2.2 GB of workspace);
+// beyond that the grid is full either way. R-MAT 14 (9,107 core vertices, 16
+// passes of 512): 54.9 ms one by one, 40.0 / 33.8 / 31.3 by 2 / 4 / 8; R-MAT 16
+// (32,842, 8 passes of 256, FP64) 83.0, 64.0 / 55.7 / 50.2; R-MAT 18 (121,000, 4
+// of 512) 115.5, 110.6 / 111.0 by 2 / 4.
+constexpr int64_t kMergePairs = 80 * 1000 * 1000;
+int merge_passes(int64_t n, int width) { return (int)std::max<int64_t>(1, kMergePairs / (n * width)); }
+
+}  // namespace
 
 // Source order of BCC b: bounded BFS balls of nearby vertices (chain vertices
 // included), so a pass's sources see every vertex within a narrow band of
@@ -1634,8 +1667,8 @@ int batched_build(const bc_bccs *B, const BatchedConfig &cfg, const int64_t *row
         const int64_t c = cof[s];
         const int32_t p = cpos[s], k = B->chain_len[c];
         slots[slot0 + i] = Slot{s, (int32_t)c, p, 0};
-        seeds[sd++] = Seed{B->chain_l[c], p + 1, slot, 0};
-        seeds[sd++] = Seed{B->chain_r[c], k - p, slot, 0};
+        seeds[sd++] = Seed{B->chain_l[c], p + 1, slot, (int32_t)(bat0 + j)};
+        seeds[sd++] = Seed{B->chain_r[c], k - p, slot, (int32_t)(bat0 + j)};
         bt.max_seed = std::max(bt.max_seed, std::max(p + 1, k - p));
       }
       bt.nseeds = (int32_t)(sd - bt.seed_off);
@@ -1676,11 +1709,20 @@ int batched_build(const bc_bccs *B, const BatchedConfig &cfg, const int64_t *row
   const int64_t n = P->n_cap;
   const int64_t qb = P->f32 ? 4 : 8;
   const int64_t nch = (int64_t)hchunk_v.size();
-  const int64_t need = n * W * 32 * (4 + 8 + 8 + qb) + (int64_t)(tcap + 2) * n * W * 4 + n * W * 4 + n * 12 +
-                       n * W * 8 + (int64_t)W * 32 * (tcap + 2) * 4 + nch * W * 32 * 8;
+  auto need_of = [&](int64_t w) {
+    return n * w * 32 * (4 + 8 + 8 + qb) + (int64_t)(tcap + 2) * n * w * 4 + n * w * 4 + n * 12 + n * w * 8 +
+           w * 32 * (tcap + 2) * 4 + nch * w * 32 * 8;
+  };
+  const int64_t need = need_of(W);
   if (need > cfg.limit_bytes)
     return bail(BCGPU_ENOMEM, "batched workspace " + std::to_string(need >> 20) + " MiB exceeds the limit " +
                                   std::to_string(cfg.limit_bytes >> 20) + " MiB (lower the batch width)");
+  // passes run as one: as many as the rule allows, the plan will run and the
+  // workspace fits; a pass has to end on a whole group of words
+  const int64_t filled = std::min(P->n_batches, cfg.fill_end) - std::max<int64_t>(0, cfg.fill_begin);
+  P->merge = W * 32 == width ? (int)std::max<int64_t>(1, std::min<int64_t>(merge_passes(n, width), filled)) : 1;
+  while (P->merge > 1 && need_of((int64_t)P->merge * W) > cfg.limit_bytes) --P->merge;
+  const int64_t WA = (int64_t)P->merge * W;  // words a row is allocated
   P->pool = cfg.pool;
   P->stream = stream;
   auto alloc = [&](void **p, int64_t bytes) -> bool {
@@ -1699,21 +1741,21 @@ int batched_build(const bc_bccs *B, const BatchedConfig &cfg, const int64_t *row
   Args &a = P->args;
   void *p = nullptr;
   bool ok = true;
-  ok &= alloc(&p, n * W * 32 * 4); a.d = (int32_t *)p;
-  ok &= ok && alloc(&p, n * W * 32 * 8); a.sig = (double *)p;
-  ok &= ok && alloc(&p, n * W * 32 * qb); a.q = p;
-  ok &= ok && alloc(&p, (int64_t)(tcap + 2) * n * W * 4); a.lm = (uint32_t *)p;
-  ok &= ok && alloc(&p, n * W * 4); a.seen = (uint32_t *)p;
+  ok &= alloc(&p, n * WA * 32 * 4); a.d = (int32_t *)p;
+  ok &= ok && alloc(&p, n * WA * 32 * 8); a.sig = (double *)p;
+  ok &= ok && alloc(&p, n * WA * 32 * qb); a.q = p;
+  ok &= ok && alloc(&p, (int64_t)(tcap + 2) * n * WA * 4); a.lm = (uint32_t *)p;
+  ok &= ok && alloc(&p, n * WA * 4); a.seen = (uint32_t *)p;
   ok &= ok && alloc(&p, n * 4); a.lmin = (int32_t *)p;
   ok &= ok && alloc(&p, n * 4); a.lmax = (int32_t *)p;
   ok &= ok && alloc(&p, n * 4); a.gdone = (int32_t *)p;
   ok &= ok && alloc(&p, n * 4); a.armed = (int32_t *)p;
   ok &= ok && alloc(&p, (4 * ((int64_t)tcap + 3) + 2) * 4); a.wq = (int *)p;
-  ok &= ok && alloc(&p, n * W * 8); a.bcpart = (double *)p;
-  ok &= ok && alloc(&p, n * W * 32 * 8); a.cdep = (double *)p;
-  ok &= ok && alloc(&p, (int64_t)W * 32 * 8); a.wsrc = (double *)p;
-  ok &= ok && alloc(&p, (int64_t)W * 32 * (tcap + 2) * 4); a.X = (int32_t *)p;
-  ok &= ok && alloc(&p, (int64_t)W * 32 * 4); a.rexp = (int32_t *)p;
+  ok &= ok && alloc(&p, n * WA * 8); a.bcpart = (double *)p;
+  ok &= ok && alloc(&p, n * WA * 32 * 8); a.cdep = (double *)p;
+  ok &= ok && alloc(&p, WA * 32 * 8); a.wsrc = (double *)p;
+  ok &= ok && alloc(&p, WA * 32 * (tcap + 2) * 4); a.X = (int32_t *)p;
+  ok &= ok && alloc(&p, WA * 32 * 4); a.rexp = (int32_t *)p;
   ok &= ok && alloc(&p, sizeof(Ctrl)); a.ctrl = (Ctrl *)p;
   ok &= ok && alloc(&p, (int64_t)std::max<int64_t>(P->n_batches, 1) * 4); a.redo = (int *)p;
   HOST_MARK("b: ws alloc");
@@ -1778,8 +1820,8 @@ int batched_build(const bc_bccs *B, const BatchedConfig &cfg, const int64_t *row
   }
   ok = ok && upload((const void **)&a.seeds, seeds.data(), (int64_t)seeds.size() * (int64_t)sizeof(Seed));
   ok = ok && upload((const void **)&a.arms, arms.data(), (int64_t)arms.size() * (int64_t)sizeof(int2));
-  ok = ok && alloc(&p, std::max<int64_t>(nch, 1) * W * 32 * 8); a.hacc = (double *)p;
-  ok = ok && alloc(&p, std::max<int64_t>(nch, 1) * W * 4); a.hmask = (uint32_t *)p;
+  ok = ok && alloc(&p, std::max<int64_t>(nch, 1) * WA * 32 * 8); a.hacc = (double *)p;
+  ok = ok && alloc(&p, std::max<int64_t>(nch, 1) * WA * 4); a.hmask = (uint32_t *)p;
   if (!ok) return bail(BCGPU_ENOMEM, "cudaMalloc or upload of the batched workspace failed");
   cudaError_t e = cudaMemsetAsync(a.ctrl, 0, sizeof(Ctrl), stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(a.redo, 0, (size_t)std::max<int64_t>(P->n_batches, 1) * 4, stream);
@@ -1801,7 +1843,7 @@ int batched_build(const bc_bccs *B, const BatchedConfig &cfg, const int64_t *row
   if (h_bad & 2) return bail(BCGPU_EINVAL, "a core vertex adjacent to the inside of a chain");
   a.reach = reach; a.vtx_off = vtx_off;
   a.chain_start = chain_start; a.chain_len = chain_len; a.chain_l = chain_l; a.chain_r = chain_r;
-  a.n_cap = P->n_cap; a.W = W; a.tcap = tcap; a.bc = bc; a.err = err;
+  a.n_cap = P->n_cap; a.W = W; a.width = width; a.merge = 1; a.tcap = tcap; a.bc = bc; a.err = err;
   a.rescale_exp = cfg.rescale_exp > 0 ? cfg.rescale_exp : 900;
   a.wait_ns = cfg.wait_ns;
 
@@ -1968,6 +2010,8 @@ int batched_run(BatchedPlan *p, int64_t begin, int64_t end, cudaStream_t stream,
   Args a = p->args;
   a.b0 = begin;
   a.b1 = end;
+  a.merge = (int)std::min<int64_t>(p->merge, end - begin);
+  a.W = a.merge * p->W;  // a lone pass keeps the row stride batched_pass_rows reads
   void *params[] = {&a};
   cudaError_t e = cudaMemsetAsync(&p->args.ctrl->bar_count, 0, 2 * sizeof(unsigned int), stream);
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
