@@ -429,6 +429,13 @@ bool chains_are_paths(const bc_bccs *B, int32_t b) {
   return true;
 }
 
+// Pairs of arcs in BCC b's slice: a row of an odd number has a spare place.
+int64_t slice_pairs(const bc_bccs *B, int32_t b) {
+  int64_t pairs = 0;
+  for (int64_t k = B->vtx_off[b]; k < B->vtx_off[b + 1]; ++k) pairs += (B->row[k + 1] - B->row[k] + 1) / 2;
+  return pairs;
+}
+
 // Small-BCC class of each BCC (-1: not in the schedule): BCCs off the
 // multi-source passes with at most opts.tile_max vertices whose CTA fits the
 // device's shared memory and whose path counts cannot overflow FP64 without
@@ -462,9 +469,8 @@ void route_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<char> &on, std
     for (int32_t b = 0; b < B->n_bcc; ++b) {
       if (on[b]) continue;
       const int64_t vo = B->vtx_off[b], nb = B->vtx_off[b + 1] - vo;
-      const int64_t arcs = B->row[vo + nb] - B->row[vo];
-      bytes[b] = bcg::TileSlice::bytes(nb, arcs);
       if (nb > cap) continue;
+      bytes[b] = bcg::TileSlice::bytes(nb, slice_pairs(B, b));
       const int c = nb <= bcg::kTileWarpMaxVertices ? bcg::kTileWarp : bcg::kTileCta;
       if (bcg::tile_smem_bytes(fit_cls(c), nb, bytes[b]) > lim) continue;
       int64_t maxdeg = 1;
@@ -520,7 +526,8 @@ bool core_takes(const bc_bccs *B, int32_t b, std::vector<int32_t> &dist, std::ve
 // 4 or more / 3 per SM; a 1024-thread CTA of four source groups (when four
 // groups' arrays and the slice fit, and the BCC fits that class's level
 // table); 512-thread CTAs at 2 per SM; a 1024-thread CTA of two groups; one
-// 1024-thread CTA per SM. Each bucket's items are contiguous.
+// 1024-thread CTA per SM; a 1024-thread CTA of eight groups, wherever it fits.
+// Each bucket's items are contiguous.
 // With a source list (PLAIN plans: src, each BCC's sources from list[b] on)
 // the items hold places in it, and contributions go straight into the
 // fixed-point counters, so that BC is bit for bit what the per-source kernel
@@ -535,15 +542,18 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
   std::vector<int64_t> off((size_t)B->n_bcc, -1);
   std::vector<int32_t> size((size_t)B->n_bcc, 0);
   std::vector<int8_t> bucket((size_t)B->n_bcc, -1);
-  // bucket k -> class: 0 warp, 1 / 2 CTA (4+ / 3 per SM), 3 four groups, 4 CTA-512, 5 two groups, 6 CTA-1024
-  constexpr int kBucketCls[7] = {bcg::kTileWarp,    bcg::kTileCta,       bcg::kTileCta,      bcg::kTileCta1024x4,
-                                 bcg::kTileCta512, bcg::kTileCta1024x2, bcg::kTileCta1024};
+  // bucket k -> class: 0 warp, 1 / 2 CTA (4+ / 3 per SM), 3 four groups, 4 CTA-512, 5 two groups, 6 CTA-1024,
+  // 7 eight groups
+  constexpr int kBuckets = 8;
+  constexpr int kBucketCls[kBuckets] = {bcg::kTileWarp,   bcg::kTileCta,       bcg::kTileCta,     bcg::kTileCta1024x4,
+                                        bcg::kTileCta512, bcg::kTileCta1024x2, bcg::kTileCta1024, bcg::kTileCta1024x8};
   const int64_t lim = (int64_t)bcg::tile_smem_limit(ctx->device);
-  std::vector<int64_t> per((size_t)B->n_bcc, 0);
+  std::vector<int64_t> per((size_t)B->n_bcc, 0), pairs((size_t)B->n_bcc, 0);
   for (int32_t b = 0; b < B->n_bcc; ++b) {
     if (cls[b] < 0) continue;
-    const int64_t vo = B->vtx_off[b], nb = B->vtx_off[b + 1] - vo;
-    size[b] = (int32_t)bcg::TileSlice::bytes(nb, B->row[vo + nb] - B->row[vo]);
+    const int64_t nb = B->vtx_off[b + 1] - B->vtx_off[b];
+    pairs[b] = slice_pairs(B, b);
+    size[b] = (int32_t)bcg::TileSlice::bytes(nb, pairs[b]);
     if (cls[b] == bcg::kTileWarp) { bucket[b] = 0; continue; }
     per[b] = bcg::kTileSmPerSm / ((int64_t)bcg::tile_smem_bytes(bcg::kTileCta, nb, size[b]) + bcg::kTileReserved);
     bucket[b] = (int8_t)(per[b] >= 4 ? 1 : per[b] == 3 ? 2 : per[b] == 2 ? 4 : 6);
@@ -572,10 +582,11 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
       bucket[b] = (int8_t)to;
     }
   };
-  promote(3, [&](int32_t b) { return per[b] <= 3; });                    // four sources in flight, not at most three
+  promote(7, [&](int32_t b) { return per[b] <= 7; });                    // eight sources in flight, not at most seven
+  promote(3, [&](int32_t b) { return per[b] <= 3 && bucket[b] != 7; });  // four, not at most three
   promote(5, [&](int32_t b) { return per[b] <= 1 && bucket[b] == 6; });  // two instead of one
   int64_t total = 0, p_rows = 1;
-  for (int k = 0; k <= 6; ++k) {
+  for (int k = 0; k < kBuckets; ++k) {
     bc_plan::TileLaunch T;
     T.cls = kBucketCls[k];
     T.i0 = (int64_t)p->h_titems.size();
@@ -609,28 +620,27 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
     if (T.cls == bcg::kTileWarp) p->tcap = nmax + 2;
     p->tl.push_back(T);
   }
-  // slices: local row offsets (uint16 when narrow, else int32), neighbours
-  // (uint16), 16-byte aligned parts; bit 0 of a narrow slice's offset set
+  // slices: row offsets in pairs (uint16 when narrow, else int32), neighbours
+  // (uint16, a row's spare place the vertex itself), 16-byte aligned parts; bit 0
+  // of a narrow slice's offset set
   std::vector<unsigned char> blob((size_t)std::max<int64_t>(total, 16), 0);
+  std::vector<int64_t> off_flag(off);  // what the kernels read: offset | narrow
 #pragma omp parallel for schedule(dynamic, 16) if (B->n_bcc > 16)
   for (int32_t b = 0; b < B->n_bcc; ++b) {
     if (off[b] < 0) continue;  // no item
-    const int64_t vo = B->vtx_off[b], nb = B->vtx_off[b + 1] - vo, e0 = B->row[vo];
-    const int64_t arcs = B->row[vo + nb] - e0;
-    const bool narrow = bcg::TileSlice::narrow(arcs);
+    const int64_t vo = B->vtx_off[b], nb = B->vtx_off[b + 1] - vo;
+    const bool narrow = bcg::TileSlice::narrow(pairs[b]);
     unsigned char *base = blob.data() + off[b];
     uint16_t *C = reinterpret_cast<uint16_t *>(base + bcg::TileSlice::col_at(nb, narrow));
+    int64_t at = 0;
     for (int64_t v = 0; v <= nb; ++v) {
-      if (narrow) reinterpret_cast<uint16_t *>(base)[v] = (uint16_t)(B->row[vo + v] - e0);
-      else reinterpret_cast<int32_t *>(base)[v] = (int32_t)(B->row[vo + v] - e0);
+      if (narrow) reinterpret_cast<uint16_t *>(base)[v] = (uint16_t)(at / 2);
+      else reinterpret_cast<int32_t *>(base)[v] = (int32_t)(at / 2);
+      if (v == nb) break;
+      for (int64_t e = B->row[vo + v]; e < B->row[vo + v + 1]; ++e) C[at++] = (uint16_t)B->col[e];
+      if (at & 1) C[at++] = (uint16_t)v;
     }
-    for (int64_t e = 0; e < arcs; ++e) C[e] = (uint16_t)B->col[e0 + e];
-  }
-  std::vector<int64_t> off_flag(off);  // what the kernels read: offset | narrow
-  for (int32_t b = 0; b < B->n_bcc; ++b) {
-    if (off[b] < 0) continue;
-    const int64_t vo = B->vtx_off[b], nb = B->vtx_off[b + 1] - vo;
-    if (bcg::TileSlice::narrow(B->row[vo + nb] - B->row[vo])) off_flag[b] |= 1;
+    if (narrow) off_flag[b] |= 1;
   }
   p->n_titems = (int64_t)p->h_titems.size();
   int warp_grid = 1;
@@ -897,16 +907,14 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
       p->unit_visits.push_back(p->unit_visits.back() + src * nb);
     }
     // PLAIN: items of the BCCs that fit shared memory go to the small-BCC
-    // kernels (sources of an item: its own vertex, then its chains'). With a
-    // rescaling threshold of the caller's, which those do not apply, they go
-    // to the whole-BCC kernel, whose sums are the same bit for bit, so that a
-    // threshold never changes BC. Rows in shared memory instead of L2, and a BFS per chain
-    // vertex instead of a merge and a double listing: a chain-endpoint call on
-    // a BCC of 1,494 vertices went from 1.95 to 0.66 ms, 1,194 sources.
+    // kernels (sources of an item: its own vertex, then its chains'). Their path
+    // counts stay below 2^1000 and need no rescaling, whatever the threshold.
+    // Rows in shared memory instead of L2, and a BFS per chain vertex instead of
+    // a merge and a double listing: a chain-endpoint call on a BCC of 1,494
+    // vertices went from 1.95 to 0.66 ms, 1,194 sources.
     const bool listed = p->unit_sources.back() - p->unit_sources[(size_t)p->n_bat] < INT32_MAX;
     std::vector<int8_t> small((size_t)B->n_bcc, -1), core((size_t)B->n_bcc, 0);
     std::vector<int32_t> small_ecc;
-    const bool scaled = ctx->opts.rescale_exp != 0;
     if (p->mode == BCGPU_MODE_PLAIN && p->n_items > 0 && listed)
       route_tiles(ctx, B, std::vector<char>((size_t)B->n_bcc, 0), small, small_ecc, true);
     p->ws_n = (p->mode == BCGPU_MODE_PLAIN ? nb_max : nb_plain) + 2;
@@ -981,7 +989,7 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
       p->src_at.push_back((int64_t)src.size());
       p->core_at.push_back((int64_t)csrc.size());
       p->item_at.push_back((int64_t)rest.size());
-      const bool t = small[it.bcc] >= 0 && !scaled;
+      const bool t = small[it.bcc] >= 0;
       if (!t && !core[it.bcc]) {
         rest.push_back(it);
         continue;

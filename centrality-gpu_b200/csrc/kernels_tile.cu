@@ -7,20 +7,22 @@
 // BCC's size; on a batch of thousands of small graphs the CTAs then wait on
 // global-memory latency at every arc. Here a BCC that fits shared memory is
 // run from shared memory only:
-//  * the slice (local row offsets, 16-bit neighbour ids; tile.h TileSlice) is
+//  * the slice (row offsets, 16-bit neighbour ids in pairs; tile.h TileSlice) is
 //    brought in by one cp.async.bulk (a plain bulk copy from this GPU's global
 //    memory into this CTA's shared memory, completion on an mbarrier whose wait
 //    is bounded) and serves every source of the item;
 //  * levels, path counts (then q in place) and the visit order of each source
 //    live in shared memory: one set per warp in the warp class (a warp per
 //    source, eight in flight), one per source group in the CTA class (the
-//    whole CTA on one source, or, for BCCs whose single-source CTA fits only
-//    once or twice per SM, two or four groups of a 1024-thread CTA on their
-//    own sources from the one slice);
+//    whole CTA on one source, or eight, four or two groups of a 1024-thread CTA
+//    on their own sources from the one slice, wherever their arrays fit);
 //  * forward: level-synchronous, each frontier vertex pulls sigma from its
-//    predecessors and claims its successors in one scan of its row -- a row of
-//    up to kLaneDeg arcs by one lane (four arcs' loads in flight), a longer one
-//    by a whole warp (lanes over arcs, then a fixed-order warp sum);
+//    predecessors and claims its successors in one scan of its row. Warp class:
+//    a row of up to kLaneDeg arcs by one lane, a longer one by the warp. CTA
+//    class: by one thread, by kSub lanes or by a warp (kLightPairs,
+//    kMediumPairs); on a level that holds 1 / kWide of the BCC, successors are
+//    stamped with plain stores and collected by a pass over the stamps, since
+//    claiming them one by one was two thirds of a source's time;
 //  * backward: successor form, q(w) = (reach(w)+1+delta(w))/sigma(w) and
 //    delta(v) = sigma(v) * sum q (Codes/kernels_free.cu:391,409), q
 //    overwriting sigma in place;
@@ -51,10 +53,25 @@ namespace bcg {
 namespace {
 
 constexpr int kThreads = kTileWarps * 32;
-constexpr int kLaneDeg = 8;  // rows up to this many arcs: one lane; longer rows: a whole warp
-// CTA class: long rows of a level queued for the whole CTA (a row beyond the
-// queue's room is scanned at once by the warp that found it).
+constexpr int kLaneDeg = 8;  // warp class: rows up to this many arcs: one lane; longer rows: the warp
+// CTA class, rows in pairs of arcs: up to kLightPairs by one thread as its vertex
+// comes up; up to kMediumPairs queued for kSub lanes; longer ones queued for a
+// warp; a row beyond the queues' room by the thread that found it, with the same
+// sum. BA graphs: six
+// vertices in seven have up to four arcs, and the hubs hold a third of the arcs.
+constexpr int kLightPairs = 4;
+constexpr int kMediumPairs = 16;
+constexpr int kSub = 4;
 constexpr int kLongQueue = 1024;
+// A level of at least 1 / kWide of the BCC's vertices does not claim its
+// successors one by one: it stamps them (the same value whoever stores it) and
+// then collects the stamped ones with a pass over all stamps. BA batches of 30
+// graphs of 4,500-5,000 and 120 of 1,000-1,500 vertices, and the 2,000-vertex
+// graph: 75.4, 23.4 and 0.23 ms with rows of up to 8 arcs by a thread and the
+// others by a warp, every successor claimed; 67.1, 16.3 and 0.35 with the row
+// classes above; 43.9, 10.9, 0.195 / 42.0, 10.4, 0.186 / 41.1, 10.2, 0.182 / 40.5,
+// 10.1, 0.183 stamping from 1/8 / 1/16 / 1/32 / 1/64 of the BCC on.
+constexpr int kWide = 32;
 
 struct Ctl {
   unsigned long long bar;  // mbarrier of the slice copy
@@ -73,10 +90,13 @@ struct WarpLayout {  // ctl | counters [nmax][kAccDigits] | per warp: d [nmax], 
 };
 // CTA class: kBlock threads in kBlock / kGroup groups, each group on its own
 // sources with its own arrays and barrier, all groups on the one staged slice.
-// ctl | per group: sq [nmax] | d int16 [nmax] | S uint16 [nmax] | lv [kLevels]
-//     | long-row queue [kQueue] | counters cnt[4], nq[4] | slice
-// (one group: levels and queue of the class limits; several: the smaller
+// ctl | per group: sq [nmax] | d uint16 [nmax] | S uint16 [nmax] | lv uint16
+//     [kLevels] | queues of medium and long rows uint16 [kQueue] each | Counts |
+// slice (one group: levels and queues of the class limits; several: the smaller
 // limits of the grouped classes, tile.h).
+struct Counts {  // by level mod 3
+  int found[3], medium[3], large[3], pad[3];
+};
 template <int kBlock, int kGroup>
 struct CtaLayout {
   static constexpr int kG = kBlock / kGroup;
@@ -85,9 +105,9 @@ struct CtaLayout {
   __host__ __device__ static int64_t d(int64_t nmax) { return align16(8 * nmax); }
   __host__ __device__ static int64_t S(int64_t nmax) { return d(nmax) + align16(2 * nmax); }
   __host__ __device__ static int64_t lv(int64_t nmax) { return S(nmax) + align16(2 * nmax); }
-  __host__ __device__ static int64_t q(int64_t nmax) { return lv(nmax) + align16(4 * kLevels); }
-  __host__ __device__ static int64_t ctr(int64_t nmax) { return q(nmax) + align16(4 * kQueue); }
-  __host__ __device__ static int64_t group_bytes(int64_t nmax) { return ctr(nmax) + align16(8 * sizeof(int)); }
+  __host__ __device__ static int64_t q(int64_t nmax) { return lv(nmax) + align16(2 * kLevels); }
+  __host__ __device__ static int64_t ctr(int64_t nmax) { return q(nmax) + align16(2 * 2 * kQueue); }
+  __host__ __device__ static int64_t group_bytes(int64_t nmax) { return ctr(nmax) + align16(sizeof(Counts)); }
   __host__ __device__ static int64_t group(int g, int64_t nmax) { return align16(sizeof(Ctl)) + g * group_bytes(nmax); }
   __host__ __device__ static int64_t slice(int64_t nmax) { return group(kG, nmax); }
   // the group's barrier: the CTA's own when the group is the CTA, else named barrier g+1
@@ -145,7 +165,9 @@ struct View {
   const uint16_t *R16;  // set for a narrow slice
   const uint16_t *C;
   const int32_t *rch;
-  __device__ __forceinline__ int row(int32_t w) const { return R16 ? (int)R16[w] : R32[w]; }
+  __device__ __forceinline__ int pair(int32_t w) const { return R16 ? (int)R16[w] : R32[w]; }  // w's first pair
+  __device__ __forceinline__ int row(int32_t w) const { return 2 * pair(w); }                  // w's first arc
+  __device__ __forceinline__ uint32_t two(int p) const { return reinterpret_cast<const uint32_t *>(C)[p]; }
 };
 
 // Pulls the next item for the CTA (thread 0) and stages its BCC's slice if
@@ -212,11 +234,8 @@ __device__ __forceinline__ void append(ST *S, int *tail, int32_t x) {
 }
 
 // Claims unvisited vertex x (level -1) for level lev; true for the one claim
-// that wins. Levels are int32 (warp class) or int16 (CTA class).
+// that wins.
 __device__ __forceinline__ bool claim(int32_t *d, int32_t x, int lev) { return atomicCAS(d + x, -1, lev) == -1; }
-__device__ __forceinline__ bool claim(int16_t *d, int32_t x, int lev) {
-  return atomicCAS(reinterpret_cast<unsigned short *>(d + x), (unsigned short)0xffffu, (unsigned short)lev) == 0xffffu;
-}
 
 // Forward scan of one row by one thread (four arcs' loads in flight, sums in
 // arc order): pulls sigma from level dprev, claims unvisited vertices for
@@ -289,11 +308,12 @@ __device__ __forceinline__ double push_row_warp(const View &g, int e0, int e1, c
   return warp_sum(acc);
 }
 
-// delta and q of w from the successors' sum; returns delta (q overwrites sigma).
-__device__ __forceinline__ double finish(const View &g, int32_t w, double sum, double *sq, int *err) {
+// delta and q of w from the successors' sum, r = reach(w) + 1; returns delta (q
+// overwrites sigma).
+__device__ __forceinline__ double finish(double r, int32_t w, double sum, double *sq, int *err) {
   const double sw = sq[w];
   const double delta = sw * sum;
-  const double qw = ((double)__ldg(g.rch + w) + 1.0 + delta) / sw;
+  const double qw = (r + delta) / sw;
   // counts past 2^1000 too: their q would lose bits below FP64's normal range
   if (exp_bits(qw) == 0x7ff || exp_bits(delta) == 0x7ff || (unsigned)(exp_bits(sw) - 1) >= 1023 + 1000)
     set_err(err, kDevOverflow);
@@ -380,7 +400,7 @@ __device__ void warp_sweep(const View &g, int nlev, const int32_t *d, double *sq
         if (lane == j) sum = part;
       }
       if (w >= 0) {
-        const double delta = finish(g, w, sum, sq, err);  // this level's q: read by the level above only
+        const double delta = finish((double)__ldg(g.rch + w) + 1.0, w, sum, sq, err);  // this level's q: read by the level above only
         if (delta != 0.0) acc_add(cnt + (int64_t)kAccDigits * w, delta * wsrc, err);
       }
     }
@@ -433,153 +453,285 @@ __global__ void __launch_bounds__(kThreads, 1) tile_warp_kernel(TileArgs a) {
 
 // ======================================================== CTA per source ===
 
-// BFS of one group (the whole CTA, or a fixed share of its threads) from s,
-// two group barriers per level: the frontier's rows of up to kLaneDeg arcs
-// are scanned by one thread each (chunks of a level are independent: they
-// read the previous level only) while longer rows are queued; after a
-// barrier the group's warps share the queued rows; a second barrier ends the
-// level. Queue and tail counters of level l are cnt[l % 3] and nq[l % 3];
-// those of level l+1 are cleared at the start of level l, two barriers after
-// their last reader.
+// What one group of threads works on. Levels are stamped base + level, so that
+// the next source finds every stamp stale (below its base) and clears nothing.
+struct Group {
+  double *sq;       // path counts, then q
+  uint16_t *d, *S;  // stamps; vertices by level
+  uint16_t *lv;     // level offsets into S
+  uint16_t *medium, *large;
+  Counts *n;
+  int base;
+};
+
+// Claims unvisited vertex x (stamp below base) with stamp `next`: a CAS on the
+// word of two stamps, again while only the other one changed.
+__device__ __forceinline__ bool claim(const Group &G, int32_t x, int next) {
+  unsigned *word = reinterpret_cast<unsigned *>(G.d) + (x >> 1);
+  const int sh = (x & 1) * 16;
+  unsigned old = *reinterpret_cast<volatile unsigned *>(word);
+  while ((int)(old >> sh & 0xffffu) < G.base) {
+    const unsigned was = atomicCAS(word, old, (old & ~(0xffffu << sh)) | (unsigned)next << sh);
+    if (was == old) return true;
+    old = was;
+  }
+  return false;
+}
+
+// Pairs p0, p0 + step, ... < p1 of a row, two at a time, forward: the path
+// counts of the neighbours on the level before (stamp prev); the others that
+// have none yet are stamped for the next level -- on a wide level just that, else
+// claimed, and appended to S from f1 on.
+__device__ __forceinline__ double fwd_pairs(const View &g, const Group &G, int p0, int p1, int step, int prev, bool wide,
+                                            int f1, int *found) {
+  double sum = 0.0;
+  for (; p0 < p1; p0 += 2 * step) {
+    const uint32_t a = g.two(p0), b = p0 + step < p1 ? g.two(p0 + step) : a;
+    const int32_t x[4] = {(int32_t)(a & 0xffffu), (int32_t)(a >> 16), (int32_t)(b & 0xffffu), (int32_t)(b >> 16)};
+    int dx[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) dx[j] = G.d[x[j]];
+    if (p0 + step >= p1) dx[2] = dx[3] = 0xffff;  // no second pair: neither found nor to be claimed
+    double v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = dx[j] == prev ? G.sq[x[j]] : 0.0;
+    if (wide) {  // uniform over the group
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (dx[j] < G.base) *(volatile uint16_t *)(G.d + x[j]) = (uint16_t)(prev + 2);
+    } else {
+      uint32_t won = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (dx[j] < G.base && claim(G, x[j], prev + 2)) won |= 1u << j;
+      if (won) {
+        int at = f1 + atomicAdd(found, __popc(won));
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (won >> j & 1u) G.S[at++] = (uint16_t)x[j];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum += v[j];
+  }
+  return sum;
+}
+
+// Appends the vertices with stamp `stamp` to S from f1 on, eight stamps to a
+// load, in a group of kGroup threads.
+template <int kGroup>
+__device__ __forceinline__ void collect(const Group &G, int nb, int stamp, int f1, int *found, int tid) {
+  const int lane = tid & 31;
+  for (int c = 0; c < nb; c += 8 * kGroup) {  // uniform over the group
+    const int v0 = c + 8 * tid;
+    uint4 q = make_uint4(0, 0, 0, 0);  // stamps are never 0
+    if (v0 < nb) q = *reinterpret_cast<const uint4 *>(G.d + v0);
+    const unsigned w[4] = {q.x, q.y, q.z, q.w};
+    uint32_t hit = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if ((int)(w[j] & 0xffffu) == stamp) hit |= 1u << (2 * j);
+      if ((int)(w[j] >> 16) == stamp) hit |= 2u << (2 * j);
+    }
+    if (nb - v0 < 8) hit &= v0 < nb ? (1u << (nb - v0)) - 1 : 0;  // places beyond the BCC hold anything
+    const int mine = __popc(hit);
+    int upto = mine;  // of the lanes up to this one
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += y;
+    }
+    int at = 0;
+    if (lane == 31 && upto) at = atomicAdd(found, upto);
+    at = f1 + __shfl_sync(0xffffffffu, at, 31) + upto - mine;
+    for (; hit; hit &= hit - 1) G.S[at++] = (uint16_t)(v0 + __ffs(hit) - 1);
+  }
+}
+
+// The same backward: the sum of q over the neighbours on the level after.
+__device__ __forceinline__ double bwd_pairs(const View &g, const Group &G, int p0, int p1, int step, int next) {
+  double sum = 0.0;
+  for (; p0 < p1; p0 += 2 * step) {
+    const uint32_t a = g.two(p0), b = p0 + step < p1 ? g.two(p0 + step) : a;
+    const int32_t x[4] = {(int32_t)(a & 0xffffu), (int32_t)(a >> 16), (int32_t)(b & 0xffffu), (int32_t)(b >> 16)};
+    int dx[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) dx[j] = G.d[x[j]];
+    if (p0 + step >= p1) dx[2] = dx[3] = 0;
+    double v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = dx[j] == next ? G.sq[x[j]] : 0.0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum += v[j];
+  }
+  return sum;
+}
+
+// A row that found its queue full, by one thread: what `width` lanes give and
+// their butterfly sums up to, so that the sum does not depend on the order in
+// which a level's rows were queued.
+template <class Row>
+__device__ __forceinline__ double row_alone(int p0, int p1, Row row) {
+  const int width = p1 - p0 <= kMediumPairs ? kSub : 32;
+  double half[6];  // sums of 1, 2, 4, ... lanes waiting for their other half
+  double sum = 0.0;
+  for (int i = 0; i < width; ++i) {
+    // warp_sum adds lanes 16 apart first, queued_rows' sums neighbours first
+    sum = row(p0 + (width == 32 ? (int)(__brev(i) >> 27) : i), p1, width);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      if (!(i >> k & 1)) {
+        half[k] = sum;
+        break;
+      }
+      sum = half[k] + sum;
+    }
+  }
+  return sum;
+}
+
+// Queues a row of `pairs` for several lanes; false if it has to be done here.
+template <class L>
+__device__ __forceinline__ bool queue_row(const Group &G, int m, int32_t w, int pairs) {
+  if (pairs <= kLightPairs) return false;
+  int *n = pairs <= kMediumPairs ? &G.n->medium[m] : &G.n->large[m];
+  const int at = atomicAdd(n, 1);
+  if (at >= L::kQueue) return false;
+  (pairs <= kMediumPairs ? G.medium : G.large)[at] = (uint16_t)w;
+  return true;
+}
+
+// The queued rows of a level: kSub lanes each, then a warp each. row(first pair,
+// end, step) gives a lane's sum, done(w, sum) takes the total in one lane.
+template <class L, int kGroup, class Row, class Done>
+__device__ __forceinline__ void queued_rows(const View &g, const Group &G, int nm, int nl, int tid, Row row, Done done) {
+  const int sub = tid % kSub, lane = tid & 31;
+  for (int c = 0; c < nm; c += kGroup / kSub) {
+    const int k = c + tid / kSub;
+    const int32_t w = k < nm ? G.medium[k] : 0;
+    double sum = k < nm ? row(g.pair(w) + sub, g.pair(w + 1), kSub) : 0.0;
+#pragma unroll
+    for (int o = 1; o < kSub; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (k < nm && sub == 0) done(w, sum);
+  }
+  for (int k = tid >> 5; k < nl; k += kGroup / 32) {
+    const int32_t w = G.large[k];
+    const double sum = warp_sum(row(g.pair(w) + lane, g.pair(w + 1), 32));
+    if (lane == 0) done(w, sum);
+  }
+}
+
+// BFS of one group (the whole CTA, or a fixed share of its threads) from s: one
+// group barrier per level, one more where rows were queued, and on a wide level.
+// Counts of level l are at
+// l % 3; those of level l+1 are cleared at the start of level l, two barriers
+// after their last reader. Returns the number of levels, -1 on an error.
 template <int kBlock, int kGroup>
-__device__ int cta_bfs(const View &g, int32_t nb, int32_t s, int16_t *d, double *sq, uint16_t *S, int32_t *lv,
-                       int32_t *q, int *cnt, int *nq, int *err, int grp, int tid) {
+__device__ int cta_bfs(const View &g, const Group &G, int nb, int32_t s, int *err, int grp, int tid) {
   using L = CtaLayout<kBlock, kGroup>;
-  constexpr int kWarps = kGroup / 32;
-  const int lane = tid & 31, warp = tid >> 5;
-  for (int v = tid; v < nb; v += kGroup) d[v] = -1;
+  if (tid < 3) {
+    G.n->found[tid] = 0;
+    G.n->medium[tid] = 0;
+    G.n->large[tid] = 0;
+  }
   if (tid == 0) {
-    cnt[0] = 0;
-    cnt[1] = 0;
-    nq[0] = 0;
-    nq[1] = 0;
+    G.d[s] = (uint16_t)G.base;
+    G.S[0] = (uint16_t)s;
+    G.lv[0] = 0;
+    G.lv[1] = 1;
   }
   L::sync(grp);
-  if (tid == 0) {
-    d[s] = 0;
-    S[0] = (uint16_t)s;
-    sq[s] = 1.0;
-    lv[0] = 0;
-    lv[1] = 1;
-  }
-  L::sync(grp);
-  int lev = 0, f0 = 0, f1 = 1;
+  int lev = 0, m = 0, f0 = 0, f1 = 1;
   while (true) {
-    const int dprev = lev == 0 ? INT_MIN : lev - 1, dnext = lev + 1;
-    int *tail = cnt + lev % 3, *nql = nq + lev % 3;
+    const int nxt = m == 2 ? 0 : m + 1;
     if (tid == 0) {
-      cnt[(lev + 1) % 3] = 0;
-      nq[(lev + 1) % 3] = 0;
+      G.n->found[nxt] = 0;
+      G.n->medium[nxt] = 0;
+      G.n->large[nxt] = 0;
     }
-    for (int c0 = f0; c0 < f1; c0 += kGroup) {  // uniform over the group
-      const int i = c0 + tid;
-      int32_t w = -1, e0 = 0, e1 = 0;
-      if (i < f1) {
-        w = S[i];
-        e0 = g.row(w);
-        e1 = g.row(w + 1);
-      }
-      const bool big = e1 - e0 > kLaneDeg;
-      if (w >= 0 && !big) {
-        const double acc = pull_row(g, e0, e1, d, sq, S + f1, tail, dprev, dnext);
-        if (lev > 0) sq[w] = acc;
-      }
-      bool mine = false;  // a long row the queue had no room for
-      if (w >= 0 && big) {
-        const int pos = atomicAdd(nql, 1);
-        if (pos < L::kQueue) q[pos] = w;
-        else mine = true;
-      }
-      uint32_t over = __ballot_sync(0xffffffffu, mine);
-      while (over) {
-        const int j = __ffs(over) - 1;
-        over &= over - 1;
-        const int32_t wj = __shfl_sync(0xffffffffu, w, j);
-        const double acc = pull_row_warp(g, g.row(wj), g.row(wj + 1), d, sq, S + f1, tail, dprev, dnext, lane);
-        if (lane == 0 && lev > 0) sq[wj] = acc;
-      }
+    const int prev = G.base + lev - 1;  // no stamp of this source on the source's own level
+    int *found = &G.n->found[m];
+    const bool wide = (f1 - f0) * kWide >= nb;
+    for (int i = f0 + tid; i < f1; i += kGroup) {
+      const int32_t w = G.S[i];
+      const int p0 = g.pair(w), p1 = g.pair(w + 1);
+      if (queue_row<L>(G, m, w, p1 - p0)) continue;
+      auto row = [&](int q0, int q1, int step) { return fwd_pairs(g, G, q0, q1, step, prev, wide, f1, found); };
+      const double sum = p1 - p0 <= kLightPairs ? row(p0, p1, 1) : row_alone(p0, p1, row);
+      G.sq[w] = lev ? sum : 1.0;
     }
     L::sync(grp);
-    const int nlong = min(*(volatile int *)nql, L::kQueue);
-    for (int k = warp; k < nlong; k += kWarps) {
-      const int32_t w = q[k];
-      const double acc = pull_row_warp(g, g.row(w), g.row(w + 1), d, sq, S + f1, tail, dprev, dnext, lane);
-      if (lane == 0 && lev > 0) sq[w] = acc;
+    const int nm = min(*(volatile int *)&G.n->medium[m], L::kQueue), nl = min(*(volatile int *)&G.n->large[m], L::kQueue);
+    if (nm | nl) {
+      queued_rows<L, kGroup>(
+          g, G, nm, nl, tid, [&](int p0, int p1, int step) { return fwd_pairs(g, G, p0, p1, step, prev, wide, f1, found); },
+          [&](int32_t w, double sum) { G.sq[w] = lev ? sum : 1.0; });
+      L::sync(grp);
     }
-    L::sync(grp);
-    const int t = f1 + *(volatile int *)tail;
+    if (wide) {
+      collect<kGroup>(G, nb, prev + 2, f1, found, tid);
+      L::sync(grp);
+    }
+    const int t = f1 + *(volatile int *)found;
     if (t == f1) break;
     if (lev + 2 >= L::kLevels) {  // uniform; routing keeps BCCs below this depth
       if (tid == 0) set_err(err, kDevWorkspace);
       return -1;
     }
-    if (tid == 0) lv[lev + 2] = t;
+    if (tid == 0) G.lv[lev + 2] = (uint16_t)t;
     f0 = f1;
     f1 = t;
     ++lev;
+    m = nxt;
   }
   return lev + 1;
 }
 
 // One source's contribution c to vertex w: to the group's FP64 row P (one
-// writer per vertex and source), or straight into the BCC's fixed-point
-// counters when there is no row.
+// writer per vertex and source; an addition at L2, so that no load is waited
+// for), or straight into the BCC's fixed-point counters when there is no row.
 __device__ __forceinline__ void contribute(double *P, unsigned long long *acc, int32_t w, double c, int *err) {
-  if (P) P[w] += c;
+  if (P) atomicAdd(P + w, c);
   else if (c != 0.0) acc_add(acc + (int64_t)kAccDigits * w, c, err);
 }
 
-// Dependency sweep of one group, two group barriers per level as in cta_bfs;
-// each vertex's contribution is made by one thread.
+// Dependency sweep of one group, barriers as in cta_bfs; each vertex's
+// contribution is made by one thread.
 template <int kBlock, int kGroup>
-__device__ void cta_sweep(const View &g, int nlev, const int16_t *d, double *sq, const uint16_t *S, const int32_t *lv,
-                          int32_t *q, int *nq, double wsrc, double *P, unsigned long long *acc, int *err, int grp,
-                          int tid) {
+__device__ void cta_sweep(const View &g, const Group &G, int nlev, double wsrc, double *P, unsigned long long *acc, int *err,
+                          int grp, int tid) {
   using L = CtaLayout<kBlock, kGroup>;
-  constexpr int kWarps = kGroup / 32;
-  const int lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) {
-    nq[0] = 0;
-    nq[1] = 0;
+  L::sync(grp);  // the last level's counts have been read
+  if (tid < 3) {
+    G.n->medium[tid] = 0;
+    G.n->large[tid] = 0;
   }
   L::sync(grp);
-  for (int lev = nlev - 1, k3 = 0; lev >= 1; --lev, k3 = (k3 + 1) % 3) {
-    const int dsucc = lev + 1, a0 = lv[lev], a1 = lv[lev + 1];
-    int *nql = nq + k3;
-    if (tid == 0) nq[(k3 + 1) % 3] = 0;
-    for (int c0 = a0; c0 < a1; c0 += kGroup) {  // uniform over the group
-      const int i = c0 + tid;
-      int32_t w = -1, e0 = 0, e1 = 0;
-      if (i < a1) {
-        w = S[i];
-        e0 = g.row(w);
-        e1 = g.row(w + 1);
-      }
-      const bool big = e1 - e0 > kLaneDeg;
-      if (w >= 0 && !big) contribute(P, acc, w, finish(g, w, push_row(g, e0, e1, d, sq, dsucc), sq, err) * wsrc, err);
-      bool mine = false;
-      if (w >= 0 && big) {
-        const int pos = atomicAdd(nql, 1);
-        if (pos < L::kQueue) q[pos] = w;
-        else mine = true;
-      }
-      uint32_t over = __ballot_sync(0xffffffffu, mine);
-      while (over) {
-        const int j = __ffs(over) - 1;
-        over &= over - 1;
-        const int32_t wj = __shfl_sync(0xffffffffu, w, j);
-        const double sum = push_row_warp(g, g.row(wj), g.row(wj + 1), d, sq, dsucc, lane);
-        if (lane == 0) contribute(P, acc, wj, finish(g, wj, sum, sq, err) * wsrc, err);
-      }
+  for (int lev = nlev - 1, m = 0; lev >= 1; --lev, m = m == 2 ? 0 : m + 1) {
+    const int nxt = m == 2 ? 0 : m + 1, next = G.base + lev + 1, a1 = G.lv[lev + 1];
+    if (tid == 0) {
+      G.n->medium[nxt] = 0;
+      G.n->large[nxt] = 0;
+    }
+    for (int i = G.lv[lev] + tid; i < a1; i += kGroup) {
+      const int32_t w = G.S[i];
+      const int p0 = g.pair(w), p1 = g.pair(w + 1);
+      if (queue_row<L>(G, m, w, p1 - p0)) continue;
+      const double r = (double)__ldg(g.rch + w) + 1.0;
+      auto row = [&](int q0, int q1, int step) { return bwd_pairs(g, G, q0, q1, step, next); };
+      const double sum = p1 - p0 <= kLightPairs ? row(p0, p1, 1) : row_alone(p0, p1, row);
+      contribute(P, acc, w, finish(r, w, sum, G.sq, err) * wsrc, err);
     }
     L::sync(grp);
-    const int nlong = min(*(volatile int *)nql, L::kQueue);
-    for (int k = warp; k < nlong; k += kWarps) {
-      const int32_t w = q[k];
-      const double sum = push_row_warp(g, g.row(w), g.row(w + 1), d, sq, dsucc, lane);
-      if (lane == 0) contribute(P, acc, w, finish(g, w, sum, sq, err) * wsrc, err);
+    const int nm = min(*(volatile int *)&G.n->medium[m], L::kQueue), nl = min(*(volatile int *)&G.n->large[m], L::kQueue);
+    if (nm | nl) {
+      queued_rows<L, kGroup>(
+          g, G, nm, nl, tid, [&](int p0, int p1, int step) { return bwd_pairs(g, G, p0, p1, step, next); },
+          [&](int32_t w, double sum) {
+            contribute(P, acc, w, finish((double)__ldg(g.rch + w) + 1.0, w, sum, G.sq, err) * wsrc, err);
+          });
+      L::sync(grp);
     }
-    L::sync(grp);
   }
 }
 
@@ -598,12 +750,15 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) tile_cta_kernel(TileArg
   unsigned char *mine = s_raw + L::group(grp, nmax);
   // the group's FP64 row (global, L2-resident), if the launch has them
   double *P = a.ws_P ? a.ws_P + ((int64_t)blockIdx.x * L::kG + grp) * a.cap_P : nullptr;
-  double *sq = reinterpret_cast<double *>(mine);
-  int16_t *d = reinterpret_cast<int16_t *>(mine + L::d(nmax));
-  uint16_t *S = reinterpret_cast<uint16_t *>(mine + L::S(nmax));
-  int32_t *lv = reinterpret_cast<int32_t *>(mine + L::lv(nmax));
-  int32_t *q = reinterpret_cast<int32_t *>(mine + L::q(nmax));
-  int *cnt = reinterpret_cast<int *>(mine + L::ctr(nmax)), *nq = cnt + 4;
+  Group G;
+  G.sq = reinterpret_cast<double *>(mine);
+  G.d = reinterpret_cast<uint16_t *>(mine + L::d(nmax));
+  G.S = reinterpret_cast<uint16_t *>(mine + L::S(nmax));
+  G.lv = reinterpret_cast<uint16_t *>(mine + L::lv(nmax));
+  G.medium = reinterpret_cast<uint16_t *>(mine + L::q(nmax));
+  G.large = G.medium + L::kQueue;
+  G.n = reinterpret_cast<Counts *>(mine + L::ctr(nmax));
+  G.base = 1 << 16;  // the first source clears the stamps
   unsigned char *slice = s_raw + L::slice(nmax);
   const int tid = threadIdx.x;
   if (tid == 0) {
@@ -617,22 +772,29 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) tile_cta_kernel(TileArg
   int32_t nb;
   while (next_item(a, ctl, slice, phase, it, vo, nb)) {
     if (P)
-      for (int v = gtid; v < nb; v += kGroup) P[v] = 0.0;
+      for (int v = gtid; v < nb; v += kGroup) __stcg(P + v, 0.0);
     __syncthreads();
     if (tid == 0) ctl.bcc = it.bcc;  // read again only after the next barrier
     const View g = view_of(a, slice, nb, vo, it.bcc);
     unsigned long long *acc = a.acc + (int64_t)kAccDigits * vo;
     for (int32_t k = it.s0 + grp; k < it.s1; k += L::kG) {  // the group's sources in order: P's sums are fixed
       const int32_t s = source_of(a, k);
-      const int nlev = cta_bfs<kBlock, kGroup>(g, nb, s, d, sq, S, lv, q, cnt, nq, a.err, grp, gtid);
+      if (G.base + L::kLevels + 2 > 0xffff) {  // stamps start over
+        for (int v = gtid; v < (int)((nmax + 1) / 2); v += kGroup) reinterpret_cast<unsigned *>(G.d)[v] = 0;
+        G.base = 2;
+        L::sync(grp);
+      }
+      const int nlev = cta_bfs<kBlock, kGroup>(g, G, nb, s, a.err, grp, gtid);
       if (nlev < 0) break;
-      cta_sweep<kBlock, kGroup>(g, nlev, d, sq, S, lv, q, nq, (double)__ldg(g.rch + s) + 1.0, P, acc, a.err, grp,
-                                gtid);
+      cta_sweep<kBlock, kGroup>(g, G, nlev, (double)__ldg(g.rch + s) + 1.0, P, acc, a.err, grp, gtid);
+      G.base += nlev + 1;
     }
     __syncthreads();
     if (!P) continue;  // uniform over the grid
-    for (int v = gtid; v < nb; v += kGroup)
-      if (P[v] != 0.0) acc_add(acc + (int64_t)kAccDigits * v, P[v], a.err);
+    for (int v = gtid; v < nb; v += kGroup) {
+      const double c = __ldcg(P + v);
+      if (c != 0.0) acc_add(acc + (int64_t)kAccDigits * v, c, a.err);
+    }
   }
 }
 
@@ -646,11 +808,12 @@ size_t tile_smem_bytes(int cls, int64_t nmax, int64_t slice_max) {
                        : cls == kTileCta512   ? CtaLayout<512, 512>::slice(nmax)
                        : cls == kTileCta1024  ? CtaLayout<1024, 1024>::slice(nmax)
                        : cls == kTileCta1024x2 ? CtaLayout<1024, 512>::slice(nmax)
-                                              : CtaLayout<1024, 256>::slice(nmax);
+                       : cls == kTileCta1024x4 ? CtaLayout<1024, 256>::slice(nmax)
+                                              : CtaLayout<1024, 128>::slice(nmax);
   return (size_t)(head + align16(slice_max));
 }
 
-int tile_groups(int cls) { return cls == kTileCta1024x2 ? 2 : cls == kTileCta1024x4 ? 4 : 1; }
+int tile_groups(int cls) { return cls == kTileCta1024x2 ? 2 : cls == kTileCta1024x4 ? 4 : cls == kTileCta1024x8 ? 8 : 1; }
 
 // At most kItemSources: the CTA runs them (a warp each, or one after another)
 // from one staged slice; larger BCCs are split so that many CTAs share them, and
@@ -668,6 +831,7 @@ int tile_class(int64_t n, int64_t slice_bytes, size_t lim) {
   if (n > kTileMaxVertices) return -1;
   if (n <= kTileWarpMaxVertices) return fits(kTileWarp) ? kTileWarp : -1;
   const int64_t per = kTileSmPerSm / ((int64_t)tile_smem_bytes(kTileCta, n, slice_bytes) + kTileReserved);
+  if (per <= 7 && fits(kTileCta1024x8)) return kTileCta1024x8;
   if (per >= 4) return kTileCta;
   if (fits(kTileCta1024x4)) return kTileCta1024x4;
   if (per == 3) return kTileCta;
@@ -689,7 +853,8 @@ const void *tile_fn(int cls) {
          : cls == kTileCta512   ? reinterpret_cast<const void *>(tile_cta_kernel<512, 512>)
          : cls == kTileCta1024  ? reinterpret_cast<const void *>(tile_cta_kernel<1024, 1024>)
          : cls == kTileCta1024x2 ? reinterpret_cast<const void *>(tile_cta_kernel<1024, 512>)
-                                : reinterpret_cast<const void *>(tile_cta_kernel<1024, 256>);
+         : cls == kTileCta1024x4 ? reinterpret_cast<const void *>(tile_cta_kernel<1024, 256>)
+                                : reinterpret_cast<const void *>(tile_cta_kernel<1024, 128>);
 }
 }  // namespace
 
@@ -711,6 +876,7 @@ cudaError_t launch_tile(int cls, const TileArgs &a, int grid, size_t smem, cudaS
     case kTileCta1024: tile_cta_kernel<1024, 1024><<<grid, 1024, smem, stream>>>(a); break;
     case kTileCta1024x2: tile_cta_kernel<1024, 512><<<grid, 1024, smem, stream>>>(a); break;
     case kTileCta1024x4: tile_cta_kernel<1024, 256><<<grid, 1024, smem, stream>>>(a); break;
+    case kTileCta1024x8: tile_cta_kernel<1024, 128><<<grid, 1024, smem, stream>>>(a); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

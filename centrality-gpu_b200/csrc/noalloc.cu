@@ -131,26 +131,44 @@ __global__ void setup_kernel(Layout L, const int32_t *R, const int32_t *C, int32
   }
 }
 
+// First pair of row i, which starts at arc r, in a slice laid out without a
+// prefix sum: rows get the pairs they need, some one more.
+__host__ __device__ __forceinline__ int64_t slice_pair(int64_t r, int64_t i) { return (r + i + 1) / 2; }
+
 // The same for the small-BCC kernels: the BCC's slice, and items of per sources
 // each. The same checks; the kernels take no work after an error.
 __global__ void slice_kernel(unsigned char *base, Layout L, const int32_t *R, const int32_t *C, int32_t n, int32_t m,
                              const int32_t *src, int32_t nsrc, int32_t per) {
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const bool narrow = TileSlice::narrow(m);
+  const bool narrow = TileSlice::narrow(slice_pair(m, n));
   unsigned char *slice = base + kOffSlice;
   uint16_t *col = reinterpret_cast<uint16_t *>(slice + TileSlice::col_at(n, narrow));
-  for (int64_t i = tid; i <= n; i += stride) {
-    const int32_t r = R[i];
-    if (r < 0 || r > m || (i == 0 && r != 0) || (i == n && r != m) || (i < n && R[i + 1] < r))
-      set_err(L.err, kDevBadItem);
-    if (narrow) reinterpret_cast<uint16_t *>(slice)[i] = (uint16_t)r;
-    else reinterpret_cast<int32_t *>(slice)[i] = r;
-  }
-  for (int64_t e = tid; e < m; e += stride) {
-    const int32_t c = C[e];
-    if (c < 0 || c >= n) set_err(L.err, kDevBadItem);
-    col[e] = (uint16_t)c;
+  for (int64_t i = tid / 32; i <= n; i += stride / 32) {  // a warp per row
+    const int lane = (int)(tid & 31);
+    const int32_t r = R[i], r1 = i < n ? R[i + 1] : m;
+    if (r < 0 || r > m || (i == 0 && r != 0) || (i == n && r != m) || r1 < r || r1 > m) {
+      if (lane == 0) set_err(L.err, kDevBadItem);
+      continue;
+    }
+    const int64_t p = slice_pair(r, i);
+    if (lane == 0) {
+      if (narrow) reinterpret_cast<uint16_t *>(slice)[i] = (uint16_t)p;
+      else reinterpret_cast<int32_t *>(slice)[i] = (int32_t)p;
+    }
+    if (i == n) continue;
+    const int64_t places = 2 * (slice_pair(r1, i + 1) - p);
+    for (int64_t j = lane; j < places; j += 32) {
+      int32_t c = (int32_t)i;  // a spare place
+      if (j < r1 - r) {
+        c = C[r + j];
+        if (c < 0 || c >= n) {
+          set_err(L.err, kDevBadItem);
+          c = 0;
+        }
+      }
+      col[2 * p + j] = (uint16_t)c;
+    }
   }
   for (int64_t i = tid; i < nsrc; i += stride)
     if (src[i] < 0 || src[i] >= n) set_err(L.err, kDevBadItem);
@@ -162,7 +180,7 @@ __global__ void slice_kernel(unsigned char *base, Layout L, const int32_t *R, co
     L.vtx_off[1] = n;
     *L.counter = 0;
     *reinterpret_cast<int64_t *>(base + kOffTileMeta) = narrow ? 1 : 0;
-    *reinterpret_cast<int32_t *>(base + kOffTileMeta + 8) = (int32_t)TileSlice::bytes(n, m);
+    *reinterpret_cast<int32_t *>(base + kOffTileMeta + 8) = (int32_t)TileSlice::bytes(n, slice_pair(m, n));
   }
 }
 
@@ -222,7 +240,7 @@ cudaError_t enqueue(unsigned char *base, const Layout &L, int cls, size_t smem, 
     a.ws_lv = reinterpret_cast<int32_t *>(base + kOffTileLv);
     a.cap = n + 2;
     a.nmax = n;
-    a.slice_max = (int32_t)TileSlice::bytes(n, m);
+    a.slice_max = (int32_t)TileSlice::bytes(n, slice_pair(m, n));
     a.wait_ns = kDefaultWaitNs;
     a.err = L.err;
     e = launch_tile(cls, a, (int)std::min<int64_t>(grid, a.item_end), smem, stream);
@@ -285,11 +303,12 @@ extern "C" int bc_begin_free_noalloc(bc_ctx *ctx, const int32_t *R, const int32_
   const Layout L = layout(base, n);
   // the small-BCC kernels where the BCC fits; their level offsets have to fit
   // the array too
-  int cls = m <= INT32_MAX / 4 ? tile_class(n, TileSlice::bytes(n, m), tile_smem_limit(dev)) : -1;
+  const int64_t slice = TileSlice::bytes(n, slice_pair(m, n));
+  int cls = m <= INT32_MAX / 4 ? tile_class(n, slice, tile_smem_limit(dev)) : -1;
   size_t smem = 0;
   int grid = 0, sms = 0;
   if (cls >= 0) {
-    smem = tile_smem_bytes(cls, n, TileSlice::bytes(n, m));
+    smem = tile_smem_bytes(cls, n, slice);
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
       grid = sms * tile_ctas_per_sm(cls, smem);
     if (cls == kTileWarp) grid = (int)std::min<int64_t>(grid, kBytesTileLv / (4 * kTileWarps * (int64_t)(n + 2)));

@@ -25,29 +25,32 @@ struct TileItem {
 // kTileCta1024x2 / kTileCta1024x4: 1024 threads in two groups of 512 / four
 // of 256, each group on its own source with its own arrays, every group on
 // the one staged slice: two / four sources in flight per SM for BCCs whose
-// single-source CTA fits only once or twice per SM.
+// single-source CTA fits only once or twice per SM. kTileCta1024x8: eight groups
+// of 128, for BCCs whose levels are too narrow for wider groups.
 enum TileClass : int { kTileWarp = 0, kTileCta = 1, kTileCta512 = 2, kTileCta1024 = 3, kTileCta1024x2 = 4,
-                       kTileCta1024x4 = 5 };
+                       kTileCta1024x4 = 5, kTileCta1024x8 = 6 };
 constexpr int kTileWarps = 8;          // warps per CTA
 constexpr int kTileMaxLevels = 1024;   // BFS levels the CTA class records (routing keeps BCCs below)
 constexpr int kTileGroupMaxLevels = 256;  // the same for the grouped classes
-constexpr int kGroupLongQueue = 256;      // long-row queue of a group in the grouped classes
+constexpr int kGroupLongQueue = 256;      // long-row queues of a group in the grouped classes
 constexpr int64_t kTileWarpMaxVertices = 640;  // BCCs of up to this many vertices take the warp class
 constexpr int64_t kTileSmPerSm = 228 * 1024, kTileReserved = 1024;  // shared memory per SM, per-CTA reserve
 constexpr int32_t kTileMaxVertices = 65535;  // neighbour ids are 16-bit in the slice
 
 // Byte layout of one BCC's staged slice, each part starting on a 16-byte
-// boundary: local row offsets [n+1] -- uint16 when the BCC has fewer than
-// 2^16 arcs ("narrow", 2 bytes per vertex less in shared memory), else
-// int32 -- then neighbours uint16 [arcs]. A slice's offset in the slice
-// buffer is a multiple of 16; bit 0 of the offset recorded for the kernels
-// (TileArgs::slice_off) marks a narrow slice.
+// boundary: row offsets [n+1] in pairs of arcs -- uint16 with fewer than 2^16
+// pairs ("narrow", 2 bytes per vertex less in shared memory), else int32 -- then
+// neighbours uint16, two per pair, so that a row is read four bytes at a time.
+// A row's spare places hold the vertex itself, which is on no level that a scan
+// of its row looks for. A slice's offset in the slice buffer is a multiple of
+// 16; bit 0 of the offset recorded for the kernels (TileArgs::slice_off) marks a
+// narrow slice.
 struct TileSlice {
   __host__ __device__ static int64_t pad16(int64_t bytes) { return (bytes + 15) / 16 * 16; }
-  __host__ __device__ static bool narrow(int64_t arcs) { return arcs < 65536; }
+  __host__ __device__ static bool narrow(int64_t pairs) { return pairs < 65536; }
   __host__ __device__ static int64_t col_at(int64_t n, bool narrow) { return pad16((narrow ? 2 : 4) * (n + 1)); }
-  __host__ __device__ static int64_t bytes(int64_t n, int64_t arcs) {
-    return col_at(n, narrow(arcs)) + pad16(2 * arcs);
+  __host__ __device__ static int64_t bytes(int64_t n, int64_t pairs) {
+    return col_at(n, narrow(pairs)) + pad16(4 * pairs);
   }
 };
 

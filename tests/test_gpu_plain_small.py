@@ -1,8 +1,8 @@
-"""PLAIN plans whose BCCs fit shared memory run them on the small-BCC kernels
-(the others on the per-source kernel): the same BC bit for bit. A context with
-an explicit rescaling threshold (2^900, the default one) keeps every BCC on the
-per-source kernel, which is what the routed plans are compared with; the BC
-of both is the oracle's."""
+"""PLAIN plans whose BCCs fit shared memory run them on the small-BCC kernels:
+whole runs against the oracle, unit ranges against the contracted per-source
+kernel (a BATCHED plan without small-BCC items has the same units), over the
+classes of those kernels and the edges of their queues, level tables and slice
+forms; the same bits again on a second run."""
 import numpy as np
 import pytest
 
@@ -53,31 +53,30 @@ CASES = {
 
 
 @pytest.mark.parametrize("name", list(CASES))
-def test_plain_routes_give_the_same_bits(name):
+def test_plain_routes(name):
     P = pkg()
     n, u, v = CASES[name]()
     d = P.Decomposition(P.Graph.from_edges(n, u, v))
-    got = {}
-    for tag, rx in (("routed", 0), ("per-source", 900)):
-        ctx = P.Context(mode=P.MODE_PLAIN, rescale_exp=rx)
+    got = []
+    for opts in (dict(mode=P.MODE_PLAIN), dict(mode=P.MODE_BATCHED, plain_core=1 << 30, tile_max=-1), dict(mode=P.MODE_PLAIN)):
+        ctx = P.Context(**opts)
         plan = ctx.plan(d)
         k = plan.n_units
-        parts = [(0, k)] if name == "too-large" else [(0, k), (k // 3, 2 * k // 3), (k - 1, k), (0, 0)]
-        if name == "too-large":
-            parts = [(0, min(k, 600))]
-        got[tag] = []
+        parts = [(0, min(k, 600))] if name == "too-large" else [(0, k), (k // 3, 2 * k // 3), (k - 1, k), (0, 0)]
+        got.append([])
         for a, b in parts:
             plan.reset()
             plan.run(a, b)
-            got[tag].append(plan.read())
+            got[-1].append(plan.read())
         plan.close()
         ctx.close()
-    for x, y in zip(got["routed"], got["per-source"]):
-        assert np.array_equal(x, y)
+    for x, y, z in zip(*got):
+        assert np.array_equal(x, z)
+        assert rel_err(x, y) < TOL
     if name != "too-large":
         O = oracle()
         row, col = O.csr(n, u, v)
-        assert rel_err(got["routed"][0], O.brandes(n, row, col)) < TOL
+        assert rel_err(got[0][0], O.brandes(n, row, col)) < TOL
 
 
 @pytest.mark.parametrize("repeat", [1, 3])
