@@ -374,7 +374,8 @@ class Plan:
     def tile_launches(self):
         """[(class, grid)] of the small-BCC schedule's launches, in launch order
         (class: 0 warp per source; 1, 2, 3 one source per 256-, 512-, 1024-thread
-        CTA; 4, 5 a 1024-thread CTA of two / four source groups)."""
+        CTA; 4, 5 a 1024-thread CTA of two / four source groups; 6, 7, 8 a 1024-,
+        512-, 256-thread CTA of eight source groups)."""
         n = lib().bc_plan_tile_launches(self._h, None, None, 0)
         if n < 0:
             raise BcError(-n, "bc_plan_tile_launches")

@@ -526,8 +526,9 @@ bool core_takes(const bc_bccs *B, int32_t b, std::vector<int32_t> &dist, std::ve
 // 4 or more / 3 per SM; a 1024-thread CTA of four source groups (when four
 // groups' arrays and the slice fit, and the BCC fits that class's level
 // table); 512-thread CTAs at 2 per SM; a 1024-thread CTA of two groups; one
-// 1024-thread CTA per SM; a 1024-thread CTA of eight groups, wherever it fits.
-// Each bucket's items are contiguous.
+// 1024-thread CTA per SM; CTAs of eight groups, where they fit, which leaves the
+// warp class the BCCs with too many levels for the groups' tables. Each bucket's
+// items are contiguous.
 // With a source list (PLAIN plans: src, each BCC's sources from list[b] on)
 // the items hold places in it, and contributions go straight into the
 // fixed-point counters, so that BC is bit for bit what the per-source kernel
@@ -543,10 +544,11 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
   std::vector<int32_t> size((size_t)B->n_bcc, 0);
   std::vector<int8_t> bucket((size_t)B->n_bcc, -1);
   // bucket k -> class: 0 warp, 1 / 2 CTA (4+ / 3 per SM), 3 four groups, 4 CTA-512, 5 two groups, 6 CTA-1024,
-  // 7 eight groups
-  constexpr int kBuckets = 8;
+  // 7 eight groups of 128, 8 of 64, 9 of 32
+  constexpr int kBuckets = 10;
   constexpr int kBucketCls[kBuckets] = {bcg::kTileWarp,   bcg::kTileCta,       bcg::kTileCta,     bcg::kTileCta1024x4,
-                                        bcg::kTileCta512, bcg::kTileCta1024x2, bcg::kTileCta1024, bcg::kTileCta1024x8};
+                                        bcg::kTileCta512, bcg::kTileCta1024x2, bcg::kTileCta1024, bcg::kTileCta1024x8,
+                                        bcg::kTileCta512x8, bcg::kTileCta256x8};
   const int64_t lim = (int64_t)bcg::tile_smem_limit(ctx->device);
   std::vector<int64_t> per((size_t)B->n_bcc, 0), pairs((size_t)B->n_bcc, 0);
   for (int32_t b = 0; b < B->n_bcc; ++b) {
@@ -564,7 +566,7 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
   auto promote = [&](int to, auto &&eligible) {
     std::vector<int32_t> cand;
     for (int32_t b = 0; b < B->n_bcc; ++b) {
-      if (cls[b] < 0 || cls[b] == bcg::kTileWarp || !eligible(b)) continue;
+      if (cls[b] < 0 || !eligible(b)) continue;
       const int64_t nb = B->vtx_off[b + 1] - B->vtx_off[b];
       if (2 * (int64_t)ecc_of[b] + 3 >= bcg::kTileGroupMaxLevels) continue;  // levels <= 2 ecc + 1
       if ((int64_t)bcg::tile_smem_bytes(kBucketCls[to], nb, size[b]) > lim) continue;
@@ -582,9 +584,18 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
       bucket[b] = (int8_t)to;
     }
   };
-  promote(7, [&](int32_t b) { return per[b] <= 7; });                    // eight sources in flight, not at most seven
-  promote(3, [&](int32_t b) { return per[b] <= 3 && bucket[b] != 7; });  // four, not at most three
-  promote(5, [&](int32_t b) { return per[b] <= 1 && bucket[b] == 6; });  // two instead of one
+  // Small BCCs: eight groups of a warp, of two warps, of four -- wherever they
+  // fit, and where one-source CTAs would not have eight in flight either. ms for
+  // BA batches of 280-430 / 430-570 / 860-1,140 / 1,290-1,570 vertices: groups of
+  // 32 1.90 / 3.05 / 11.4 / 15.1, of 64 2.28 / 2.93 / 7.3 / 9.3, of 128 (from 900
+  // on) - / - / 9.8 / 8.5; the warp class 2.75 / 5.36 for the first two.
+  auto size_of = [&](int32_t b) { return B->vtx_off[b + 1] - B->vtx_off[b]; };
+  auto grouped = [&](int32_t b) { return bucket[b] >= 7; };
+  promote(9, [&](int32_t b) { return size_of(b) <= bcg::kTileGroups32; });
+  promote(8, [&](int32_t b) { return size_of(b) <= bcg::kTileGroups64 && !grouped(b); });
+  promote(7, [&](int32_t b) { return cls[b] != bcg::kTileWarp && per[b] <= 7 && !grouped(b); });
+  promote(3, [&](int32_t b) { return cls[b] != bcg::kTileWarp && per[b] <= 3 && !grouped(b); });  // four, not at most three
+  promote(5, [&](int32_t b) { return cls[b] != bcg::kTileWarp && per[b] <= 1 && bucket[b] == 6; });  // two instead of one
   int64_t total = 0, p_rows = 1;
   for (int k = 0; k < kBuckets; ++k) {
     bc_plan::TileLaunch T;

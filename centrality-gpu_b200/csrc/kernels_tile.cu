@@ -101,7 +101,7 @@ template <int kBlock, int kGroup>
 struct CtaLayout {
   static constexpr int kG = kBlock / kGroup;
   static constexpr int kLevels = kG == 1 ? kTileMaxLevels : kTileGroupMaxLevels;
-  static constexpr int kQueue = kG == 1 ? kLongQueue : kGroupLongQueue;
+  static constexpr int kQueue = kG == 1 ? kLongQueue : kGroup < 128 ? kGroup : kGroupLongQueue;
   __host__ __device__ static int64_t d(int64_t nmax) { return align16(8 * nmax); }
   __host__ __device__ static int64_t S(int64_t nmax) { return d(nmax) + align16(2 * nmax); }
   __host__ __device__ static int64_t lv(int64_t nmax) { return S(nmax) + align16(2 * nmax); }
@@ -114,6 +114,8 @@ struct CtaLayout {
   __device__ __forceinline__ static void sync(int g) {
     if constexpr (kG == 1) {
       __syncthreads();
+    } else if constexpr (kGroup == 32) {
+      __syncwarp();
     } else {
       asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(kGroup) : "memory");
     }
@@ -800,7 +802,9 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) tile_cta_kernel(TileArg
 
 }  // namespace
 
-int block_of(int cls) { return cls >= kTileCta1024 ? 1024 : cls == kTileCta512 ? 512 : kThreads; }
+int block_of(int cls) {
+  return cls == kTileCta512 || cls == kTileCta512x8 ? 512 : cls >= kTileCta1024 && cls <= kTileCta1024x8 ? 1024 : kThreads;
+}
 
 size_t tile_smem_bytes(int cls, int64_t nmax, int64_t slice_max) {
   const int64_t head = cls == kTileWarp       ? WarpLayout::slice(nmax)
@@ -809,11 +813,13 @@ size_t tile_smem_bytes(int cls, int64_t nmax, int64_t slice_max) {
                        : cls == kTileCta1024  ? CtaLayout<1024, 1024>::slice(nmax)
                        : cls == kTileCta1024x2 ? CtaLayout<1024, 512>::slice(nmax)
                        : cls == kTileCta1024x4 ? CtaLayout<1024, 256>::slice(nmax)
-                                              : CtaLayout<1024, 128>::slice(nmax);
+                       : cls == kTileCta1024x8 ? CtaLayout<1024, 128>::slice(nmax)
+                       : cls == kTileCta512x8  ? CtaLayout<512, 64>::slice(nmax)
+                                               : CtaLayout<256, 32>::slice(nmax);
   return (size_t)(head + align16(slice_max));
 }
 
-int tile_groups(int cls) { return cls == kTileCta1024x2 ? 2 : cls == kTileCta1024x4 ? 4 : cls == kTileCta1024x8 ? 8 : 1; }
+int tile_groups(int cls) { return cls == kTileCta1024x2 ? 2 : cls == kTileCta1024x4 ? 4 : cls >= kTileCta1024x8 ? 8 : 1; }
 
 // At most kItemSources: the CTA runs them (a warp each, or one after another)
 // from one staged slice; larger BCCs are split so that many CTAs share them, and
@@ -829,6 +835,8 @@ int32_t tile_item_sources(int cls, int64_t grid, int64_t sources) {
 int tile_class(int64_t n, int64_t slice_bytes, size_t lim) {
   auto fits = [&](int cls) { return tile_smem_bytes(cls, n, slice_bytes) <= lim; };
   if (n > kTileMaxVertices) return -1;
+  if (n <= kTileGroups32 && fits(kTileCta256x8)) return kTileCta256x8;
+  if (n <= kTileGroups64 && fits(kTileCta512x8)) return kTileCta512x8;
   if (n <= kTileWarpMaxVertices) return fits(kTileWarp) ? kTileWarp : -1;
   const int64_t per = kTileSmPerSm / ((int64_t)tile_smem_bytes(kTileCta, n, slice_bytes) + kTileReserved);
   if (per <= 7 && fits(kTileCta1024x8)) return kTileCta1024x8;
@@ -854,7 +862,9 @@ const void *tile_fn(int cls) {
          : cls == kTileCta1024  ? reinterpret_cast<const void *>(tile_cta_kernel<1024, 1024>)
          : cls == kTileCta1024x2 ? reinterpret_cast<const void *>(tile_cta_kernel<1024, 512>)
          : cls == kTileCta1024x4 ? reinterpret_cast<const void *>(tile_cta_kernel<1024, 256>)
-                                : reinterpret_cast<const void *>(tile_cta_kernel<1024, 128>);
+         : cls == kTileCta1024x8 ? reinterpret_cast<const void *>(tile_cta_kernel<1024, 128>)
+         : cls == kTileCta512x8  ? reinterpret_cast<const void *>(tile_cta_kernel<512, 64>)
+                                 : reinterpret_cast<const void *>(tile_cta_kernel<256, 32>);
 }
 }  // namespace
 
@@ -877,6 +887,8 @@ cudaError_t launch_tile(int cls, const TileArgs &a, int grid, size_t smem, cudaS
     case kTileCta1024x2: tile_cta_kernel<1024, 512><<<grid, 1024, smem, stream>>>(a); break;
     case kTileCta1024x4: tile_cta_kernel<1024, 256><<<grid, 1024, smem, stream>>>(a); break;
     case kTileCta1024x8: tile_cta_kernel<1024, 128><<<grid, 1024, smem, stream>>>(a); break;
+    case kTileCta512x8: tile_cta_kernel<512, 64><<<grid, 512, smem, stream>>>(a); break;
+    case kTileCta256x8: tile_cta_kernel<256, 32><<<grid, 256, smem, stream>>>(a); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

@@ -2,10 +2,10 @@
 // takes a range of sources of one BCC small enough for shared memory, stages
 // the BCC's CSR slice there with one bulk copy, and keeps every per-source
 // array in shared memory too. Two classes:
-//   kTileWarp  one warp per source (eight sources in flight per CTA), for the
-//              smallest BCCs;
-//   kTileCta   the whole CTA on one source at a time, for BCCs up to several
-//              thousand vertices.
+//   kTileWarp  one warp per source (eight sources in flight per CTA), its level
+//              offsets in global memory, for small BCCs of many levels;
+//   kTileCta   the whole CTA, or a group of its threads, on one source at a
+//              time, for BCCs up to several thousand vertices.
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -26,14 +26,17 @@ struct TileItem {
 // of 256, each group on its own source with its own arrays, every group on
 // the one staged slice: two / four sources in flight per SM for BCCs whose
 // single-source CTA fits only once or twice per SM. kTileCta1024x8: eight groups
-// of 128, for BCCs whose levels are too narrow for wider groups.
+// of 128, for BCCs whose levels are too narrow for wider groups; kTileCta512x8 and
+// kTileCta256x8: eight groups of 64 and of a warp, for smaller ones still, two and
+// four CTAs per SM.
 enum TileClass : int { kTileWarp = 0, kTileCta = 1, kTileCta512 = 2, kTileCta1024 = 3, kTileCta1024x2 = 4,
-                       kTileCta1024x4 = 5, kTileCta1024x8 = 6 };
+                       kTileCta1024x4 = 5, kTileCta1024x8 = 6, kTileCta512x8 = 7, kTileCta256x8 = 8 };
 constexpr int kTileWarps = 8;          // warps per CTA
 constexpr int kTileMaxLevels = 1024;   // BFS levels the CTA class records (routing keeps BCCs below)
 constexpr int kTileGroupMaxLevels = 256;  // the same for the grouped classes
 constexpr int kGroupLongQueue = 256;      // long-row queues of a group in the grouped classes
 constexpr int64_t kTileWarpMaxVertices = 640;  // BCCs of up to this many vertices take the warp class
+constexpr int64_t kTileGroups32 = 640, kTileGroups64 = 1200;  // largest BCCs for groups of 32, of 64 threads
 constexpr int64_t kTileSmPerSm = 228 * 1024, kTileReserved = 1024;  // shared memory per SM, per-CTA reserve
 constexpr int32_t kTileMaxVertices = 65535;  // neighbour ids are 16-bit in the slice
 

@@ -239,7 +239,8 @@ int64_t bc_plan_unit_sources(const bc_plan *plan, int64_t begin, int64_t end, in
 int64_t bc_plan_device_bytes(const bc_plan *plan);
 /* The small-BCC schedule's launches, in launch order: each one's CTA class
  * (0 warp per source; 1, 2, 3: one source per 256-, 512-, 1024-thread CTA;
- * 4, 5: a 1024-thread CTA of two / four source groups) and grid size. Writes
+ * 4, 5: a 1024-thread CTA of two / four source groups; 6, 7, 8: a 1024-, 512-,
+ * 256-thread CTA of eight source groups) and grid size. Writes
  * up to cap entries; returns the number of launches (negative error code on
  * failure). Introspection for tests and tools; no reference counterpart. */
 int bc_plan_tile_launches(const bc_plan *plan, int32_t *cls, int32_t *grid, int32_t cap);

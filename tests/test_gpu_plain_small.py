@@ -22,6 +22,12 @@ def cycle_with_chords(n, chords, seed):
     return (n,) + graphs().simple_edges(n, u, v)
 
 
+def ladder(rungs):
+    i = np.arange(rungs)
+    return (2 * rungs,) + graphs().simple_edges(2 * rungs, np.concatenate([i[:-1], rungs + i[:-1], i]),
+                                                np.concatenate([i[1:], rungs + i[1:], rungs + i]))
+
+
 def star_and_grid():
     """A hub row far longer than a warp next to a BCC of many levels (too deep
     for the classes with short level tables) and one-cycle BCCs."""
@@ -30,12 +36,7 @@ def star_and_grid():
     wheel = (400,) + G.simple_edges(400, np.concatenate([np.zeros(399, int), hub]),
                                     np.concatenate([hub, np.roll(hub, 1)]))
     ring = (700,) + G.simple_edges(700, np.arange(700), (np.arange(700) + 1) % 700)
-    ladder_n = 1200  # 600 rungs: 600 levels
-    i = np.arange(600)
-    lu = np.concatenate([i[:-1], 600 + i[:-1], i])
-    lv = np.concatenate([i[1:], 600 + i[1:], 600 + i])
-    ladder = (ladder_n,) + G.simple_edges(ladder_n, lu, lv)
-    return G.pack_graphs([wheel, ring, ladder, (3,) + G.simple_edges(3, [0, 1, 2], [1, 2, 0])])[:3]
+    return G.pack_graphs([wheel, ring, ladder(600), (3,) + G.simple_edges(3, [0, 1, 2], [1, 2, 0])])[:3]
 
 
 CASES = {
@@ -44,6 +45,9 @@ CASES = {
     "cta-class": lambda: cycle_with_chords(641, 500, 3),
     "wide-rows": lambda: cycle_with_chords(300, 12000, 4),
     "int32-offsets": lambda: cycle_with_chords(800, 40000, 5),
+    "groups-of-64": lambda: cycle_with_chords(1200, 1500, 9),
+    "groups-of-128": lambda: cycle_with_chords(1201, 1500, 10),
+    "deep-small": lambda: ladder(300),
     "mid": lambda: cycle_with_chords(2900, 5000, 6),
     "large": lambda: cycle_with_chords(6500, 9000, 7),
     "too-large": lambda: cycle_with_chords(17000, 6000, 8),
