@@ -12,6 +12,7 @@
 #include "core.h"
 #include "internal.h"
 #include "plain.h"
+#include "team.h"
 #include "tile.h"
 
 #include <algorithm>
@@ -20,6 +21,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <new>
 #include <set>
 #include <string>
@@ -280,6 +282,9 @@ int validate(bc_ctx *ctx, const bc_bccs *B) {
   }
   return BCGPU_OK;
 }
+
+// Workspace that a plan takes without asking for the free memory first.
+constexpr int64_t kUnasked = 1 << 24;
 
 // Bytes of the fixed-point BC counters of n packed vertices, as dalloc sizes them.
 size_t acc_bytes(int64_t n) {
@@ -845,10 +850,16 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
     return bail(cuda_fail(ctx, cudaGetLastError(), "cudaMemsetAsync"));
   HOST_MARK("uploads");
 
-  size_t free_b = 0, total_b = 0;
-  CK(ctx, cudaMemGetInfo(&free_b, &total_b));
-  const double avail_b = (double)free_b + (double)pool_spare(ctx);
-  int64_t limit = ctx->opts.workspace_limit > 0 ? ctx->opts.workspace_limit : (int64_t)(0.8 * avail_b);
+  // Device bytes the plan may take. The free memory is asked for only where the
+  // answer can matter (70 us, a third of a call on a graph of 60 vertices).
+  int64_t limit = ctx->opts.workspace_limit;
+  auto free_limit = [&]() -> int {
+    if (limit > 0) return BCGPU_OK;
+    size_t free_b = 0, total_b = 0;
+    CK(ctx, cudaMemGetInfo(&free_b, &total_b));
+    limit = (int64_t)(0.8 * ((double)free_b + (double)pool_spare(ctx)));
+    return BCGPU_OK;
+  };
   // BATCHED: BCCs off the multi-source passes that fit the small-BCC schedule
   std::vector<int8_t> tile;
   std::vector<int32_t> tile_ecc;
@@ -868,6 +879,7 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
     plain_items(B, items, &skip);
   }
   if (p->mode == BCGPU_MODE_BATCHED && n_on > 0) {
+    if ((rc = free_limit())) return bail(rc);
     bcg::BatchedConfig cfg;
     cfg.width = ctx->opts.batch_width;
     cfg.delta_fp32c = ctx->opts.delta == BCGPU_DELTA_FP32C;
@@ -933,7 +945,16 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
     // Four 256-thread CTAs per SM (four sources in flight) when their rows
     // fit the budget, else two of 512, else one of 1024 per SM; with
     // plain_ctas_per_sm 8 or 16, CTAs of 128 or 64 threads are tried first.
-    int64_t avail = limit - p->device_bytes - 64 * (int64_t)ctx->sms;
+    // Where every item is a small BCC's, the slot of the row export is all there
+    // is to hold: a few of those are allocated without asking what is free.
+    const bool all_small = p->mode == BCGPU_MODE_PLAIN &&
+                           std::none_of(items.begin(), items.end(), [&](const auto &it) { return small[it.bcc] < 0; });
+    if (!all_small || 2 * per_slot > kUnasked) {
+      if ((rc = free_limit())) return bail(rc);
+    } else if (limit <= 0) {
+      limit = INT64_MAX;
+    }
+    const int64_t avail = limit - p->device_bytes - 64 * (int64_t)ctx->sms;
     if (avail < 2 * per_slot) return bail(fail(ctx, BCGPU_ENOMEM, "workspace for the largest BCC exceeds the limit"));
     int grid = 0;
     const int first = ctx->opts.plain_ctas_per_sm > 4 ? 1024 / ctx->opts.plain_ctas_per_sm : 256;
@@ -1054,6 +1075,7 @@ int create_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem>
   bc_plan *p = nullptr;
   int rc;
   try {
+    const bcg::SmallTeam team(B ? B->n_packed : 0, B ? B->n_arcs : 0);
     rc = validate(ctx, B);
     if (rc == BCGPU_OK) {
       const cudaError_t e = cudaSetDevice(ctx->device);
@@ -1135,9 +1157,11 @@ extern "C" int bc_create(const bc_opts *opts, bc_ctx **out) {
   if (dev < 0) {  // highest compute capability, as the reference's choose_device (Codes/begin_gpupgm.cu:8-39)
     int best = -1;
     for (int i = 0; i < count; ++i) {
-      cudaDeviceProp pr;
-      if (cudaGetDeviceProperties(&pr, i) != cudaSuccess) continue;
-      int cc = pr.major * 10 + pr.minor;
+      int major = 0, minor = 0;
+      if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, i) != cudaSuccess ||
+          cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, i) != cudaSuccess)
+        continue;
+      const int cc = major * 10 + minor;
       if (cc > best) { best = cc; dev = i; }
     }
   }
@@ -1152,14 +1176,20 @@ extern "C" int bc_create(const bc_opts *opts, bc_ctx **out) {
     return BCGPU_ECUDA;
   };
   if ((e = cudaSetDevice(dev)) != cudaSuccess) return bad(e, "cudaSetDevice");
-  cudaDeviceProp pr;
-  if ((e = cudaGetDeviceProperties(&pr, dev)) != cudaSuccess) return bad(e, "cudaGetDeviceProperties");
-  if (pr.major < 10) {
-    g_create_err = std::string("device ") + pr.name + " is not sm_100 (kernels are built for sm_100a only)";
-    bc_destroy(ctx);
-    return BCGPU_ECUDA;
+  // attributes, not the whole property record: that takes 2.5 ms to fill
+  int major = 0;
+  if ((e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev)) != cudaSuccess ||
+      (e = cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+    return bad(e, "cudaDeviceGetAttribute");
+  if (major < 10) {
+    cudaDeviceProp pr;
+    if ((e = cudaGetDeviceProperties(&pr, dev)) != cudaSuccess) return bad(e, "cudaGetDeviceProperties");
+    if (pr.major < 10) {
+      g_create_err = std::string("device ") + pr.name + " is not sm_100 (kernels are built for sm_100a only)";
+      bc_destroy(ctx);
+      return BCGPU_ECUDA;
+    }
   }
-  ctx->sms = pr.multiProcessorCount;
   if (o.stream) ctx->stream = (cudaStream_t)o.stream;
   else {
     if ((e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess)
@@ -1540,14 +1570,25 @@ extern "C" int bc_plan_read(bc_plan *p, double *bc_out) {
     CK(p->ctx, cudaSetDevice(p->ctx->device));
     int rc = check_dev_err(p);
     if (rc) return rc;
-    std::vector<double> packed((size_t)p->n_packed);
+    const std::unique_ptr<double[]> packed(new double[(size_t)p->n_packed]);  // not cleared: the copy fills it
     if (p->n_packed)
-      CK(p->ctx, cudaMemcpyAsync(packed.data(), p->bc, sizeof(double) * (size_t)p->n_packed, cudaMemcpyDeviceToHost,
+      CK(p->ctx, cudaMemcpyAsync(packed.get(), p->bc, sizeof(double) * (size_t)p->n_packed, cudaMemcpyDeviceToHost,
                                  p->ctx->stream));
     CK(p->ctx, cudaStreamSynchronize(p->ctx->stream));
     p->d2h_bytes += (int64_t)sizeof(double) * p->n_packed;
-    for (int32_t v = 0; v < p->n_orig; ++v) bc_out[v] = p->art.empty() ? 0.0 : p->art[v];
-    for (int64_t k = 0; k < p->n_packed; ++k) bc_out[p->orig[k]] += packed[k];  // fixed order: deterministic
+    // Each thread folds the vertices it owns and reads the whole list for them: a
+    // vertex's terms are added in packed order, whatever the team.
+    const bcg::SmallTeam team(p->n_orig, p->n_packed);
+#pragma omp parallel
+    {
+      const int64_t T = omp_get_num_threads(), t = omp_get_thread_num();
+      const int32_t lo = (int32_t)(p->n_orig * t / T), hi = (int32_t)(p->n_orig * (t + 1) / T);
+      for (int32_t v = lo; v < hi; ++v) bc_out[v] = p->art.empty() ? 0.0 : p->art[v];
+      for (int64_t k = 0; k < p->n_packed; ++k) {
+        const int32_t v = p->orig[k];
+        if (v >= lo && v < hi) bc_out[v] += packed[k];
+      }
+    }
     return BCGPU_OK;
   });
 }

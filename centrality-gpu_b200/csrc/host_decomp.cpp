@@ -26,6 +26,7 @@
 //    walked directly from their endpoints in O(n_b + m_b).
 #include "bchost.h"
 #include "decomp.h"
+#include "team.h"
 
 #include <algorithm>
 #include <chrono>
@@ -128,6 +129,7 @@ extern "C" int bc_graph_from_edges(int32_t n, int64_t m, const int32_t *u, const
   if (!g) return BCGPU_ENOMEM;
   int rc;
   try {
+    const bcg::SmallTeam team(n, 2 * m);
     rc = build_csr(n, m, u, v, g);
   } catch (const std::bad_alloc &) {
     rc = BCGPU_ENOMEM;
@@ -1130,6 +1132,7 @@ extern "C" int bc_decompose(const bc_graph *g, bc_decomp **out) {
   if (!D) return BCGPU_ENOMEM;
   int rc;
   try {
+    const bcg::SmallTeam team(g->n, (int64_t)g->col.size());
     rc = decompose(g, D);
   } catch (const std::bad_alloc &) {
     rc = BCGPU_ENOMEM;
