@@ -83,21 +83,16 @@ constexpr int kSmallCore = 16384;  // cores below this many vertices use kHeavyD
 constexpr int kChunkArcs = BCGPU_BATCHED_CHUNK;  // arcs per heavy chunk
 constexpr int kHalf = 4;           // words per pass over a vertex row
 // Resident CTAs per SM the kernel is compiled for (registers per thread =
-// 65536 / (kThreads * kMinCtas)) and hit values gathered at once per lane in
-// a row pass; profiling builds may override both. Six CTAs (40 registers,
+// 65536 / (kThreads * kMinCtas)); profiling builds may override it. Six CTAs (40 registers,
 // some spilled to local memory) with the one-arc hit walk measured fastest
 // on RMAT-20 at 512 sources per pass: 135 / 139 / 147 / 124 GTEPS for 4 / 5 /
 // 6 / 8 CTAs per SM.
 #ifndef BCGPU_BATCHED_MIN_CTAS
 #define BCGPU_BATCHED_MIN_CTAS 6
 #endif
-#ifndef BCGPU_BATCHED_GATHER
-#define BCGPU_BATCHED_GATHER 4
-#endif
-// Hit walk of a row pass: n >= 1 = an arc is walked once for all kHalf
-// words of the task (one shuffle of its neighbour), n arcs' values loaded at
-// once (n * kHalf loads in flight); 0 = word by word, BCGPU_BATCHED_GATHER
-// hits at a time. The same terms are added in the same order either way.
+// Hit walk of a row pass: an arc is walked once for all kHalf words of the task
+// (one shuffle of its neighbour), this many arcs' values loaded at once (times
+// kHalf loads in flight).
 #ifndef BCGPU_BATCHED_WALK
 #define BCGPU_BATCHED_WALK 1
 #endif
@@ -109,7 +104,6 @@ constexpr int kMinCtas = BCGPU_BATCHED_MIN_CTAS;
 #define BCGPU_BATCHED_TASKS 32
 #endif
 constexpr int kTasksPerWarp = BCGPU_BATCHED_TASKS;
-constexpr int kGatherHits = BCGPU_BATCHED_GATHER;
 
 // One source of a pass. chain < 0: the core vertex src (level 0). Otherwise
 // src is the chain vertex at position pos of chain `chain` (global index).
@@ -401,7 +395,7 @@ __device__ __forceinline__ T warp_or(T v) {
 template <typename T, bool kComp, int kLev>
 __device__ __forceinline__ void row_pass(const Args &a, const uint32_t *masks, const T *vals, int64_t e0, int64_t e1,
                                          int w0, int nw, const uint32_t (&filt)[kHalf], uint32_t (&any)[kHalf],
-                                         Acc<kComp> (&acc)[kHalf], int lane, int t, int tend = 0) {
+                                         Acc<kComp> (&acc)[kHalf], int lane, int t, bool scaled = false, int tend = 0) {
   const int W = a.W;
   for (int64_t base = e0; base < e1; base += 32) {
     const int64_t e = base + lane;
@@ -423,7 +417,6 @@ __device__ __forceinline__ void row_pass(const Args &a, const uint32_t *masks, c
       f[k] &= filt[k];
       any[k] |= f[k];
     }
-#if BCGPU_BATCHED_WALK
     uint32_t fo = 0;
 #pragma unroll
     for (int k = 0; k < kHalf; ++k) fo |= f[k];
@@ -433,7 +426,7 @@ __device__ __forceinline__ void row_pass(const Args &a, const uint32_t *masks, c
     const int32_t *xb0 = kLev ? a.X + (int64_t)(w0 * 32 + lane) * (a.tcap + 2) : nullptr;
     int xt[kHalf];
 #pragma unroll
-    for (int k = 0; k < kHalf; ++k) xt[k] = (kLev && hits) ? __ldcg(xb0 + k * xs + t) : 0;
+    for (int k = 0; k < kHalf; ++k) xt[k] = (kLev && scaled && hits) ? __ldcg(xb0 + k * xs + t) : 0;
     const T *vrow = vals + (int64_t)w0 * 32 + lane;
     constexpr int kArcs = BCGPU_BATCHED_WALK;  // hit arcs whose values are loaded at once
     while (hits) {  // uniform: arcs with a hit in some word, in arc order
@@ -453,7 +446,7 @@ __device__ __forceinline__ void row_pass(const Args &a, const uint32_t *masks, c
           const uint32_t fj = __shfl_sync(0xffffffffu, f[k], j);
           if ((fj >> lane) & 1u) {
             x[r][k] = __ldcg(vu + k * 32);
-            if (kLev) {
+            if (kLev && scaled) {
               const int xl = __ldcg(xb0 + k * xs + lj);
               x[r][k] = (T)scale2((double)x[r][k], kLev == 1 ? xl - xt[k] : xt[k] - xl);
             }
@@ -465,35 +458,6 @@ __device__ __forceinline__ void row_pass(const Args &a, const uint32_t *masks, c
 #pragma unroll
         for (int k = 0; k < kHalf; ++k) acc[k].add((double)x[r][k]);
     }
-#else
-#pragma unroll
-    for (int k = 0; k < kHalf; ++k) {
-      uint32_t hits = __ballot_sync(0xffffffffu, f[k] != 0u);
-      const T *vk = vals + (int64_t)(w0 + k) * 32 + lane;
-      const int32_t *xb = kLev ? a.X + (int64_t)((w0 + k) * 32 + lane) * (a.tcap + 2) : nullptr;
-      const int xt = kLev ? __ldcg(xb + t) : 0;
-      while (hits) {  // uniform
-        T x[kGatherHits];
-#pragma unroll
-        for (int r = 0; r < kGatherHits; ++r) {
-          x[r] = (T)0;
-          if (hits) {  // uniform
-            const int j = __ffs(hits) - 1;
-            hits &= hits - 1;
-            const uint32_t fj = __shfl_sync(0xffffffffu, f[k], j);
-            const int32_t uj = __shfl_sync(0xffffffffu, u, j);
-            const int lj = kLev ? __shfl_sync(0xffffffffu, lvl, j) : 0;
-            if ((fj >> lane) & 1u) {
-              x[r] = __ldcg(vk + (int64_t)uj * W * 32);
-              if (kLev) x[r] = (T)scale2((double)x[r], kLev == 1 ? __ldcg(xb + lj) - xt : xt - __ldcg(xb + lj));
-            }
-          }
-        }
-#pragma unroll
-        for (int r = 0; r < kGatherHits; ++r) acc[k].add((double)x[r]);
-      }
-    }
-#endif
   }
 }
 
@@ -541,7 +505,7 @@ __device__ __forceinline__ void arm_arcs(const Args &a, int64_t e0, int64_t e1, 
 constexpr int kArcGroup = 4;
 __device__ __forceinline__ int level_index(const Args &a, int d) { return min(max(d, 0), a.tcap + 1); }
 __device__ __forceinline__ void chain_in(const Args &a, const Slot *slots, int nslots, int32_t v, int w, int64_t c0,
-                                         int64_t c1, int lane) {
+                                         int64_t c1, int lane, bool scaled) {
   const int W = a.W;
   const int b = w * 32 + lane;
   const bool live = b < nslots;
@@ -553,7 +517,7 @@ __device__ __forceinline__ void chain_in(const Args &a, const Slot *slots, int n
     A.d = __ldcg(a.d + iv);
     A.s = __ldcg(a.sig + iv);
     sl = slots[b];
-    A.x = __ldcg(xb + level_index(a, A.d));
+    A.x = scaled ? __ldcg(xb + level_index(a, A.d)) : 0;
   }
   double sum = 0.0;
   for (int64_t base = c0; base < c1; base += 32) {
@@ -584,7 +548,7 @@ __device__ __forceinline__ void chain_in(const Args &a, const Slot *slots, int n
         sB[r] = ld ? __ldcg(a.sig + ib) : 1.0;
       }
 #pragma unroll
-      for (int r = 0; r < kArcGroup; ++r) xB[r] = (live && j0 + r < cnt) ? __ldcg(xb + level_index(a, dB[r])) : 0;
+      for (int r = 0; r < kArcGroup; ++r) xB[r] = (scaled && live && j0 + r < cnt) ? __ldcg(xb + level_index(a, dB[r])) : 0;
 #pragma unroll
       for (int r = 0; r < kArcGroup; ++r) {
         if (!live || j0 + r >= cnt) continue;
@@ -619,7 +583,7 @@ __device__ __forceinline__ void chain_in(const Args &a, const Slot *slots, int n
 // delta, q and the BC partial of one (vertex, word) at level lev.
 template <typename QT>
 __device__ __forceinline__ void finish_dep(const Args &a, const Slot *slots, const int32_t *rch, int32_t v, int w,
-                                           int lev, uint32_t act, int lane, double sum, bool chains) {
+                                           int lev, uint32_t act, int lane, double sum, bool chains, bool scaled) {
   constexpr bool kF32 = sizeof(QT) == 4;
   if (!act) return;
   const int W = a.W;
@@ -628,7 +592,7 @@ __device__ __forceinline__ void finish_dep(const Args &a, const Slot *slots, con
     const int b = w * 32 + lane;
     const int64_t idx = ((int64_t)v * W + w) * 32 + lane;
     const double sv = a.sig[idx];
-    const int xd = a.X[(int64_t)b * (a.tcap + 2) + lev] - a.X[(int64_t)b * (a.tcap + 2) + lev + 1];
+    const int xd = scaled ? a.X[(int64_t)b * (a.tcap + 2) + lev] - a.X[(int64_t)b * (a.tcap + 2) + lev + 1] : 0;
     const double delta = scale2(sv * sum, xd) + (chains ? __ldcg(a.cdep + idx) : 0.0);
     const double qv = ((double)rch[v] + 1.0 + delta) / sv;
     if (kF32) {
@@ -804,6 +768,11 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
 
     // ---- forward: levels t -> t+1
     int t = 0, tlast = 0;
+    // Some level so far was rescaled: else every X is 0, and none is read. A slot's
+    // levels are next to each other in X, so that a warp's read of it takes 32
+    // sectors, where the path counts take 8, and waits for the slot's level first:
+    // chain in-flow on R-MAT 20, two passes of 512, 28 -> 22.9 ms without it.
+    bool scaled = false;
     const unsigned long long all_found = (unsigned long long)n * (unsigned long long)bt.nslots;
     while (true) {
       unsigned long long nf = 0;  // pairs this warp found on this level
@@ -833,8 +802,8 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
           const int64_t e0 = hce0[c], e1 = hce1[c], sp = HS[v];
           const int64_t per = (e1 - e0 + kWarpsPerCta - 1) / kWarpsPerCta;
           const int64_t s0 = e0 + wib * per, s1 = min(e1, s0 + per);
-          if (s0 < min(s1, sp)) row_pass<double, false, 0>(a, lmt, a.sig, s0, min(s1, sp), w0, nw, unseen, any, acc, lane, t);
-          if (max(s0, sp) < s1) row_pass<double, false, 1>(a, a.lm, a.sig, max(s0, sp), s1, w0, nw, unseen, any, acc, lane, t);
+          if (s0 < min(s1, sp)) row_pass<double, false, 0>(a, lmt, a.sig, s0, min(s1, sp), w0, nw, unseen, any, acc, lane, t, scaled);
+          if (max(s0, sp) < s1) row_pass<double, false, 1>(a, a.lm, a.sig, max(s0, sp), s1, w0, nw, unseen, any, acc, lane, t, scaled);
         }
 #pragma unroll
         for (int k = 0; k < kHalf; ++k) {
@@ -881,8 +850,8 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
             for (int k = 0; k < kHalf; ++k) { unseen[k] = k < nw ? ~seen[k] : 0u; any[k] = 0; u_any |= unseen[k]; }
             if (!u_any) continue;
             Acc<false> acc[kHalf];
-            if (e0 < sp) row_pass<double, false, 0>(a, lmt, a.sig, e0, sp, w0, nw, unseen, any, acc, lane, t);
-            if (sp < e1) row_pass<double, false, 1>(a, a.lm, a.sig, sp, e1, w0, nw, unseen, any, acc, lane, t);
+            if (e0 < sp) row_pass<double, false, 0>(a, lmt, a.sig, e0, sp, w0, nw, unseen, any, acc, lane, t, scaled);
+            if (sp < e1) row_pass<double, false, 1>(a, a.lm, a.sig, sp, e1, w0, nw, unseen, any, acc, lane, t, scaled);
             int first = 0;
 #pragma unroll
             for (int k = 0; k < kHalf; ++k) {
@@ -983,6 +952,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
         grid_sync(a);
       }
       if (more) tlast = t + 1;
+      scaled = scaled || resc;
       if (cta_failed(a)) break;
       // done when every slot has reached every core vertex (later seeds then
       // reach seen vertices only); else level t+2 needs a non-empty level
@@ -1010,7 +980,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
         const int32_t v = (int32_t)(task / words);
         const int w = (int)(task % words);
         const int64_t c0 = HS[v], c1 = HR[v + 1];
-        if (c0 < c1) chain_in(a, slots, bt.nslots, v, w, c0, c1, lane);
+        if (c0 < c1) chain_in(a, slots, bt.nslots, v, w, c0, c1, lane, scaled);
       }
       grid_sync(a);
     }
@@ -1045,8 +1015,8 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
           const int64_t per = (e1 - e0 + kWarpsPerCta - 1) / kWarpsPerCta;
           const int64_t s0 = e0 + wib * per, s1 = min(e1, s0 + per);
           if (lev < tlast && s0 < min(s1, sp))
-            row_pass<QT, kComp, 0>(a, lm_next, q, s0, min(s1, sp), w0, nw, act, any, acc, lane, lev + 1);
-          if (max(s0, sp) < s1) row_pass<QT, kComp, 2>(a, a.lm, q, max(s0, sp), s1, w0, nw, act, any, acc, lane, lev + 1, tlast);
+            row_pass<QT, kComp, 0>(a, lm_next, q, s0, min(s1, sp), w0, nw, act, any, acc, lane, lev + 1, scaled);
+          if (max(s0, sp) < s1) row_pass<QT, kComp, 2>(a, a.lm, q, max(s0, sp), s1, w0, nw, act, any, acc, lane, lev + 1, scaled, tlast);
         }
 #pragma unroll
         for (int k = 0; k < kHalf; ++k) S.acc[k][lane] = acc[k].value();
@@ -1091,11 +1061,11 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
             }
             if (!a_any) continue;
             Acc<kComp> acc[kHalf];
-            if (lev < tlast && e0 < sp) row_pass<QT, kComp, 0>(a, lm_next, q, e0, sp, w0, nw, act, any, acc, lane, lev + 1);
-            if (sp < e1) row_pass<QT, kComp, 2>(a, a.lm, q, sp, e1, w0, nw, act, any, acc, lane, lev + 1, tlast);
+            if (lev < tlast && e0 < sp) row_pass<QT, kComp, 0>(a, lm_next, q, e0, sp, w0, nw, act, any, acc, lane, lev + 1, scaled);
+            if (sp < e1) row_pass<QT, kComp, 2>(a, a.lm, q, sp, e1, w0, nw, act, any, acc, lane, lev + 1, scaled, tlast);
 #pragma unroll
             for (int k = 0; k < kHalf; ++k)
-              if (k < nw) finish_dep<QT>(a, slots, rch, v, w0 + k, lev, act[k], lane, acc[k].value(), sp < e1);
+              if (k < nw) finish_dep<QT>(a, slots, rch, v, w0 + k, lev, act[k], lane, acc[k].value(), sp < e1, scaled);
           }
         }
       }
@@ -1111,7 +1081,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
           if (!act) continue;
           double sum = 0.0;
           for (int32_t c = hfst[h]; c < hfst[h + 1]; ++c) sum += __ldcg(a.hacc + ((hc0 + c) * W + w) * 32 + lane);
-          finish_dep<QT>(a, slots, rch, v, w, lev, act, lane, sum, HS[v] < HR[v + 1]);
+          finish_dep<QT>(a, slots, rch, v, w, lev, act, lane, sum, HS[v] < HR[v + 1], scaled);
         }
       }
       grid_sync(a);
@@ -1165,17 +1135,17 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
             const bool sig = tieL || tieR || viaL || viaR;
             if (sig) {
               eL.s = __ldcg(a.sig + iL);
-              eL.x = __ldcg(xb + level_index(a, eL.d));
+              eL.x = scaled ? __ldcg(xb + level_index(a, eL.d)) : 0;
               eR.s = __ldcg(a.sig + iR);
-              eR.x = __ldcg(xb + level_index(a, eR.d));
+              eR.x = scaled ? __ldcg(xb + level_index(a, eR.d)) : 0;
             }
             if (viaR || srcL) {
               eL.qs = (double)__ldcg(qq + iL);
-              if (!sig) eL.x = __ldcg(xb + level_index(a, eL.d));
+              if (!sig) eL.x = scaled ? __ldcg(xb + level_index(a, eL.d)) : 0;
             }
             if (viaL || srcR) {
               eR.qs = (double)__ldcg(qq + iR);
-              if (!sig) eR.x = __ldcg(xb + level_index(a, eR.d));
+              if (!sig) eR.x = scaled ? __ldcg(xb + level_index(a, eR.d)) : 0;
             }
           }
           const double wsrc = live ? a.wsrc[b] : 0.0;
