@@ -83,18 +83,11 @@ constexpr int kSmallCore = 16384;  // cores below this many vertices use kHeavyD
 constexpr int kChunkArcs = BCGPU_BATCHED_CHUNK;  // arcs per heavy chunk
 constexpr int kHalf = 4;           // words per pass over a vertex row
 // Resident CTAs per SM the kernel is compiled for (registers per thread =
-// 65536 / (kThreads * kMinCtas)); profiling builds may override it. Six CTAs (40 registers,
-// some spilled to local memory) with the one-arc hit walk measured fastest
-// on RMAT-20 at 512 sources per pass: 135 / 139 / 147 / 124 GTEPS for 4 / 5 /
-// 6 / 8 CTAs per SM.
+// 65536 / (kThreads * kMinCtas)); profiling builds may override it. Six CTAs (40
+// registers, some spilled to local memory): two passes of 512 sources on RMAT-20
+// take 199 / 183 / 180.5 ms for 4 / 5 / 6 CTAs per SM.
 #ifndef BCGPU_BATCHED_MIN_CTAS
 #define BCGPU_BATCHED_MIN_CTAS 6
-#endif
-// Hit walk of a row pass: an arc is walked once for all kHalf words of the task
-// (one shuffle of its neighbour), this many arcs' values loaded at once (times
-// kHalf loads in flight).
-#ifndef BCGPU_BATCHED_WALK
-#define BCGPU_BATCHED_WALK 1
 #endif
 constexpr int kMinCtas = BCGPU_BATCHED_MIN_CTAS;
 // Light-row tasks per warp and level at least (smaller vertex blocks when
@@ -175,8 +168,7 @@ struct Args {
   void *q;
   uint32_t *lm;     // [tcap+2][n_cap][W]
   uint32_t *seen;   // [n_cap][W]
-  int32_t *lmin, *lmax;
-  int32_t *gdone;   // [n_cap] groups of 4 words already seen by all their slots (a lower bound)
+  int32_t *lmin;    // [n_cap] first level on which some slot reached the vertex
   int32_t *armed;   // [n_cap] first level on which some slot can reach the vertex (a neighbour was reached)
   int *wq;          // [4*(tcap+3)+2] work counters: light rows forward (t), backward (tcap+3+lev); heavy chunks (2*(tcap+3)+t, 3*(tcap+3)+lev); chain in-flow (4*(tcap+3)); chain vertices (4*(tcap+3)+1)
   double *bcpart;   // [n_cap][W] BC partials of the core vertices
@@ -376,11 +368,46 @@ __device__ __forceinline__ void load_row(const uint32_t *p, int nw, uint32_t (&m
   }
 }
 
-template <typename T>
-__device__ __forceinline__ T warp_or(T v) {
+// Walks the arcs of a strip of 32 (lane j: neighbour u, level lvl, hit masks f)
+// that hit in some word, in arc order, and adds their values (vrow: the task's
+// first word, this lane's slot).
+template <typename T, bool kComp, int kLev>
+__device__ __forceinline__ void walk_hits(const Args &a, const T *vrow, uint32_t u, int lvl, const uint32_t (&f)[kHalf],
+                                          Acc<kComp> (&acc)[kHalf], int lane, int w0 = 0, int t = 0,
+                                          bool scaled = false) {
+  const int W = a.W;
+  uint32_t fo = 0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v |= __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+  for (int k = 0; k < kHalf; ++k) fo |= f[k];
+  uint32_t hits = __ballot_sync(0xffffffffu, fo != 0u);
+  // level exponent bases of the task's slots: word k's at xb0 + k * xs
+  const int64_t xs = (int64_t)32 * (a.tcap + 2);
+  const int32_t *xb0 = kLev ? a.X + (int64_t)(w0 * 32 + lane) * (a.tcap + 2) : nullptr;
+  int xt[kHalf];
+#pragma unroll
+  for (int k = 0; k < kHalf; ++k) xt[k] = (kLev && scaled && hits) ? __ldcg(xb0 + k * xs + t) : 0;
+  while (hits) {  // uniform
+    const int j = __ffs(hits) - 1;
+    hits &= hits - 1;
+    const uint32_t uj = __shfl_sync(0xffffffffu, u, j);
+    const int lj = kLev ? __shfl_sync(0xffffffffu, lvl, j) : 0;
+    const T *vu = vrow + (int64_t)uj * W * 32;
+    T x[kHalf];
+#pragma unroll
+    for (int k = 0; k < kHalf; ++k) {
+      const uint32_t fj = __shfl_sync(0xffffffffu, f[k], j);
+      x[k] = (T)0;
+      if ((fj >> lane) & 1u) {
+        x[k] = __ldcg(vu + k * 32);
+        if (kLev && scaled) {
+          const int xl = __ldcg(xb0 + k * xs + lj);
+          x[k] = (T)scale2((double)x[k], kLev == 1 ? xl - xt[k] : xt[k] - xl);
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kHalf; ++k) acc[k].add((double)x[k]);
+  }
 }
 
 // One pull / successor pass over arcs [e0, e1) for words [w0, w0+nw):
@@ -417,74 +444,35 @@ __device__ __forceinline__ void row_pass(const Args &a, const uint32_t *masks, c
       f[k] &= filt[k];
       any[k] |= f[k];
     }
-    uint32_t fo = 0;
-#pragma unroll
-    for (int k = 0; k < kHalf; ++k) fo |= f[k];
-    uint32_t hits = __ballot_sync(0xffffffffu, fo != 0u);
-    // level exponent bases of the task's slots: word k's at xb0 + k * xs
-    const int64_t xs = (int64_t)32 * (a.tcap + 2);
-    const int32_t *xb0 = kLev ? a.X + (int64_t)(w0 * 32 + lane) * (a.tcap + 2) : nullptr;
-    int xt[kHalf];
-#pragma unroll
-    for (int k = 0; k < kHalf; ++k) xt[k] = (kLev && scaled && hits) ? __ldcg(xb0 + k * xs + t) : 0;
-    const T *vrow = vals + (int64_t)w0 * 32 + lane;
-    constexpr int kArcs = BCGPU_BATCHED_WALK;  // hit arcs whose values are loaded at once
-    while (hits) {  // uniform: arcs with a hit in some word, in arc order
-      T x[kArcs][kHalf];
-#pragma unroll
-      for (int r = 0; r < kArcs; ++r) {
-#pragma unroll
-        for (int k = 0; k < kHalf; ++k) x[r][k] = (T)0;
-        if (!hits) continue;  // uniform
-        const int j = __ffs(hits) - 1;
-        hits &= hits - 1;
-        const int32_t uj = __shfl_sync(0xffffffffu, u, j);
-        const int lj = kLev ? __shfl_sync(0xffffffffu, lvl, j) : 0;
-        const T *vu = vrow + (int64_t)uj * W * 32;
-#pragma unroll
-        for (int k = 0; k < kHalf; ++k) {
-          const uint32_t fj = __shfl_sync(0xffffffffu, f[k], j);
-          if ((fj >> lane) & 1u) {
-            x[r][k] = __ldcg(vu + k * 32);
-            if (kLev && scaled) {
-              const int xl = __ldcg(xb0 + k * xs + lj);
-              x[r][k] = (T)scale2((double)x[r][k], kLev == 1 ? xl - xt[k] : xt[k] - xl);
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < kArcs; ++r)
-#pragma unroll
-        for (int k = 0; k < kHalf; ++k) acc[k].add((double)x[r][k]);
-    }
+    walk_hits<T, kComp, kLev>(a, vals + (int64_t)w0 * 32 + lane, u, lvl, f, acc, lane, w0, t, scaled);
   }
 }
 
-// Stores the result of one (vertex, word) of the forward step; returns the
-// number of slots that reached the vertex, plus 256 when this is the first
-// time any slot reached it (uniform over the warp).
+// Path counts of one (vertex, word) of the forward step: its new slots' levels
+// and counts (the heaviest count of a level that needs rescaling is noted).
+__device__ __forceinline__ void put_counts(const Args &a, int32_t v, int w, int t, uint32_t newm, int lane, double acc) {
+  if (!((newm >> lane) & 1u)) return;
+  const int64_t idx = ((int64_t)v * a.W + w) * 32 + lane;
+  a.d[idx] = t + 1;
+  a.sig[idx] = acc;
+  if (exp_bits(acc) - 1023 >= a.rescale_exp && acc > pow2(a.rescale_exp)) {  // acc > 2^rescale_exp, acc normal
+    atomicMax(a.rexp + w * 32 + lane, exp_bits(acc) - 1023);
+    a.ctrl->rescale[t & 1] = 1;
+  }
+}
+
+// Stores the result of one (vertex, word) of a heavy row; returns the number
+// of slots that reached the vertex (uniform over the warp).
 __device__ __forceinline__ int finish_pull(const Args &a, int32_t v, int w, int t, uint32_t newm, int lane,
                                            double acc) {
   if (!newm) return 0;
-  int first = 0;
-  const int64_t idx = ((int64_t)v * a.W + w) * 32 + lane;
-  if ((newm >> lane) & 1u) {
-    a.d[idx] = t + 1;
-    a.sig[idx] = acc;
-    if (exp_bits(acc) - 1023 >= a.rescale_exp && acc > pow2(a.rescale_exp)) {  // acc > 2^rescale_exp, acc normal
-      atomicMax(a.rexp + w * 32 + lane, exp_bits(acc) - 1023);
-      a.ctrl->rescale[t & 1] = 1;
-    }
-  }
+  put_counts(a, v, w, t, newm, lane, acc);
   if (lane == 0) {
     a.lm[((int64_t)(t + 1) * a.n_cap + v) * a.W + w] = newm;
     a.seen[(int64_t)v * a.W + w] |= newm;
-    a.ctrl->more[t & 1] = 1;
-    first = atomicMin(a.lmin + v, t + 1) == INT_MAX;
-    atomicMax(a.lmax + v, t + 1);
+    atomicMin(a.lmin + v, t + 1);
   }
-  return __popc(newm) + (__shfl_sync(0xffffffffu, first, 0) << 8);
+  return __popc(newm);
 }
 
 // Arms the neighbours of a vertex first reached on level lvl: a neighbour
@@ -580,30 +568,38 @@ __device__ __forceinline__ void chain_in(const Args &a, const Slot *slots, int n
   a.cdep[iv] = sum;
 }
 
-// delta, q and the BC partial of one (vertex, word) at level lev.
-template <typename QT>
-__device__ __forceinline__ void finish_dep(const Args &a, const Slot *slots, const int32_t *rch, int32_t v, int w,
-                                           int lev, uint32_t act, int lane, double sum, bool chains, bool scaled) {
+// delta, q and the BC partial (in word w0's place) of kWords words of a vertex
+// at level lev; every load is issued before the first use.
+template <typename QT, int kWords>
+__device__ __forceinline__ void finish_dep(const Args &a, int32_t reach, int32_t v, int w0, int lev,
+                                           const uint32_t (&act)[kWords], int lane, const double (&sum)[kWords],
+                                           bool chains, bool scaled) {
   constexpr bool kF32 = sizeof(QT) == 4;
-  if (!act) return;
-  const int W = a.W;
+  const int64_t idx = ((int64_t)v * a.W + w0) * 32 + lane;
+  double sv[kWords], in[kWords];
+#pragma unroll
+  for (int k = 0; k < kWords; ++k) {
+    const bool on = (act[k] >> lane) & 1u;
+    sv[k] = on ? __ldcg(a.sig + idx + k * 32) : 1.0;
+    in[k] = on && chains ? __ldcg(a.cdep + idx + k * 32) : 0.0;
+  }
   double contrib = 0.0;
-  if ((act >> lane) & 1u) {
-    const int b = w * 32 + lane;
-    const int64_t idx = ((int64_t)v * W + w) * 32 + lane;
-    const double sv = a.sig[idx];
+#pragma unroll
+  for (int k = 0; k < kWords; ++k) {
+    if (!((act[k] >> lane) & 1u)) continue;
+    const int b = (w0 + k) * 32 + lane;
     const int xd = scaled ? a.X[(int64_t)b * (a.tcap + 2) + lev] - a.X[(int64_t)b * (a.tcap + 2) + lev + 1] : 0;
-    const double delta = scale2(sv * sum, xd) + (chains ? __ldcg(a.cdep + idx) : 0.0);
-    const double qv = ((double)rch[v] + 1.0 + delta) / sv;
+    const double delta = scale2(sv[k] * sum[k], xd) + in[k];
+    const double qv = ((double)reach + 1.0 + delta) / sv[k];
     if (kF32) {
       const double aq = fabs(qv);
       if (!(aq >= (double)FLT_MIN * 0x1p24 && aq <= (double)FLT_MAX * 0x1p-24)) atomicExch(&a.ctrl->range_err, 1);
     }
-    reinterpret_cast<QT *>(a.q)[idx] = (QT)qv;
-    contrib = delta * a.wsrc[b];
+    reinterpret_cast<QT *>(a.q)[idx + k * 32] = (QT)qv;
+    contrib += delta * a.wsrc[b];
   }
-  contrib = warp_sum(contrib);  // fixed-order reduction of this word's slots
-  if (lane == 0) a.bcpart[(int64_t)v * W + w] += contrib;
+  contrib = warp_sum(contrib);  // fixed-order reduction of the slots
+  if (lane == 0) atomicAdd(a.bcpart + (int64_t)v * a.W + w0, contrib);  // one writer a level: no wait for the old value
 }
 
 // Vertex blocks of a phase: each warp's first block is its own index, later
@@ -615,24 +611,27 @@ __device__ __forceinline__ int64_t next_block(int *counter, int lane) {
   return nwarps() + __shfl_sync(0xffffffffu, b, 0);
 }
 
-// Vertex of lane l in light-row block vb (bs vertices per block, nblk
-// blocks): strided over the core (BCGPU_BATCHED_CONTIG 0: every block mixes
-// early, high-degree vertices of the BFS order with late ones) or
-// consecutive (1: neighbouring rows share cached mask rows, and with blocks
-// handed out in order a level ends on the cheap late vertices; 177.3
-// against 172.0 GTEPS on RMAT-20).
-#ifndef BCGPU_BATCHED_CONTIG
-#define BCGPU_BATCHED_CONTIG 1
-#endif
-__device__ __forceinline__ int64_t block_vertex(int64_t vb, int l, int bs, int64_t nblk) {
-#if BCGPU_BATCHED_CONTIG
-  (void)nblk;
-  return vb * bs + l;
-#else
-  (void)bs;
-  return vb + (int64_t)l * nblk;
-#endif
-}
+// A block's rows, one per lane, in 32 bits each: a row's place after the block's
+// first, and its arcs (low half) and unit arcs (high half) when it is a light
+// one. Blocks are consecutive vertices: neighbouring rows share cached mask
+// rows, and with blocks handed out in order a level ends on the cheap late
+// vertices of the BFS order (177.3 GTEPS on RMAT-20, against 172.0 with every
+// block strided over the core).
+struct RowLane {
+  uint32_t at = 0, len = 0;
+  static __device__ __forceinline__ RowLane load(const int64_t *HR, const int64_t *HS, int64_t v, int64_t rb,
+                                                 int32_t heavy_deg) {
+    const int64_t e0 = HR[v], e1 = HR[v + 1], sp = HS[v];
+    return RowLane{(uint32_t)(e0 - rb), e1 - e0 <= heavy_deg ? (uint32_t)(e1 - e0) | (uint32_t)(sp - e0) << 16 : 0u};
+  }
+  __device__ __forceinline__ bool light() const { return len != 0; }
+  // the first neighbours (unit arcs) of lane j's row, one a lane
+  __device__ __forceinline__ uint32_t strip(const Args &a, int64_t rb, int j, int lane) const {
+    const uint32_t at_j = __shfl_sync(0xffffffffu, at, j), len_j = __shfl_sync(0xffffffffu, len, j);
+    return lane < (int)(len_j >> 16) ? (uint32_t)ldg(a.hcol + rb + at_j + lane) : 0u;
+  }
+};
+static_assert(kHeavyDeg < 1 << 16, "a light row's length takes 16 bits");
 
 // Heavy-row chunk tasks of a phase: each CTA's first task is its own index;
 // later ones in a fixed stride (BCGPU_BATCHED_HEAVY_DYN 0) or from the
@@ -732,7 +731,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
       a.bcpart[i] = 0.0;
       a.lm[i] = 0;                         // level 0
       a.lm[(int64_t)a.n_cap * W + i] = 0;  // level 1
-      if (w == 0) { a.lmin[i / W] = INT_MAX; a.lmax[i / W] = -1; a.gdone[i / W] = 0; a.armed[i / W] = INT_MAX; }
+      if (w == 0) { a.lmin[i / W] = INT_MAX; a.armed[i / W] = INT_MAX; }
     }
     for (int64_t i = gtid; i < (int64_t)W * 32; i += gthreads) {
       a.rexp[i] = INT_MIN;
@@ -756,7 +755,6 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
       atomicOr(a.lm + (int64_t)s.src * W + (b >> 5), 1u << (b & 31));
       atomicOr(a.seen + (int64_t)s.src * W + (b >> 5), 1u << (b & 31));
       atomicMin(a.lmin + s.src, 0);
-      atomicMax(a.lmax + s.src, 0);
       atomicAdd(&a.ctrl->found, 1ull);
     }
     for (int64_t i = gwarp(); i < bt.narm; i += nwarps()) {  // neighbours of sources and seeded vertices
@@ -776,6 +774,13 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
     const unsigned long long all_found = (unsigned long long)n * (unsigned long long)bt.nslots;
     while (true) {
       unsigned long long nf = 0;  // pairs this warp found on this level
+      // Once a warp and phase: every warp writes the same words, and a store for
+      // each row reached made that one address what the level waited for.
+      auto report = [&](unsigned long long found) {
+        if (lane != 0 || !found) return;
+        atomicAdd(&a.ctrl->found, found);
+        a.ctrl->more[t & 1] = 1;
+      };
       if (t + 1 > a.tcap) { set_err(a.err, kDevWorkspace); break; }
       const uint32_t *lmt = a.lm + (int64_t)t * a.n_cap * W;
       // the next level's flags and masks start clear (nothing reads them on this level)
@@ -807,7 +812,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
         }
 #pragma unroll
         for (int k = 0; k < kHalf; ++k) {
-          any[k] = warp_or(any[k]);
+          any[k] = __reduce_or_sync(0xffffffffu, any[k]);
           S.acc[k][lane] = acc[k].value();
           if (lane == 0) S.any[k] = any[k];  // this warp's hit masks, for the combine
         }
@@ -821,63 +826,75 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
         }
         __syncthreads();
       }
-      // light rows: (vertex block, quarter) tasks, lane-parallel activity check
+      // light rows: (vertex block, quarter) tasks. Lane l holds vertex l's row and
+      // unseen slots; the next active row's first neighbours are loaded while
+      // this one's counts are gathered. Bound by the latency of a row's chain of
+      // loads (neighbours, their masks, counts), 48 warps an SM in flight. Two
+      // passes of 512 on R-MAT 20: the forward rows took 89.7 ms with a flag store a
+      // row, the row's masks re-read a row at a time and 20 shuffles to fold the
+      // hits, 51.1 ms so; the backward rows, likewise, 74.2 and 69.2. CTAs per SM 4 /
+      // 5 / 6: 199 / 183 / 180.5 ms a kernel.
       for (int64_t tk = gwarp(); tk < ntask; tk = next_block(a.wq + t, lane)) {
-        const int64_t vb = tk / halves;
+        const int64_t v0 = tk / halves * bs;
         const int w0 = (int)(tk % halves) * kHalf;
-        const int nw = kHalf;
-        const int64_t vl = block_vertex(vb, lane, bs, nblk);
-        int64_t e0l = 0, e1l = 0, spl = 0;
-        bool on = false;
+        const int64_t vl = v0 + lane;
+        RowLane row{};
+        uint4 un = make_uint4(0, 0, 0, 0);
+        int32_t lmin = 0;
+        const int64_t rb = HR[v0];
         if (lane < bs && vl < n) {
-          e0l = HR[vl];
-          e1l = HR[vl + 1];
-          spl = HS[vl];
-          on = e1l - e0l <= bt.heavy_deg && __ldcg(a.gdone + vl) < groups && __ldcg(a.armed + vl) <= t + 1;
+          const uint4 seen = ld4(a.seen + vl * W + w0);
+          const int32_t armed = __ldcg(a.armed + vl);
+          lmin = __ldcg(a.lmin + vl);
+          row = RowLane::load(HR, HS, vl, rb, bt.heavy_deg);
+          if (armed <= t + 1 && row.light()) un = make_uint4(~seen.x, ~seen.y, ~seen.z, ~seen.w);
         }
-        uint32_t todo = __ballot_sync(0xffffffffu, on);
+        uint32_t todo = __ballot_sync(0xffffffffu, (un.x | un.y | un.z | un.w) != 0u);
+        uint32_t ahead = todo ? row.strip(a, rb, __ffs(todo) - 1, lane) : 0u;
         while (todo) {
           const int j = __ffs(todo) - 1;
           todo &= todo - 1;
-          const int32_t v = (int32_t)block_vertex(vb, j, bs, nblk);
-          const int64_t e0 = __shfl_sync(0xffffffffu, e0l, j), e1 = __shfl_sync(0xffffffffu, e1l, j);
-          const int64_t sp = __shfl_sync(0xffffffffu, spl, j);
-          {
-            uint32_t seen[kHalf], unseen[kHalf], any[kHalf];
-            load_row(a.seen + (int64_t)v * W + w0, nw, seen);
-            uint32_t u_any = 0;
+          const uint32_t u = ahead;
+          if (todo) ahead = row.strip(a, rb, __ffs(todo) - 1, lane);
+          const int32_t v = (int32_t)v0 + j;
+          const int64_t e0 = rb + __shfl_sync(0xffffffffu, row.at, j);
+          const uint32_t len = __shfl_sync(0xffffffffu, row.len, j);
+          const int units = (int)(len >> 16), arcs = (int)(len & 0xffff);
+          const uint32_t unseen[kHalf] = {__shfl_sync(0xffffffffu, un.x, j), __shfl_sync(0xffffffffu, un.y, j),
+                                          __shfl_sync(0xffffffffu, un.z, j), __shfl_sync(0xffffffffu, un.w, j)};
+          uint32_t any[kHalf];
+          load_row(lmt + (int64_t)u * W + w0, lane < units ? kHalf : 0, any);
 #pragma unroll
-            for (int k = 0; k < kHalf; ++k) { unseen[k] = k < nw ? ~seen[k] : 0u; any[k] = 0; u_any |= unseen[k]; }
-            if (!u_any) continue;
-            Acc<false> acc[kHalf];
-            if (e0 < sp) row_pass<double, false, 0>(a, lmt, a.sig, e0, sp, w0, nw, unseen, any, acc, lane, t, scaled);
-            if (sp < e1) row_pass<double, false, 1>(a, a.lm, a.sig, sp, e1, w0, nw, unseen, any, acc, lane, t, scaled);
-            int first = 0;
+          for (int k = 0; k < kHalf; ++k) any[k] &= unseen[k];
+          Acc<false> acc[kHalf];
+          walk_hits<double, false, 0>(a, a.sig + (int64_t)w0 * 32 + lane, u, 0, any, acc, lane);
+          if (units > 32)
+            row_pass<double, false, 0>(a, lmt, a.sig, e0 + 32, e0 + units, w0, kHalf, unseen, any, acc, lane, t);
+          if (units < arcs)
+            row_pass<double, false, 1>(a, a.lm, a.sig, e0 + units, e0 + arcs, w0, kHalf, unseen, any, acc, lane, t, scaled);
+          uint32_t hit = 0;
 #pragma unroll
-            for (int k = 0; k < kHalf; ++k) {
-              if (k >= nw) continue;
-              const uint32_t m = warp_or(any[k]);
-              const int r = finish_pull(a, v, w0 + k, t, m, lane, acc[k].value());
-              nf += r & 255;
-              first |= r >> 8;
-              any[k] = m;
-            }
-            if (first) arm_arcs(a, e0, e1, t + 1, lane, 32);
-#pragma unroll
-            for (int g = 0; g < kHalf / 4; ++g) {  // groups now seen by all their slots
-              if (4 * g >= nw || lane != 0) continue;
-              bool was = true, now = true;
-#pragma unroll
-              for (int k = 4 * g; k < 4 * g + 4; ++k) {
-                was = was && unseen[k] == 0u;
-                now = now && (unseen[k] & ~any[k]) == 0u;
-              }
-              if (now && !was) atomicAdd(a.gdone + v, 1);
-            }
+          for (int k = 0; k < kHalf; ++k) {
+            any[k] = __reduce_or_sync(0xffffffffu, any[k]);
+            hit |= any[k];
+            nf += __popc(any[k]);
           }
+          if (!hit) continue;
+#pragma unroll
+          for (int k = 0; k < kHalf; ++k) put_counts(a, v, w0 + k, t, any[k], lane, acc[k].value());
+          int first = 0;
+          const bool fresh = __shfl_sync(0xffffffffu, lmin, j) == INT_MAX;  // not reached on an earlier level
+          if (lane == 0) {
+            *reinterpret_cast<uint4 *>(a.lm + ((int64_t)(t + 1) * a.n_cap + v) * W + w0) =
+                make_uint4(any[0], any[1], any[2], any[3]);
+            *reinterpret_cast<uint4 *>(a.seen + (int64_t)v * W + w0) =
+                make_uint4(~unseen[0] | any[0], ~unseen[1] | any[1], ~unseen[2] | any[2], ~unseen[3] | any[3]);
+            if (fresh) first = atomicMin(a.lmin + v, t + 1) == INT_MAX;
+          }
+          if (fresh && __shfl_sync(0xffffffffu, first, 0)) arm_arcs(a, e0, e0 + arcs, t + 1, lane, 32);
         }
       }
-      if (lane == 0 && nf) atomicAdd(&a.ctrl->found, nf);
+      report(nf);
       nf = 0;
       grid_sync(a);
       PHASE_MARK(1);
@@ -894,9 +911,9 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
             acc += __ldcg(a.hacc + ((hc0 + c) * W + w) * 32 + lane);
             m |= __ldcg(a.hmask + (hc0 + c) * W + w);
           }
-          nf += finish_pull(a, v, w, t, m, lane, acc) & 255;  // heavy rows arm in the next phase
+          nf += finish_pull(a, v, w, t, m, lane, acc);  // heavy rows arm in the next phase
         }
-        if (lane == 0 && nf) atomicAdd(&a.ctrl->found, nf);
+        report(nf);
         grid_sync(a);
         PHASE_MARK(2);
       }
@@ -914,7 +931,6 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
             a.sig[idx] = one;
             atomicOr(a.lm + ((int64_t)(t + 1) * a.n_cap + s.v) * W + w, bit);
             atomicMin(a.lmin + s.v, t + 1);
-            atomicMax(a.lmax + s.v, t + 1);
             a.ctrl->more[t & 1] = 1;
             atomicAdd(&a.ctrl->found, 1ull);
           } else if (a.d[idx] == t + 1) {
@@ -1001,11 +1017,10 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
         const int32_t v = hv[hcv[c]];
         uint32_t act[kHalf], any[kHalf];
         load_row(lm_here + (int64_t)v * W + w0, nw, act);
-        const bool in_span = lev >= __ldcg(a.lmin + v) && lev <= __ldcg(a.lmax + v);
         uint32_t a_any = 0;
 #pragma unroll
         for (int k = 0; k < kHalf; ++k) {
-          act[k] = (in_span && k < nw) ? act[k] : 0u;
+          act[k] = k < nw ? act[k] : 0u;
           any[k] = 0;
           a_any |= act[k];
         }
@@ -1030,43 +1045,46 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
       }
       const int wqi = a.tcap + 3 + lev;
       for (int64_t tk = gwarp(); tk < ntask; tk = next_block(a.wq + wqi, lane)) {
-        const int64_t vb = tk / halves;
+        const int64_t v0 = tk / halves * bs;
         const int w0 = (int)(tk % halves) * kHalf;
-        const int nw = kHalf;
-        const int64_t vl = block_vertex(vb, lane, bs, nblk);
-        int64_t e0l = 0, e1l = 0, spl = 0;
-        bool on = false;
-        if (lane < bs && vl < n && lev >= __ldcg(a.lmin + vl) && lev <= __ldcg(a.lmax + vl)) {
-          e0l = HR[vl];
-          e1l = HR[vl + 1];
-          spl = HS[vl];
-          on = e1l - e0l <= bt.heavy_deg;
+        const int64_t vl = v0 + lane;
+        RowLane row{};
+        uint4 on = make_uint4(0, 0, 0, 0);  // the vertex's slots on this level
+        int32_t reach = 0;
+        const int64_t rb = HR[v0];
+        if (lane < bs && vl < n) {
+          on = ld4(lm_here + vl * W + w0);
+          row = RowLane::load(HR, HS, vl, rb, bt.heavy_deg);
+          reach = rch[vl];
+          if (!row.light()) on = make_uint4(0, 0, 0, 0);
         }
-        uint32_t todo = __ballot_sync(0xffffffffu, on);
+        uint32_t todo = __ballot_sync(0xffffffffu, (on.x | on.y | on.z | on.w) != 0u);
+        uint32_t ahead = todo ? row.strip(a, rb, __ffs(todo) - 1, lane) : 0u;
         while (todo) {
           const int j = __ffs(todo) - 1;
           todo &= todo - 1;
-          const int32_t v = (int32_t)block_vertex(vb, j, bs, nblk);
-          const int64_t e0 = __shfl_sync(0xffffffffu, e0l, j), e1 = __shfl_sync(0xffffffffu, e1l, j);
-          const int64_t sp = __shfl_sync(0xffffffffu, spl, j);
-          {
-            uint32_t act[kHalf], any[kHalf];
-            load_row(lm_here + (int64_t)v * W + w0, nw, act);
-            uint32_t a_any = 0;
+          const uint32_t u = ahead;
+          if (todo) ahead = row.strip(a, rb, __ffs(todo) - 1, lane);
+          const int32_t v = (int32_t)v0 + j;
+          const int64_t e0 = rb + __shfl_sync(0xffffffffu, row.at, j);
+          const uint32_t len = __shfl_sync(0xffffffffu, row.len, j);
+          const int units = (int)(len >> 16), arcs = (int)(len & 0xffff);
+          const uint32_t act[kHalf] = {__shfl_sync(0xffffffffu, on.x, j), __shfl_sync(0xffffffffu, on.y, j),
+                                       __shfl_sync(0xffffffffu, on.z, j), __shfl_sync(0xffffffffu, on.w, j)};
+          Acc<kComp> acc[kHalf];
+          uint32_t any[kHalf] = {};
+          if (lev < tlast) {
+            load_row(lm_next + (int64_t)u * W + w0, lane < units ? kHalf : 0, any);
 #pragma unroll
-            for (int k = 0; k < kHalf; ++k) {
-              act[k] = k < nw ? act[k] : 0u;
-              any[k] = 0;
-              a_any |= act[k];
-            }
-            if (!a_any) continue;
-            Acc<kComp> acc[kHalf];
-            if (lev < tlast && e0 < sp) row_pass<QT, kComp, 0>(a, lm_next, q, e0, sp, w0, nw, act, any, acc, lane, lev + 1, scaled);
-            if (sp < e1) row_pass<QT, kComp, 2>(a, a.lm, q, sp, e1, w0, nw, act, any, acc, lane, lev + 1, scaled, tlast);
-#pragma unroll
-            for (int k = 0; k < kHalf; ++k)
-              if (k < nw) finish_dep<QT>(a, slots, rch, v, w0 + k, lev, act[k], lane, acc[k].value(), sp < e1, scaled);
+            for (int k = 0; k < kHalf; ++k) any[k] &= act[k];
+            walk_hits<QT, kComp, 0>(a, q + (int64_t)w0 * 32 + lane, u, 0, any, acc, lane);
+            if (units > 32)
+              row_pass<QT, kComp, 0>(a, lm_next, q, e0 + 32, e0 + units, w0, kHalf, act, any, acc, lane, lev + 1);
           }
+          if (units < arcs)
+            row_pass<QT, kComp, 2>(a, a.lm, q, e0 + units, e0 + arcs, w0, kHalf, act, any, acc, lane, lev + 1, scaled, tlast);
+          const double sum[kHalf] = {acc[0].value(), acc[1].value(), acc[2].value(), acc[3].value()};
+          finish_dep<QT, kHalf>(a, __shfl_sync(0xffffffffu, reach, j), v, w0, lev, act, lane, sum, units < arcs, scaled);
         }
       }
       if (nheavy) {
@@ -1076,12 +1094,11 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
           const int32_t h = (int32_t)(task / wpad);
           const int w = (int)(task % wpad);
           const int32_t v = hv[h];
-          if (lev < __ldcg(a.lmin + v) || lev > __ldcg(a.lmax + v)) continue;
           const uint32_t act = __ldcg(lm_here + (int64_t)v * W + w);
           if (!act) continue;
           double sum = 0.0;
           for (int32_t c = hfst[h]; c < hfst[h + 1]; ++c) sum += __ldcg(a.hacc + ((hc0 + c) * W + w) * 32 + lane);
-          finish_dep<QT>(a, slots, rch, v, w, lev, act, lane, sum, HS[v] < HR[v + 1], scaled);
+          finish_dep<QT, 1>(a, rch[v], v, w, lev, {act}, lane, {sum}, HS[v] < HR[v + 1], scaled);
         }
       }
       grid_sync(a);
@@ -1732,8 +1749,6 @@ int batched_build(const bc_bccs *B, const BatchedConfig &cfg, const int64_t *row
   ok &= ok && alloc(&p, (int64_t)(tcap + 2) * n * WA * 4); a.lm = (uint32_t *)p;
   ok &= ok && alloc(&p, n * WA * 4); a.seen = (uint32_t *)p;
   ok &= ok && alloc(&p, n * 4); a.lmin = (int32_t *)p;
-  ok &= ok && alloc(&p, n * 4); a.lmax = (int32_t *)p;
-  ok &= ok && alloc(&p, n * 4); a.gdone = (int32_t *)p;
   ok &= ok && alloc(&p, n * 4); a.armed = (int32_t *)p;
   ok &= ok && alloc(&p, (4 * ((int64_t)tcap + 3) + 2) * 4); a.wq = (int *)p;
   ok &= ok && alloc(&p, n * WA * 8); a.bcpart = (double *)p;
