@@ -83,11 +83,12 @@ constexpr int kSmallCore = 16384;  // cores below this many vertices use kHeavyD
 constexpr int kChunkArcs = BCGPU_BATCHED_CHUNK;  // arcs per heavy chunk
 constexpr int kHalf = 4;           // words per pass over a vertex row
 // Resident CTAs per SM the kernel is compiled for (registers per thread =
-// 65536 / (kThreads * kMinCtas)); profiling builds may override it. Six CTAs (40
-// registers, some spilled to local memory): two passes of 512 sources on RMAT-20
-// take 199 / 183 / 180.5 ms for 4 / 5 / 6 CTAs per SM.
+// 65536 / (kThreads * kMinCtas)); profiling builds may override it. Five CTAs (48
+// registers, some spilled to local memory): two passes of 512 sources on R-MAT 20
+// take 164.9 / 155.0 / 158.1 ms for 4 / 5 / 6 CTAs per SM, all passes of R-MAT 14
+// 164.5 / 161.4 / 169.5 ms.
 #ifndef BCGPU_BATCHED_MIN_CTAS
-#define BCGPU_BATCHED_MIN_CTAS 6
+#define BCGPU_BATCHED_MIN_CTAS 5
 #endif
 constexpr int kMinCtas = BCGPU_BATCHED_MIN_CTAS;
 // Light-row tasks per warp and level at least (smaller vertex blocks when
@@ -252,12 +253,13 @@ __device__ __forceinline__ unsigned long long gtimer() {
 __device__ __forceinline__ int64_t gwarp() { return ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; }
 __device__ __forceinline__ int64_t nwarps() { return ((int64_t)gridDim.x * blockDim.x) >> 5; }
 
-// ---- compensated FP32 accumulation (Neumaier's two-sum variant)
+// ---- compensated FP32 accumulation of terms >= 0: the exact error of each sum
+// (Dekker's fast two-sum, the larger of the two first) goes into c
 struct Comp32 {
   float s = 0.f, c = 0.f;
   __device__ __forceinline__ void add(float x) {
     const float t = s + x;
-    c += fabsf(s) >= fabsf(x) ? (s - t) + x : (x - t) + s;
+    c += fminf(s, x) - (t - fmaxf(s, x));
     s = t;
   }
   __device__ __forceinline__ double value() const { return (double)s + (double)c; }
@@ -329,14 +331,16 @@ __device__ __forceinline__ double end_dep(const Stretch &s, const End &A, const 
 }
 
 // ============================================================== forward ====
-// A task is one vertex row for kHalf 32-slot words: lane j loads arc j's
-// neighbour and its mask words (one aligned 16-byte load), then, word by
-// word, the arcs that hit (a ballot) are walked in arc order and their value
-// rows gathered four at a time (lane = slot, coalesced) into per-(word,
-// slot) accumulators held in registers. Adds follow arc order, so sums are
+// A task is one vertex row for a quarter: kHalf 32-slot words, 128 slots. Lane j
+// loads arc j's neighbour and its mask words (one aligned 16-byte load); the arcs
+// that hit go to the warp's shared memory in arc order and are walked there, each
+// with one load of its values: lane l has slots 4l ... 4l+3 of the quarter, whose
+// values are one sector (FP64) or half of one. Adds follow arc order, so sums are
 // deterministic.
+constexpr int kLaneSlots = 4;  // slots of a lane: consecutive ones
+static_assert(kLaneSlots * 32 == kHalf * 32, "a warp's lanes cover a quarter");
 
-// Per-(word, slot) accumulator of a row pass: FP64, or compensated FP32.
+// Per-slot accumulator of a row pass: FP64, or compensated FP32.
 template <bool kComp>
 struct Acc {
   double s = 0.0;
@@ -350,12 +354,43 @@ struct Acc<true> {
   __device__ __forceinline__ double value() const { return c.value(); }
 };
 
-// Per-warp shared memory: partial sums and hit masks of the heavy-row chunks,
-// combined across the CTA's warps in fixed order.
+// Per-warp shared memory: partial sums (by slot of the quarter) and hit masks of
+// the heavy-row chunks, combined across the CTA's warps in fixed order; the hits
+// of a strip of 32 arcs: masks, neighbours, levels.
 struct WarpScratch {
-  double acc[kHalf][32];
+  double acc[kHalf * 32];
   uint32_t any[kHalf];
+  uint32_t hit[32][kHalf];
+  uint32_t hit_u[32];
+  int32_t hit_lvl[32];
 };
+
+// A lane's place in a quarter: its word and the first of its slots' bits there.
+__device__ __forceinline__ int lane_word(int lane) { return lane >> 3; }
+__device__ __forceinline__ int lane_bit(int lane) { return (lane & 7) * kLaneSlots; }
+
+// A lane's four values, past L1 (other SMs wrote them): one load.
+__device__ __forceinline__ void ld_slots(const double *p, double (&x)[kLaneSlots]) {
+  asm volatile("ld.global.cg.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3]) : "l"(p));
+}
+__device__ __forceinline__ void ld_slots(const float *p, float (&x)[kLaneSlots]) {
+  const float4 v = __ldcg(reinterpret_cast<const float4 *>(p));
+  x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+}
+__device__ __forceinline__ void st_slots(double *p, const double (&x)[kLaneSlots]) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(x[0]), "d"(x[1]), "d"(x[2]), "d"(x[3]) : "memory");
+}
+__device__ __forceinline__ void st_slots(float *p, const float (&x)[kLaneSlots]) {
+  *reinterpret_cast<float4 *>(p) = make_float4(x[0], x[1], x[2], x[3]);
+}
+
+// The word whose bits the lanes of an eight hold, in all of them.
+__device__ __forceinline__ uint32_t word_of(uint32_t bits, int lane) {
+  uint32_t m = bits << lane_bit(lane);
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
+  return m;
+}
 
 __device__ __forceinline__ uint4 ld4(const uint32_t *p) { return __ldcg(reinterpret_cast<const uint4 *>(p)); }
 
@@ -369,45 +404,46 @@ __device__ __forceinline__ void load_row(const uint32_t *p, int nw, uint32_t (&m
 }
 
 // Walks the arcs of a strip of 32 (lane j: neighbour u, level lvl, hit masks f)
-// that hit in some word, in arc order, and adds their values (vrow: the task's
-// first word, this lane's slot).
+// that hit in some word, in arc order, and adds their values (vrow: this lane's
+// first slot); got: the lane's slots that were hit.
 template <typename T, bool kComp, int kLev>
-__device__ __forceinline__ void walk_hits(const Args &a, const T *vrow, uint32_t u, int lvl, const uint32_t (&f)[kHalf],
-                                          Acc<kComp> (&acc)[kHalf], int lane, int w0 = 0, int t = 0,
-                                          bool scaled = false) {
-  const int W = a.W;
-  uint32_t fo = 0;
+__device__ __forceinline__ void walk_hits(const Args &a, WarpScratch &S, const T *vrow, uint32_t u, int lvl,
+                                          const uint32_t (&f)[kHalf], uint32_t &got, Acc<kComp> (&acc)[kLaneSlots],
+                                          int lane, int w0 = 0, int t = 0, bool scaled = false) {
+  const bool mine = (f[0] | f[1] | f[2] | f[3]) != 0u;
+  const uint32_t hits = __ballot_sync(0xffffffffu, mine);
+  if (!hits) return;
+  if (mine) {
+    const int at = __popc(hits & ((1u << lane) - 1u));
+    *reinterpret_cast<uint4 *>(S.hit[at]) = make_uint4(f[0], f[1], f[2], f[3]);
+    S.hit_u[at] = u;
+    if (kLev) S.hit_lvl[at] = lvl;
+  }
+  __syncwarp();
+  // level exponent bases of the lane's slots: slot k's at xb + k * (tcap + 2)
+  const int32_t *xb = kLev ? a.X + (int64_t)(w0 * 32 + kLaneSlots * lane) * (a.tcap + 2) : nullptr;
+  const uint32_t *mine_at = &S.hit[0][lane_word(lane)];
+  const int sh = lane_bit(lane), n = __popc(hits);
+  const int64_t stride = (int64_t)a.W * 32;
+  for (int i = 0; i < n; ++i) {
+    const uint32_t m = mine_at[i * kHalf] >> sh & 15u;
+    const T *vu = vrow + (int64_t)S.hit_u[i] * stride;
+    got |= m;
+    T x[kLaneSlots] = {(T)0, (T)0, (T)0, (T)0};
+    if (m) ld_slots(vu, x);
+    if (kLev && scaled) {
+      const int lj = S.hit_lvl[i];
 #pragma unroll
-  for (int k = 0; k < kHalf; ++k) fo |= f[k];
-  uint32_t hits = __ballot_sync(0xffffffffu, fo != 0u);
-  // level exponent bases of the task's slots: word k's at xb0 + k * xs
-  const int64_t xs = (int64_t)32 * (a.tcap + 2);
-  const int32_t *xb0 = kLev ? a.X + (int64_t)(w0 * 32 + lane) * (a.tcap + 2) : nullptr;
-  int xt[kHalf];
-#pragma unroll
-  for (int k = 0; k < kHalf; ++k) xt[k] = (kLev && scaled && hits) ? __ldcg(xb0 + k * xs + t) : 0;
-  while (hits) {  // uniform
-    const int j = __ffs(hits) - 1;
-    hits &= hits - 1;
-    const uint32_t uj = __shfl_sync(0xffffffffu, u, j);
-    const int lj = kLev ? __shfl_sync(0xffffffffu, lvl, j) : 0;
-    const T *vu = vrow + (int64_t)uj * W * 32;
-    T x[kHalf];
-#pragma unroll
-    for (int k = 0; k < kHalf; ++k) {
-      const uint32_t fj = __shfl_sync(0xffffffffu, f[k], j);
-      x[k] = (T)0;
-      if ((fj >> lane) & 1u) {
-        x[k] = __ldcg(vu + k * 32);
-        if (kLev && scaled) {
-          const int xl = __ldcg(xb0 + k * xs + lj);
-          x[k] = (T)scale2((double)x[k], kLev == 1 ? xl - xt[k] : xt[k] - xl);
+      for (int k = 0; k < kLaneSlots; ++k)
+        if (m >> k & 1u) {
+          const int xl = __ldcg(xb + k * (a.tcap + 2) + lj), xt = __ldcg(xb + k * (a.tcap + 2) + t);
+          x[k] = (T)scale2((double)x[k], kLev == 1 ? xl - xt : xt - xl);
         }
-      }
     }
 #pragma unroll
-    for (int k = 0; k < kHalf; ++k) acc[k].add((double)x[k]);
+    for (int k = 0; k < kLaneSlots; ++k) acc[k].add((double)(m >> k & 1u ? x[k] : (T)0));
   }
+  __syncwarp();  // the next strip writes the same places
 }
 
 // One pull / successor pass over arcs [e0, e1) for words [w0, w0+nw):
@@ -418,11 +454,11 @@ __device__ __forceinline__ void walk_hits(const Args &a, const T *vrow, uint32_t
 //            X to level t's) or level t + hk[e] (kLev == 2, backward: q
 //            rebased to level t's X; levels above tend are empty)
 //   vals     per-slot values gathered on a hit (sigma, or q)
-// Adds into acc[k] and ORs the hits into any[k] (per lane).
+// Adds into acc, and the lane's hit slots into got.
 template <typename T, bool kComp, int kLev>
-__device__ __forceinline__ void row_pass(const Args &a, const uint32_t *masks, const T *vals, int64_t e0, int64_t e1,
-                                         int w0, int nw, const uint32_t (&filt)[kHalf], uint32_t (&any)[kHalf],
-                                         Acc<kComp> (&acc)[kHalf], int lane, int t, bool scaled = false, int tend = 0) {
+__device__ __forceinline__ void row_pass(const Args &a, WarpScratch &S, const uint32_t *masks, const T *vals, int64_t e0,
+                                         int64_t e1, int w0, int nw, const uint32_t (&filt)[kHalf], uint32_t &got,
+                                         Acc<kComp> (&acc)[kLaneSlots], int lane, int t, bool scaled = false, int tend = 0) {
   const int W = a.W;
   for (int64_t base = e0; base < e1; base += 32) {
     const int64_t e = base + lane;
@@ -440,39 +476,51 @@ __device__ __forceinline__ void row_pass(const Args &a, const uint32_t *masks, c
     const uint32_t *mrow = kLev ? masks + ((int64_t)(valid ? lvl : 0) * a.n_cap + u) * W + w0 : masks + (int64_t)u * W + w0;
     load_row(mrow, valid ? nw : 0, f);
 #pragma unroll
-    for (int k = 0; k < kHalf; ++k) {
-      f[k] &= filt[k];
-      any[k] |= f[k];
+    for (int k = 0; k < kHalf; ++k) f[k] &= filt[k];
+    walk_hits<T, kComp, kLev>(a, S, vals + (int64_t)w0 * 32 + kLaneSlots * lane, u, lvl, f, got, acc, lane, w0, t, scaled);
+  }
+}
+
+// Path counts that a lane's slots (the first: b, of kN) of the forward step got:
+// their levels and counts (the heaviest count of a level that needs rescaling is
+// noted). Slots outside `got` keep theirs.
+template <int kN>
+__device__ __forceinline__ void put_counts(const Args &a, int32_t v, int b, int t, uint32_t got, const double (&acc)[kN]) {
+  const int64_t idx = (int64_t)v * a.W * 32 + b;
+  bool whole = false;
+  if constexpr (kN == kLaneSlots) {
+    whole = got == 15u;
+    if (whole) {
+      *reinterpret_cast<int4 *>(a.d + idx) = make_int4(t + 1, t + 1, t + 1, t + 1);
+      st_slots(a.sig + idx, acc);
     }
-    walk_hits<T, kComp, kLev>(a, vals + (int64_t)w0 * 32 + lane, u, lvl, f, acc, lane, w0, t, scaled);
+  }
+#pragma unroll
+  for (int k = 0; k < kN; ++k) {
+    if (!(got >> k & 1u)) continue;
+    if (!whole) {
+      a.d[idx + k] = t + 1;
+      a.sig[idx + k] = acc[k];
+    }
+    if (exp_bits(acc[k]) - 1023 >= a.rescale_exp && acc[k] > pow2(a.rescale_exp)) {  // acc > 2^rescale_exp, acc normal
+      atomicMax(a.rexp + b + k, exp_bits(acc[k]) - 1023);
+      a.ctrl->rescale[t & 1] = 1;
+    }
   }
 }
 
-// Path counts of one (vertex, word) of the forward step: its new slots' levels
-// and counts (the heaviest count of a level that needs rescaling is noted).
-__device__ __forceinline__ void put_counts(const Args &a, int32_t v, int w, int t, uint32_t newm, int lane, double acc) {
-  if (!((newm >> lane) & 1u)) return;
-  const int64_t idx = ((int64_t)v * a.W + w) * 32 + lane;
-  a.d[idx] = t + 1;
-  a.sig[idx] = acc;
-  if (exp_bits(acc) - 1023 >= a.rescale_exp && acc > pow2(a.rescale_exp)) {  // acc > 2^rescale_exp, acc normal
-    atomicMax(a.rexp + w * 32 + lane, exp_bits(acc) - 1023);
-    a.ctrl->rescale[t & 1] = 1;
-  }
-}
-
-// Stores the result of one (vertex, word) of a heavy row; returns the number
-// of slots that reached the vertex (uniform over the warp).
+// Stores the result of one (vertex, word) of a heavy row; lane 0 returns
+// the number of slots that reached the vertex.
 __device__ __forceinline__ int finish_pull(const Args &a, int32_t v, int w, int t, uint32_t newm, int lane,
                                            double acc) {
   if (!newm) return 0;
-  put_counts(a, v, w, t, newm, lane, acc);
+  put_counts<1>(a, v, w * 32 + lane, t, newm >> lane & 1u, {acc});
   if (lane == 0) {
     a.lm[((int64_t)(t + 1) * a.n_cap + v) * a.W + w] = newm;
     a.seen[(int64_t)v * a.W + w] |= newm;
     atomicMin(a.lmin + v, t + 1);
   }
-  return __popc(newm);
+  return lane == 0 ? __popc(newm) : 0;
 }
 
 // Arms the neighbours of a vertex first reached on level lvl: a neighbour
@@ -568,35 +616,57 @@ __device__ __forceinline__ void chain_in(const Args &a, const Slot *slots, int n
   a.cdep[iv] = sum;
 }
 
-// delta, q and the BC partial (in word w0's place) of kWords words of a vertex
-// at level lev; every load is issued before the first use.
-template <typename QT, int kWords>
-__device__ __forceinline__ void finish_dep(const Args &a, int32_t reach, int32_t v, int w0, int lev,
-                                           const uint32_t (&act)[kWords], int lane, const double (&sum)[kWords],
-                                           bool chains, bool scaled) {
+// delta and q of a lane's slots (the first: b, of kN) of a vertex at level lev, and
+// the BC partial of the warp's slots (in word w0's place); every load is issued
+// before the first use.
+template <typename QT, int kN>
+__device__ __forceinline__ void finish_dep(const Args &a, int32_t reach, int32_t v, int w0, int b, int lev, uint32_t act,
+                                           int lane, const double (&sum)[kN], bool chains, bool scaled) {
   constexpr bool kF32 = sizeof(QT) == 4;
-  const int64_t idx = ((int64_t)v * a.W + w0) * 32 + lane;
-  double sv[kWords], in[kWords];
+  const int64_t idx = (int64_t)v * a.W * 32 + b;
+  double sv[kN], in[kN], ws[kN];
 #pragma unroll
-  for (int k = 0; k < kWords; ++k) {
-    const bool on = (act[k] >> lane) & 1u;
-    sv[k] = on ? __ldcg(a.sig + idx + k * 32) : 1.0;
-    in[k] = on && chains ? __ldcg(a.cdep + idx + k * 32) : 0.0;
+  for (int k = 0; k < kN; ++k) {
+    sv[k] = 1.0;
+    in[k] = ws[k] = 0.0;
+  }
+  if (act) {
+    if constexpr (kN == kLaneSlots) {
+      ld_slots(a.sig + idx, sv);
+      ld_slots(a.wsrc + b, ws);
+      if (chains) ld_slots(a.cdep + idx, in);
+    } else {
+      sv[0] = __ldcg(a.sig + idx);
+      ws[0] = __ldcg(a.wsrc + b);
+      if (chains) in[0] = __ldcg(a.cdep + idx);
+    }
   }
   double contrib = 0.0;
+  QT qs[kN];
 #pragma unroll
-  for (int k = 0; k < kWords; ++k) {
-    if (!((act[k] >> lane) & 1u)) continue;
-    const int b = (w0 + k) * 32 + lane;
-    const int xd = scaled ? a.X[(int64_t)b * (a.tcap + 2) + lev] - a.X[(int64_t)b * (a.tcap + 2) + lev + 1] : 0;
+  for (int k = 0; k < kN; ++k) {
+    if (!(act >> k & 1u)) continue;
+    const int64_t xb = (int64_t)(b + k) * (a.tcap + 2) + lev;
+    const int xd = scaled ? a.X[xb] - a.X[xb + 1] : 0;
     const double delta = scale2(sv[k] * sum[k], xd) + in[k];
     const double qv = ((double)reach + 1.0 + delta) / sv[k];
     if (kF32) {
       const double aq = fabs(qv);
       if (!(aq >= (double)FLT_MIN * 0x1p24 && aq <= (double)FLT_MAX * 0x1p-24)) atomicExch(&a.ctrl->range_err, 1);
     }
-    reinterpret_cast<QT *>(a.q)[idx + k * 32] = (QT)qv;
-    contrib += delta * a.wsrc[b];
+    qs[k] = (QT)qv;
+    contrib += delta * ws[k];
+  }
+  QT *q = reinterpret_cast<QT *>(a.q) + idx;
+  bool whole = false;
+  if constexpr (kN == kLaneSlots) {
+    whole = act == 15u;
+    if (whole) st_slots(q, qs);
+  }
+  if (!whole) {
+#pragma unroll
+    for (int k = 0; k < kN; ++k)
+      if (act >> k & 1u) q[k] = qs[k];
   }
   contrib = warp_sum(contrib);  // fixed-order reduction of the slots
   if (lane == 0) atomicAdd(a.bcpart + (int64_t)v * a.W + w0, contrib);  // one writer a level: no wait for the old value
@@ -773,10 +843,12 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
     bool scaled = false;
     const unsigned long long all_found = (unsigned long long)n * (unsigned long long)bt.nslots;
     while (true) {
-      unsigned long long nf = 0;  // pairs this warp found on this level
+      unsigned int nf = 0;  // pairs this lane found on this level (fewer than 2^32: a lane's slots of a warp's rows)
       // Once a warp and phase: every warp writes the same words, and a store for
       // each row reached made that one address what the level waited for.
       auto report = [&](unsigned long long found) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) found += __shfl_xor_sync(0xffffffffu, found, o);
         if (lane != 0 || !found) return;
         atomicAdd(&a.ctrl->found, found);
         a.ctrl->more[t & 1] = 1;
@@ -797,30 +869,28 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
         const int w0 = (int)(task % halves) * kHalf;
         const int nw = min(kHalf, wpad - w0);
         const int32_t v = hv[hcv[c]];
-        uint32_t unseen[kHalf], any[kHalf];
+        uint32_t unseen[kHalf], got = 0;
         load_row(a.seen + (int64_t)v * W + w0, nw, unseen);
         uint32_t u_any = 0;
 #pragma unroll
-        for (int k = 0; k < kHalf; ++k) { unseen[k] = k < nw ? ~unseen[k] : 0u; any[k] = 0; u_any |= unseen[k]; }
-        Acc<false> acc[kHalf];
+        for (int k = 0; k < kHalf; ++k) { unseen[k] = k < nw ? ~unseen[k] : 0u; u_any |= unseen[k]; }
+        Acc<false> acc[kLaneSlots];
         if (u_any && __ldcg(a.armed + v) <= t + 1) {  // uniform over the CTA
           const int64_t e0 = hce0[c], e1 = hce1[c], sp = HS[v];
           const int64_t per = (e1 - e0 + kWarpsPerCta - 1) / kWarpsPerCta;
           const int64_t s0 = e0 + wib * per, s1 = min(e1, s0 + per);
-          if (s0 < min(s1, sp)) row_pass<double, false, 0>(a, lmt, a.sig, s0, min(s1, sp), w0, nw, unseen, any, acc, lane, t, scaled);
-          if (max(s0, sp) < s1) row_pass<double, false, 1>(a, a.lm, a.sig, max(s0, sp), s1, w0, nw, unseen, any, acc, lane, t, scaled);
+          if (s0 < min(s1, sp)) row_pass<double, false, 0>(a, S, lmt, a.sig, s0, min(s1, sp), w0, nw, unseen, got, acc, lane, t, scaled);
+          if (max(s0, sp) < s1) row_pass<double, false, 1>(a, S, a.lm, a.sig, max(s0, sp), s1, w0, nw, unseen, got, acc, lane, t, scaled);
         }
 #pragma unroll
-        for (int k = 0; k < kHalf; ++k) {
-          any[k] = __reduce_or_sync(0xffffffffu, any[k]);
-          S.acc[k][lane] = acc[k].value();
-          if (lane == 0) S.any[k] = any[k];  // this warp's hit masks, for the combine
-        }
+        for (int k = 0; k < kLaneSlots; ++k) S.acc[kLaneSlots * lane + k] = acc[k].value();
+        got = word_of(got, lane);
+        if (lane_bit(lane) == 0) S.any[lane_word(lane)] = got;  // this warp's hit masks, for the combine
         __syncthreads();
         for (int k = wib; k < nw; k += kWarpsPerCta) {  // fixed warp order
           double tot = 0.0;
           uint32_t mm = 0;
-          for (int x = 0; x < kWarpsPerCta; ++x) { tot += scratch[x].acc[k][lane]; mm |= scratch[x].any[k]; }
+          for (int x = 0; x < kWarpsPerCta; ++x) { tot += scratch[x].acc[k * 32 + lane]; mm |= scratch[x].any[k]; }
           a.hacc[((hc0 + c) * W + w0 + k) * 32 + lane] = tot;
           if (lane == 0) a.hmask[(hc0 + c) * W + w0 + k] = mm;
         }
@@ -829,11 +899,10 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
       // light rows: (vertex block, quarter) tasks. Lane l holds vertex l's row and
       // unseen slots; the next active row's first neighbours are loaded while
       // this one's counts are gathered. Bound by the latency of a row's chain of
-      // loads (neighbours, their masks, counts), 48 warps an SM in flight. Two
-      // passes of 512 on R-MAT 20: the forward rows took 89.7 ms with a flag store a
-      // row, the row's masks re-read a row at a time and 20 shuffles to fold the
-      // hits, 51.1 ms so; the backward rows, likewise, 74.2 and 69.2. CTAs per SM 4 /
-      // 5 / 6: 199 / 183 / 180.5 ms a kernel.
+      // loads (neighbours, their masks, counts), 40 warps an SM in flight, and by
+      // instructions issued. Two passes of 512 on R-MAT 20, forward / backward rows:
+      // 51.1 / 69.2 ms with a word's slot a lane, that is four loads, five shuffles
+      // and four masks a hit; 41.4 / 58.9 ms with four slots a lane.
       for (int64_t tk = gwarp(); tk < ntask; tk = next_block(a.wq + t, lane)) {
         const int64_t v0 = tk / halves * bs;
         const int w0 = (int)(tk % halves) * kHalf;
@@ -862,35 +931,29 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
           const int units = (int)(len >> 16), arcs = (int)(len & 0xffff);
           const uint32_t unseen[kHalf] = {__shfl_sync(0xffffffffu, un.x, j), __shfl_sync(0xffffffffu, un.y, j),
                                           __shfl_sync(0xffffffffu, un.z, j), __shfl_sync(0xffffffffu, un.w, j)};
-          uint32_t any[kHalf];
-          load_row(lmt + (int64_t)u * W + w0, lane < units ? kHalf : 0, any);
+          uint32_t f[kHalf], got = 0;
+          load_row(lmt + (int64_t)u * W + w0, lane < units ? kHalf : 0, f);
 #pragma unroll
-          for (int k = 0; k < kHalf; ++k) any[k] &= unseen[k];
-          Acc<false> acc[kHalf];
-          walk_hits<double, false, 0>(a, a.sig + (int64_t)w0 * 32 + lane, u, 0, any, acc, lane);
+          for (int k = 0; k < kHalf; ++k) f[k] &= unseen[k];
+          Acc<false> acc[kLaneSlots];
+          walk_hits<double, false, 0>(a, S, a.sig + (int64_t)w0 * 32 + kLaneSlots * lane, u, 0, f, got, acc, lane);
           if (units > 32)
-            row_pass<double, false, 0>(a, lmt, a.sig, e0 + 32, e0 + units, w0, kHalf, unseen, any, acc, lane, t);
+            row_pass<double, false, 0>(a, S, lmt, a.sig, e0 + 32, e0 + units, w0, kHalf, unseen, got, acc, lane, t);
           if (units < arcs)
-            row_pass<double, false, 1>(a, a.lm, a.sig, e0 + units, e0 + arcs, w0, kHalf, unseen, any, acc, lane, t, scaled);
-          uint32_t hit = 0;
-#pragma unroll
-          for (int k = 0; k < kHalf; ++k) {
-            any[k] = __reduce_or_sync(0xffffffffu, any[k]);
-            hit |= any[k];
-            nf += __popc(any[k]);
+            row_pass<double, false, 1>(a, S, a.lm, a.sig, e0 + units, e0 + arcs, w0, kHalf, unseen, got, acc, lane, t, scaled);
+          if (!__ballot_sync(0xffffffffu, got != 0u)) continue;
+          nf += __popc(got);
+          const double sum[kLaneSlots] = {acc[0].value(), acc[1].value(), acc[2].value(), acc[3].value()};
+          put_counts<kLaneSlots>(a, v, w0 * 32 + kLaneSlots * lane, t, got, sum);
+          got = word_of(got, lane);
+          if (lane_bit(lane) == 0) {  // a lane for each word
+            const int k = lane_word(lane);
+            a.lm[((int64_t)(t + 1) * a.n_cap + v) * W + w0 + k] = got;
+            a.seen[(int64_t)v * W + w0 + k] = ~(k == 0 ? unseen[0] : k == 1 ? unseen[1] : k == 2 ? unseen[2] : unseen[3]) | got;
           }
-          if (!hit) continue;
-#pragma unroll
-          for (int k = 0; k < kHalf; ++k) put_counts(a, v, w0 + k, t, any[k], lane, acc[k].value());
           int first = 0;
           const bool fresh = __shfl_sync(0xffffffffu, lmin, j) == INT_MAX;  // not reached on an earlier level
-          if (lane == 0) {
-            *reinterpret_cast<uint4 *>(a.lm + ((int64_t)(t + 1) * a.n_cap + v) * W + w0) =
-                make_uint4(any[0], any[1], any[2], any[3]);
-            *reinterpret_cast<uint4 *>(a.seen + (int64_t)v * W + w0) =
-                make_uint4(~unseen[0] | any[0], ~unseen[1] | any[1], ~unseen[2] | any[2], ~unseen[3] | any[3]);
-            if (fresh) first = atomicMin(a.lmin + v, t + 1) == INT_MAX;
-          }
+          if (lane == 0 && fresh) first = atomicMin(a.lmin + v, t + 1) == INT_MAX;
           if (fresh && __shfl_sync(0xffffffffu, first, 0)) arm_arcs(a, e0, e0 + arcs, t + 1, lane, 32);
         }
       }
@@ -1015,30 +1078,29 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
         const int w0 = (int)(task % halves) * kHalf;
         const int nw = min(kHalf, wpad - w0);
         const int32_t v = hv[hcv[c]];
-        uint32_t act[kHalf], any[kHalf];
+        uint32_t act[kHalf], got = 0;
         load_row(lm_here + (int64_t)v * W + w0, nw, act);
         uint32_t a_any = 0;
 #pragma unroll
         for (int k = 0; k < kHalf; ++k) {
           act[k] = k < nw ? act[k] : 0u;
-          any[k] = 0;
           a_any |= act[k];
         }
-        Acc<kComp> acc[kHalf];
+        Acc<kComp> acc[kLaneSlots];
         if (a_any) {  // uniform over the CTA
           const int64_t e0 = hce0[c], e1 = hce1[c], sp = HS[v];
           const int64_t per = (e1 - e0 + kWarpsPerCta - 1) / kWarpsPerCta;
           const int64_t s0 = e0 + wib * per, s1 = min(e1, s0 + per);
           if (lev < tlast && s0 < min(s1, sp))
-            row_pass<QT, kComp, 0>(a, lm_next, q, s0, min(s1, sp), w0, nw, act, any, acc, lane, lev + 1, scaled);
-          if (max(s0, sp) < s1) row_pass<QT, kComp, 2>(a, a.lm, q, max(s0, sp), s1, w0, nw, act, any, acc, lane, lev + 1, scaled, tlast);
+            row_pass<QT, kComp, 0>(a, S, lm_next, q, s0, min(s1, sp), w0, nw, act, got, acc, lane, lev + 1, scaled);
+          if (max(s0, sp) < s1) row_pass<QT, kComp, 2>(a, S, a.lm, q, max(s0, sp), s1, w0, nw, act, got, acc, lane, lev + 1, scaled, tlast);
         }
 #pragma unroll
-        for (int k = 0; k < kHalf; ++k) S.acc[k][lane] = acc[k].value();
+        for (int k = 0; k < kLaneSlots; ++k) S.acc[kLaneSlots * lane + k] = acc[k].value();
         __syncthreads();
         for (int k = wib; k < nw; k += kWarpsPerCta) {  // fixed warp order
           double tot = 0.0;
-          for (int x = 0; x < kWarpsPerCta; ++x) tot += scratch[x].acc[k][lane];
+          for (int x = 0; x < kWarpsPerCta; ++x) tot += scratch[x].acc[k * 32 + lane];
           a.hacc[((hc0 + c) * W + w0 + k) * 32 + lane] = tot;
         }
         __syncthreads();
@@ -1071,20 +1133,24 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
           const int units = (int)(len >> 16), arcs = (int)(len & 0xffff);
           const uint32_t act[kHalf] = {__shfl_sync(0xffffffffu, on.x, j), __shfl_sync(0xffffffffu, on.y, j),
                                        __shfl_sync(0xffffffffu, on.z, j), __shfl_sync(0xffffffffu, on.w, j)};
-          Acc<kComp> acc[kHalf];
-          uint32_t any[kHalf] = {};
+          Acc<kComp> acc[kLaneSlots];
+          uint32_t got = 0;
           if (lev < tlast) {
-            load_row(lm_next + (int64_t)u * W + w0, lane < units ? kHalf : 0, any);
+            uint32_t f[kHalf];
+            load_row(lm_next + (int64_t)u * W + w0, lane < units ? kHalf : 0, f);
 #pragma unroll
-            for (int k = 0; k < kHalf; ++k) any[k] &= act[k];
-            walk_hits<QT, kComp, 0>(a, q + (int64_t)w0 * 32 + lane, u, 0, any, acc, lane);
+            for (int k = 0; k < kHalf; ++k) f[k] &= act[k];
+            walk_hits<QT, kComp, 0>(a, S, q + (int64_t)w0 * 32 + kLaneSlots * lane, u, 0, f, got, acc, lane);
             if (units > 32)
-              row_pass<QT, kComp, 0>(a, lm_next, q, e0 + 32, e0 + units, w0, kHalf, act, any, acc, lane, lev + 1);
+              row_pass<QT, kComp, 0>(a, S, lm_next, q, e0 + 32, e0 + units, w0, kHalf, act, got, acc, lane, lev + 1);
           }
           if (units < arcs)
-            row_pass<QT, kComp, 2>(a, a.lm, q, e0 + units, e0 + arcs, w0, kHalf, act, any, acc, lane, lev + 1, scaled, tlast);
-          const double sum[kHalf] = {acc[0].value(), acc[1].value(), acc[2].value(), acc[3].value()};
-          finish_dep<QT, kHalf>(a, __shfl_sync(0xffffffffu, reach, j), v, w0, lev, act, lane, sum, units < arcs, scaled);
+            row_pass<QT, kComp, 2>(a, S, a.lm, q, e0 + units, e0 + arcs, w0, kHalf, act, got, acc, lane, lev + 1, scaled, tlast);
+          const double sum[kLaneSlots] = {acc[0].value(), acc[1].value(), acc[2].value(), acc[3].value()};
+          const int k = lane_word(lane);
+          const uint32_t own = (k == 0 ? act[0] : k == 1 ? act[1] : k == 2 ? act[2] : act[3]) >> lane_bit(lane) & 15u;
+          finish_dep<QT, kLaneSlots>(a, __shfl_sync(0xffffffffu, reach, j), v, w0, w0 * 32 + kLaneSlots * lane, lev, own, lane,
+                                     sum, units < arcs, scaled);
         }
       }
       if (nheavy) {
@@ -1098,7 +1164,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
           if (!act) continue;
           double sum = 0.0;
           for (int32_t c = hfst[h]; c < hfst[h + 1]; ++c) sum += __ldcg(a.hacc + ((hc0 + c) * W + w) * 32 + lane);
-          finish_dep<QT, 1>(a, rch[v], v, w, lev, {act}, lane, {sum}, HS[v] < HR[v + 1], scaled);
+          finish_dep<QT, 1>(a, rch[v], v, w, w * 32 + lane, lev, act >> lane & 1u, lane, {sum}, HS[v] < HR[v + 1], scaled);
         }
       }
       grid_sync(a);
