@@ -132,6 +132,8 @@ struct Ctrl {
   unsigned long long found;  // forward: (core vertex, slot) pairs reached so far
 };
 
+constexpr int32_t kNoSlot = -2;
+
 struct Args {
   // contracted rows of the core vertices; BCC b's rows start at hvo[b]
   const int64_t *hvo;
@@ -175,6 +177,7 @@ struct Args {
   double *bcpart;   // [n_cap][W] BC partials of the core vertices
   double *cdep;     // [n_cap][W][32] dependency a core vertex receives from its chains' vertices
   double *wsrc;     // [B] reach(source)+1 of each slot of the pass
+  int32_t *schain;  // [B] chain of each slot's source (-1: a core vertex; kNoSlot: no slot)
   int32_t *X;       // [B][tcap+2]
   int32_t *rexp;    // [B] per-level max exponent (rescale)
   int64_t n_cap;    // core rows allocated (>= largest core)
@@ -293,6 +296,11 @@ struct End {
   double s, qs;
 };
 __device__ __forceinline__ End source_end() { return End{0, 0, 1.0, 0.0}; }
+
+// The share of A's paths, sA / (sA + sB), while no level was rescaled: one division
+// where 1 / (1 + sB / sA) takes two. Halves, so that the sum of two counts that
+// FP64 holds is one as well.
+__device__ __forceinline__ double path_share(double sA, double sB) { return 0.5 * sA / (0.5 * sA + 0.5 * sB); }
 
 // Dependency of stretch vertex i on the slot's source when i takes its
 // shortest paths from A (2i < D): the chain vertices beyond i on the A-fed
@@ -531,31 +539,37 @@ __device__ __forceinline__ void arm_arcs(const Args &a, int64_t e0, int64_t e1, 
 
 // ============================================================== backward ===
 
-// What core vertex v receives from the vertices of its chains, for the 32
-// slots of word w (the part that needs only forward results): cdep[v][w][.].
-// Chain-arc data are loaded lane-parallel, 32 arcs at a time; then, four arcs
-// at a time, the far ends' levels and path counts in one batch of loads (a
-// tie needs the path counts on about half the slots, so a warp nearly always
-// needs them: loading them with the levels takes one memory round trip per
-// group instead of one more per tying arc), then their level exponents.
-constexpr int kArcGroup = 4;
 __device__ __forceinline__ int level_index(const Args &a, int d) { return min(max(d, 0), a.tcap + 1); }
-__device__ __forceinline__ void chain_in(const Args &a, const Slot *slots, int nslots, int32_t v, int w, int64_t c0,
-                                         int64_t c1, int lane, bool scaled) {
-  const int W = a.W;
-  const int b = w * 32 + lane;
-  const bool live = b < nslots;
-  const int64_t iv = ((int64_t)v * W + w) * 32 + lane;
-  const int32_t *xb = a.X + (int64_t)b * (a.tcap + 2);
-  End A{0, 0, 1.0, 0.0};
-  Slot sl{0, -1, 0, 0};
-  if (live) {
-    A.d = __ldcg(a.d + iv);
-    A.s = __ldcg(a.sig + iv);
-    sl = slots[b];
-    A.x = scaled ? __ldcg(xb + level_index(a, A.d)) : 0;
-  }
-  double sum = 0.0;
+__device__ __forceinline__ int level_base(const Args &a, int b, int d) {
+  return __ldcg(a.X + (int64_t)b * (a.tcap + 2) + level_index(a, d));
+}
+
+// What a slot of an end receives from a chain of k vertices with prefix sums P (out
+// of line: chains with something hanging off, rescaled levels, and the slots whose
+// source sits on the chain, at pos >= 0).
+__device__ __noinline__ double chain_in_any(const double *P, int k, bool right, int pos, const End &A, const End &B) {
+  if (pos < 0) return end_dep(Stretch{P, 0, k, right}, A, B);
+  return end_dep(right ? Stretch{P, pos + 1, k, true} : Stretch{P, 0, pos, false}, A, source_end());  // ends at the source
+}
+
+// What core vertex v receives from the vertices of its chains, for 32 * kInSlots
+// slots, this lane's from b on (the part that needs only forward results): cdep.
+// Chain-arc data are loaded lane-parallel, 32 arcs at a time, and handed around; an
+// arc's levels and path counts at its far end are loaded together (a tie needs the
+// path counts on about half the slots, so a warp nearly always needs them). Bound
+// by the instructions of the closed form, and by registers. Two passes of 512 on
+// R-MAT 20: 23.9 ms with one slot a lane and two divisions a tie; 17.8 with two
+// slots; with two or four arcs in flight 20.6 and 23.3, with four slots 31.8 (spills).
+constexpr int kInSlots = 2;
+__device__ __forceinline__ void chain_in(const Args &a, const Slot *slots, int32_t v, int b, int64_t c0, int64_t c1,
+                                         int lane, bool scaled) {
+  const int64_t stride = (int64_t)a.W * 32;
+  const int64_t iv = (int64_t)v * stride + b;
+  const int2 dv = __ldcg(reinterpret_cast<const int2 *>(a.d + iv)), cv = __ldcg(reinterpret_cast<const int2 *>(a.schain + b));
+  const double2 sv = __ldcg(reinterpret_cast<const double2 *>(a.sig + iv));
+  const int32_t dA[kInSlots] = {dv.x, dv.y}, ch[kInSlots] = {cv.x, cv.y};
+  const double sA[kInSlots] = {sv.x, sv.y};
+  double sum[kInSlots] = {0.0, 0.0};
   for (int64_t base = c0; base < c1; base += 32) {
     const int64_t e = base + lane;
     int32_t u = 0, cid = 0, k = 0;
@@ -567,53 +581,33 @@ __device__ __forceinline__ void chain_in(const Args &a, const Slot *slots, int n
       poff = ldg(a.cpre_off + (cid >> 1));
     }
     const int cnt = (int)min((int64_t)32, c1 - base);
-    for (int j0 = 0; j0 < cnt; j0 += kArcGroup) {
-      int32_t uj[kArcGroup], cj[kArcGroup], kj[kArcGroup], dB[kArcGroup], xB[kArcGroup];
-      int64_t pj[kArcGroup];
-      double sB[kArcGroup];
+    for (int j = 0; j < cnt; ++j) {
+      const int64_t iu = (int64_t)__shfl_sync(0xffffffffu, u, j) * stride + b;
+      const int2 dB = __ldcg(reinterpret_cast<const int2 *>(a.d + iu));
+      const double2 sB = __ldcg(reinterpret_cast<const double2 *>(a.sig + iu));
+      const int cj = __shfl_sync(0xffffffffu, cid, j), kj = __shfl_sync(0xffffffffu, k, j);
+      const int64_t pj = __shfl_sync(0xffffffffu, poff, j);
 #pragma unroll
-      for (int r = 0; r < kArcGroup; ++r) {  // the far ends' levels and path counts, all in flight
-        const int j = (j0 + r) & 31;
-        uj[r] = __shfl_sync(0xffffffffu, u, j);
-        cj[r] = __shfl_sync(0xffffffffu, cid, j);
-        kj[r] = __shfl_sync(0xffffffffu, k, j);
-        pj[r] = __shfl_sync(0xffffffffu, poff, j);
-        const int64_t ib = ((int64_t)uj[r] * W + w) * 32 + lane;
-        const bool ld = live && j0 + r < cnt;
-        dB[r] = ld ? __ldcg(a.d + ib) : 0;
-        sB[r] = ld ? __ldcg(a.sig + ib) : 1.0;
-      }
-#pragma unroll
-      for (int r = 0; r < kArcGroup; ++r) xB[r] = (scaled && live && j0 + r < cnt) ? __ldcg(xb + level_index(a, dB[r])) : 0;
-#pragma unroll
-      for (int r = 0; r < kArcGroup; ++r) {
-        if (!live || j0 + r >= cnt) continue;
-        const bool same = sl.chain == (cj[r] >> 1);  // the source sits on this chain
-        if (pj[r] < 0 && !same) {
+      for (int r = 0; r < kInSlots; ++r) {
+        const bool same = ch[r] == (cj >> 1);  // the source sits on this chain
+        const int db = r ? dB.y : dB.x;
+        const double sb = r ? sB.y : sB.x;
+        if (!same && pj < 0 && !scaled) {
           // nothing hangs off the chain: prefix sums are positions; the
           // vertices up to P = D/2 are fed from A, the one at D/2 ties when D is even
-          const int D = dB[r] + kj[r] - A.d - 1;
+          const int D = db + kj - dA[r] - 1, P = D >> 1;
           if (D < 0) continue;
-          const int P = D >> 1;
-          if ((D & 1) == 0 && P <= kj[r] - 1)
-            sum += (double)P + 1.0 / (1.0 + scale2(sB[r] / A.s, xB[r] - A.x));
-          else
-            sum += (double)(min(kj[r] - 1, P) + 1);
-          continue;
+          if (!(D & 1) && P < kj) sum[r] += (double)P + path_share(sA[r], sb);
+          else sum[r] += (double)(min(kj - 1, P) + 1);
+        } else if (ch[r] != kNoSlot) {
+          const End A{dA[r], scaled ? level_base(a, b + r, dA[r]) : 0, sA[r], 0.0};
+          const End B{db, scaled ? level_base(a, b + r, db) : 0, sb, 0.0};
+          sum[r] += chain_in_any(pj < 0 ? nullptr : a.cpre + pj, kj, cj & 1, same ? slots[b + r].pos : -1, A, B);
         }
-        const bool right = cj[r] & 1;
-        const double *Pj = pj[r] < 0 ? nullptr : a.cpre + pj[r];
-        Stretch st{Pj, 0, kj[r], right};
-        End B{dB[r], xB[r], sB[r], 0.0};
-        if (same) {  // the stretch ends at the source
-          B = source_end();
-          st = right ? Stretch{Pj, sl.pos + 1, kj[r], true} : Stretch{Pj, 0, sl.pos, false};
-        }
-        sum += end_dep(st, A, B);
       }
     }
   }
-  a.cdep[iv] = sum;
+  *reinterpret_cast<double2 *>(a.cdep + iv) = make_double2(sum[0], sum[1]);
 }
 
 // delta and q of a lane's slots (the first: b, of kN) of a vertex at level lev, and
@@ -710,17 +704,6 @@ static_assert(kHeavyDeg < 1 << 16, "a light row's length takes 16 bits");
 #ifndef BCGPU_BATCHED_HEAVY_DYN
 #define BCGPU_BATCHED_HEAVY_DYN 1
 #endif
-// Chain in-flow tasks (core vertex, word): a fixed warp stride (0) or a
-// work counter (1), as the light rows (168.7 against 161.9 GTEPS on
-// RMAT-20: a hub's words carry thousands of chain arcs each). Chain-vertex
-// tasks (one chain, every word) likewise (BCGPU_BATCHED_CHAINV_DYN: 167.9-
-// 168.0 against 165.5).
-#ifndef BCGPU_BATCHED_CHAININ_DYN
-#define BCGPU_BATCHED_CHAININ_DYN 1
-#endif
-#ifndef BCGPU_BATCHED_CHAINV_DYN
-#define BCGPU_BATCHED_CHAINV_DYN 1
-#endif
 __device__ __forceinline__ int64_t next_chunk_task(int64_t task, int *counter) {
 #if BCGPU_BATCHED_HEAVY_DYN
   __shared__ int s_next;
@@ -807,6 +790,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
       a.rexp[i] = INT_MIN;
       a.X[i * (a.tcap + 2)] = 0;
       a.wsrc[i] = i < bt.nslots ? (double)rch[slots[i].src] + 1.0 : 0.0;
+      a.schain[i] = i < bt.nslots ? slots[i].chain : kNoSlot;
     }
     for (int64_t i = gtid; i < 4 * ((int64_t)a.tcap + 3) + 2; i += gthreads) a.wq[i] = 0;
     if (gtid == 0) {
@@ -1051,15 +1035,11 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
     }
     // what the core vertices receive from their chains' vertices
     if (bt.kmax) {
-#if BCGPU_BATCHED_CHAININ_DYN
-      for (int64_t task = gwarp(); task < (int64_t)n * words; task = next_block(a.wq + 4 * (a.tcap + 3), lane)) {
-#else
-      for (int64_t task = gwarp(); task < (int64_t)n * words; task += nwarps()) {
-#endif
-        const int32_t v = (int32_t)(task / words);
-        const int w = (int)(task % words);
+      const int parts = (words + kInSlots - 1) / kInSlots;
+      for (int64_t task = gwarp(); task < (int64_t)n * parts; task = next_block(a.wq + 4 * (a.tcap + 3), lane)) {
+        const int32_t v = (int32_t)(task / parts);
         const int64_t c0 = HS[v], c1 = HR[v + 1];
-        if (c0 < c1) chain_in(a, slots, bt.nslots, v, w, c0, c1, lane, scaled);
+        if (c0 < c1) chain_in(a, slots, v, ((int)(task % parts) * 32 + lane) * kInSlots, c0, c1, lane, scaled);
       }
       grid_sync(a);
     }
@@ -1172,20 +1152,19 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
       PHASE_COUNT(17);
     }
 
-    // ---- chain vertices: one warp per chain, every word; each lane sums its
-    // slots' contributions over the words (registers for chains of up to
-    // kRegVerts vertices), then one warp reduction per chain vertex goes
-    // straight into BC (one writer per vertex: fixed order)
-    {
+    // ---- chain vertices: one warp per chain, every slot, two neighbouring ones a
+    // lane; each lane sums its slots' contributions (registers for chains of up to
+    // kRegVerts vertices), then one warp reduction per chain vertex goes straight
+    // into BC (one writer per vertex: fixed order). Bound by the instructions of
+    // the closed form: two passes of 512 on R-MAT 20 took 28.3 ms with a slot a lane
+    // and two divisions for each side of a tie, 16.5 so.
+    if (bt.kmax) {
       constexpr int kRegVerts = 8;
       const int bad = *(volatile int *)&a.ctrl->range_err;
       const int64_t ch0 = a.chain_off[bt.bcc];
       const int64_t nch = a.chain_off[bt.bcc + 1] - ch0;
-#if BCGPU_BATCHED_CHAINV_DYN
+      const QT *qq = reinterpret_cast<const QT *>(a.q);
       for (int64_t task = gwarp(); task < nch; task = next_block(a.wq + 4 * (a.tcap + 3) + 1, lane)) {
-#else
-      for (int64_t task = gwarp(); task < nch; task += nwarps()) {
-#endif
         const int64_t c = ch0 + task;
         const int32_t L = a.chain_l[c], R = a.chain_r[c], cs = a.chain_start[c], k = a.chain_len[c];
         const int64_t poff = a.cpre_off[c];
@@ -1193,85 +1172,105 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
         double part[kRegVerts];
 #pragma unroll
         for (int j = 0; j < kRegVerts; ++j) part[j] = 0.0;
-        for (int w = 0; w < words; ++w) {
-          const int b = w * 32 + lane;
-          const bool live = b < bt.nslots;
-          const int64_t iL = ((int64_t)L * W + w) * 32 + lane, iR = ((int64_t)R * W + w) * 32 + lane;
-          End eL{0, 0, 1.0, 0.0}, eR{0, 0, 1.0, 0.0};
-          int on = -1;
-          if (live) {  // the ends' levels, then only the path counts / q the closed forms use
-            eL.d = __ldcg(a.d + iL);
-            eR.d = __ldcg(a.d + iR);
-            const Slot sl = slots[b];
-            on = sl.chain == c ? sl.pos : -1;
-            // stretches: [L, R] or, with the source on the chain, [L, source] and [source, R]
-            const int mL = on < 0 ? k : on, dBL = on < 0 ? eR.d : 0;           // seen from L
-            const int mR = on < 0 ? k : k - 1 - on, dBR = on < 0 ? eL.d : 0;  // seen from R
-            const int DL = dBL + mL - eL.d - 1, DR = dBR + mR - eR.d - 1;
-            const bool tieL = mL > 0 && DL >= 0 && (DL & 1) == 0 && DL / 2 <= mL - 1;
-            const bool tieR = mR > 0 && DR >= 0 && (DR & 1) == 0 && DR / 2 <= mR - 1;
-            // B's paths through the stretch: R fed via the chain from L, or L from R
-            const bool viaL = on < 0 && eR.d == eL.d + k + 1, viaR = on < 0 && eL.d == eR.d + k + 1;
-            const bool srcL = on >= 0 && eL.d == on + 1, srcR = on >= 0 && eR.d == k - on;  // fed from the source
-            const int32_t *xb = a.X + (int64_t)b * (a.tcap + 2);
-            const QT *qq = reinterpret_cast<const QT *>(a.q);
-            const bool sig = tieL || tieR || viaL || viaR;
-            if (sig) {
-              eL.s = __ldcg(a.sig + iL);
-              eL.x = scaled ? __ldcg(xb + level_index(a, eL.d)) : 0;
-              eR.s = __ldcg(a.sig + iR);
-              eR.x = scaled ? __ldcg(xb + level_index(a, eR.d)) : 0;
-            }
-            if (viaR || srcL) {
-              eL.qs = (double)__ldcg(qq + iL);
-              if (!sig) eL.x = scaled ? __ldcg(xb + level_index(a, eL.d)) : 0;
-            }
-            if (viaL || srcR) {
-              eR.qs = (double)__ldcg(qq + iR);
-              if (!sig) eR.x = scaled ? __ldcg(xb + level_index(a, eR.d)) : 0;
+        for (int b = 2 * lane; b < wpad * 32; b += 64) {
+          const int64_t iL = (int64_t)L * W * 32 + b, iR = (int64_t)R * W * 32 + b;
+          // the ends' levels, then only the path counts / q the closed forms use
+          const int2 dL2 = __ldcg(reinterpret_cast<const int2 *>(a.d + iL)), dR2 = __ldcg(reinterpret_cast<const int2 *>(a.d + iR));
+          const int2 on2 = __ldcg(reinterpret_cast<const int2 *>(a.schain + b));
+          const double2 ws2 = __ldcg(reinterpret_cast<const double2 *>(a.wsrc + b));
+          const int32_t dL[2] = {dL2.x, dL2.y}, dR[2] = {dR2.x, dR2.y}, on[2] = {on2.x, on2.y};
+          const double ws[2] = {ws2.x, ws2.y};
+          bool tie[2], sig = false, via = false;
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const int D = dR[r] + k - dL[r] - 1;
+            tie[r] = D >= 0 && !(D & 1) && D < 2 * k;
+            const bool far = D > 2 * k - 1 || D < -1;  // |level difference| = k + 1: one end's paths come over the chain
+            sig |= tie[r] || far;
+            via |= far;
+          }
+          double2 sL2 = make_double2(1.0, 1.0), sR2 = sL2;
+          QT qL[2] = {}, qR[2] = {};
+          if (sig) {
+            sL2 = __ldcg(reinterpret_cast<const double2 *>(a.sig + iL));
+            sR2 = __ldcg(reinterpret_cast<const double2 *>(a.sig + iR));
+          }
+          if (via) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              qL[r] = __ldcg(qq + iL + r);
+              qR[r] = __ldcg(qq + iR + r);
             }
           }
-          const double wsrc = live ? a.wsrc[b] : 0.0;
-          // Source off the chain (the common case), in prefix sums from L:
-          // vertex j is fed from L iff 2j <= D; a tie vertex t = D/2 shares
-          // its reach+1 between the sides in proportion to sigma_L, sigma_R;
-          // else the L-fed vertices end at pl, and the far end's q enters
-          // when the chain carries its shortest paths.
-          int tv = -1, pl = -1;
-          double fL = 0.0, fR = 0.0;  // L-side and R-side constants
-          if (live && on < 0) {
-            const int D = eR.d + k - eL.d - 1;
-            if (D >= 0 && (D & 1) == 0 && D / 2 <= k - 1) {
-              tv = D / 2;
-              const double p0 = chain_pre(P, tv), p1 = chain_pre(P, tv + 1), wt = p1 - p0;
-              fL = p0 + wt / (1.0 + scale2(eR.s / eL.s, eR.x - eL.x));
-              fR = -p1 + wt / (1.0 + scale2(eL.s / eR.s, eL.x - eR.x));
-            } else {
-              pl = D >= 0 ? min(k - 1, D / 2) : -1;
-              const double p1 = chain_pre(P, pl + 1);
-              fL = p1 + (eR.d == eL.d + k + 1 ? scale2(eL.s * eR.qs, eL.x - eR.x) : 0.0);
-              fR = -p1 + (eL.d == eR.d + k + 1 ? scale2(eR.s * eL.qs, eR.x - eL.x) : 0.0);
+          const double sL[2] = {sL2.x, sL2.y}, sR[2] = {sR2.x, sR2.y};
+          bool own = false;  // a slot's source sits on the chain
+          int lo[2], hi[2];
+          double fL[2], fR[2];  // L-side and R-side constants
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            own |= on[r] == c;
+            lo[r] = 0;
+            hi[r] = k;  // nothing from this slot
+            fL[r] = fR[r] = 0.0;
+            if (on[r] == kNoSlot || on[r] == c) continue;
+            // in prefix sums from L: vertex j is fed from L iff 2j <= D; a tie
+            // vertex t = D/2 shares its reach+1 between the sides in proportion to
+            // sigma_L, sigma_R; else the L-fed vertices end at D/2, and the far
+            // end's q enters when the chain carries its shortest paths.
+            const int D = dR[r] + k - dL[r] - 1;
+            lo[r] = D < 0 ? 0 : min(k, (D >> 1) + (tie[r] ? 0 : 1));  // vertices [0, lo) are fed from L
+            hi[r] = tie[r] ? lo[r] + 1 : lo[r];                       // [hi, k) from R
+            const int x = scaled ? level_base(a, b + r, dL[r]) - level_base(a, b + r, dR[r]) : 0;
+            const double p0 = chain_pre(P, lo[r]), p1 = chain_pre(P, hi[r]);
+            fL[r] = p0;
+            fR[r] = -p1;
+            if (tie[r]) {
+              fL[r] += scaled ? (p1 - p0) / (1.0 + scale2(sR[r] / sL[r], -x)) : (p1 - p0) * path_share(sL[r], sR[r]);
+              fR[r] += scaled ? (p1 - p0) / (1.0 + scale2(sL[r] / sR[r], x)) : (p1 - p0) * path_share(sR[r], sL[r]);
+            } else if (D >= 2 * k) {
+              fL[r] += scale2(sL[r] * (double)qR[r], x);
+            } else if (D <= -2) {
+              fR[r] += scale2(sR[r] * (double)qL[r], -x);
             }
           }
-          auto dep_of = [&](int j) -> double {
-            if (!live) return 0.0;
-            if (on < 0) {
-              if (j == tv) return 0.0;
-              const bool from_l = tv >= 0 ? j < tv : j <= pl;
-              return (from_l ? fL - chain_pre(P, j + 1) : chain_pre(P, j) + fR) * wsrc;
-            }
-            if (j < on) return stretch_dep(Stretch{P, 0, on, false}, j, eL, source_end()) * wsrc;
-            if (j > on) return stretch_dep(Stretch{P, on + 1, k, false}, j - on - 1, source_end(), eR) * wsrc;
-            return 0.0;
+          auto dep = [&](int r, int j) {
+            const double y = j < lo[r] ? fL[r] - chain_pre(P, j + 1) : chain_pre(P, j) + fR[r];
+            return j >= lo[r] && j < hi[r] ? 0.0 : y * ws[r];
+          };
+          auto add = [&](int j, double x) {
+            const double tot = warp_sum(x);
+            if (lane == 0 && !bad) a.bc[vo + cs + j] += tot;
           };
           if (k <= kRegVerts) {
 #pragma unroll
             for (int j = 0; j < kRegVerts; ++j)
-              if (j < k) part[j] += dep_of(j);
+              if (j < k) part[j] += dep(0, j) + dep(1, j);
           } else {
-            for (int j = 0; j < k; ++j) {
-              const double tot = warp_sum(dep_of(j));
-              if (lane == 0 && !bad) a.bc[vo + cs + j] += tot;
+            for (int j = 0; j < k; ++j) add(j, dep(0, j) + dep(1, j));
+          }
+          if (__any_sync(0xffffffffu, own)) {  // rare: [L, source] and [source, R]
+            for (int r = 0; r < 2; ++r) {
+              const bool mine = (r ? on2.y : on2.x) == c;
+              const double wr = r ? ws2.y : ws2.x;
+              int pos = 0;
+              End eL{0, 0, 1.0, 0.0}, eR{0, 0, 1.0, 0.0};
+              if (mine) {
+                pos = slots[b + r].pos;
+                eL.d = r ? dL2.y : dL2.x;
+                eR.d = r ? dR2.y : dR2.x;
+                eL.s = __ldcg(a.sig + iL + r);
+                eR.s = __ldcg(a.sig + iR + r);
+                if (eL.d == pos + 1) eL.qs = (double)__ldcg(qq + iL + r);  // fed from the source
+                if (eR.d == k - pos) eR.qs = (double)__ldcg(qq + iR + r);
+                eL.x = scaled ? level_base(a, b + r, eL.d) : 0;
+                eR.x = scaled ? level_base(a, b + r, eR.d) : 0;
+              }
+              for (int j = 0; j < k; ++j) {
+                double x = 0.0;
+                if (mine && j < pos) x = stretch_dep(Stretch{P, 0, pos, false}, j, eL, source_end()) * wr;
+                if (mine && j > pos) x = stretch_dep(Stretch{P, pos + 1, k, false}, j - pos - 1, source_end(), eR) * wr;
+                add(j, x);
+              }
             }
           }
         }
@@ -1820,6 +1819,7 @@ int batched_build(const bc_bccs *B, const BatchedConfig &cfg, const int64_t *row
   ok &= ok && alloc(&p, n * WA * 8); a.bcpart = (double *)p;
   ok &= ok && alloc(&p, n * WA * 32 * 8); a.cdep = (double *)p;
   ok &= ok && alloc(&p, WA * 32 * 8); a.wsrc = (double *)p;
+  ok &= ok && alloc(&p, WA * 32 * 4); a.schain = (int32_t *)p;
   ok &= ok && alloc(&p, WA * 32 * (tcap + 2) * 4); a.X = (int32_t *)p;
   ok &= ok && alloc(&p, WA * 32 * 4); a.rexp = (int32_t *)p;
   ok &= ok && alloc(&p, sizeof(Ctrl)); a.ctrl = (Ctrl *)p;
