@@ -83,12 +83,12 @@ constexpr int kSmallCore = 16384;  // cores below this many vertices use kHeavyD
 constexpr int kChunkArcs = BCGPU_BATCHED_CHUNK;  // arcs per heavy chunk
 constexpr int kHalf = 4;           // words per pass over a vertex row
 // Resident CTAs per SM the kernel is compiled for (registers per thread =
-// 65536 / (kThreads * kMinCtas)); profiling builds may override it. Five CTAs (48
-// registers, some spilled to local memory): two passes of 512 sources on R-MAT 20
-// take 164.9 / 155.0 / 158.1 ms for 4 / 5 / 6 CTAs per SM, all passes of R-MAT 14
-// 164.5 / 161.4 / 169.5 ms.
+// 65536 / (kThreads * kMinCtas)); profiling builds may override it. Two passes of
+// 512 sources take, for 5 / 4 CTAs per SM: R-MAT 20 139.4 / 139.6 ms, R-MAT 17
+// 23.8 / 22.3 and in FP64 24.6 / 22.7; all passes of R-MAT 14 140.7 / 139.5. (With one
+// hit in flight R-MAT 20 took 164.9 / 155.0 / 158.1 ms for 4 / 5 / 6.)
 #ifndef BCGPU_BATCHED_MIN_CTAS
-#define BCGPU_BATCHED_MIN_CTAS 5
+#define BCGPU_BATCHED_MIN_CTAS 4
 #endif
 constexpr int kMinCtas = BCGPU_BATCHED_MIN_CTAS;
 // Light-row tasks per warp and level at least (smaller vertex blocks when
@@ -433,7 +433,22 @@ __device__ __forceinline__ void walk_hits(const Args &a, WarpScratch &S, const T
   const uint32_t *mine_at = &S.hit[0][lane_word(lane)];
   const int sh = lane_bit(lane), n = __popc(hits);
   const int64_t stride = (int64_t)a.W * 32;
-  for (int i = 0; i < n; ++i) {
+  int i = 0;
+  if (kLev == 0 && sizeof(T) == 4) {  // two hits' loads in flight: FP64 values would spill
+    for (; i + 2 <= n; i += 2) {
+      const uint32_t m0 = mine_at[i * kHalf] >> sh & 15u, m1 = mine_at[i * kHalf + kHalf] >> sh & 15u;
+      got |= m0 | m1;
+      T x[kLaneSlots] = {(T)0, (T)0, (T)0, (T)0}, y[kLaneSlots] = {(T)0, (T)0, (T)0, (T)0};
+      if (m0) ld_slots(vrow + (int64_t)S.hit_u[i] * stride, x);
+      if (m1) ld_slots(vrow + (int64_t)S.hit_u[i + 1] * stride, y);
+#pragma unroll
+      for (int k = 0; k < kLaneSlots; ++k) {
+        acc[k].add((double)(m0 >> k & 1u ? x[k] : (T)0));
+        acc[k].add((double)(m1 >> k & 1u ? y[k] : (T)0));
+      }
+    }
+  }
+  for (; i < n; ++i) {
     const uint32_t m = mine_at[i * kHalf] >> sh & 15u;
     const T *vu = vrow + (int64_t)S.hit_u[i] * stride;
     got |= m;
@@ -883,7 +898,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) batched_kernel(Args a) {
       // light rows: (vertex block, quarter) tasks. Lane l holds vertex l's row and
       // unseen slots; the next active row's first neighbours are loaded while
       // this one's counts are gathered. Bound by the latency of a row's chain of
-      // loads (neighbours, their masks, counts), 40 warps an SM in flight, and by
+      // loads (neighbours, their masks, counts), 32 warps an SM in flight, and by
       // instructions issued. Two passes of 512 on R-MAT 20, forward / backward rows:
       // 51.1 / 69.2 ms with a word's slot a lane, that is four loads, five shuffles
       // and four masks a hit; 41.4 / 58.9 ms with four slots a lane.
