@@ -77,6 +77,12 @@ constexpr int kHeavyDeg = BCGPU_BATCHED_HEAVY_DEG;
 // 32.1 for 128, 55.8 / 31.3 for 512).
 constexpr int kHeavyDegSmall = 512;
 constexpr int kSmallCore = 16384;  // cores below this many vertices use kHeavyDegSmall
+// On large cores a level has enough other rows to hide a longer one behind, and a
+// chunked row costs a partial sum in memory and its combine. Two passes of 512, rows
+// up to 1024 / 2048 arcs on a warp: R-MAT 17 (55,000 core vertices) 22.3 / 23.1 ms,
+// R-MAT 18 46.4 / 51.1, R-MAT 19 87.9 / 87.9, R-MAT 20 (430,000) 139.8 / 132.8.
+constexpr int kHeavyDegLarge = 2 * kHeavyDeg;
+constexpr int kLargeCore = 1 << 18;  // cores from this many vertices on use kHeavyDegLarge
 #ifndef BCGPU_BATCHED_CHUNK
 #define BCGPU_BATCHED_CHUNK 2048
 #endif
@@ -710,7 +716,7 @@ struct RowLane {
     return lane < (int)(len_j >> 16) ? (uint32_t)ldg(a.hcol + rb + at_j + lane) : 0u;
   }
 };
-static_assert(kHeavyDeg < 1 << 16, "a light row's length takes 16 bits");
+static_assert(kHeavyDegLarge < 1 << 16, "a light row's length takes 16 bits");
 
 // Heavy-row chunk tasks of a phase: each CTA's first task is its own index;
 // later ones in a fixed stride (BCGPU_BATCHED_HEAVY_DYN 0) or from the
@@ -1658,7 +1664,7 @@ int batched_build(const bc_bccs *B, const BatchedConfig &cfg, const int64_t *row
     HOST_MARK("b: chains");
     // contracted rows: unit arcs first, then chain arcs
     hvo.push_back((int64_t)hrow.size());
-    const int heavy_deg = npl < kSmallCore ? kHeavyDegSmall : kHeavyDeg;
+    const int heavy_deg = npl < kSmallCore ? kHeavyDegSmall : npl < kLargeCore ? kHeavyDeg : kHeavyDegLarge;
     // Every arc of a core vertex becomes one contracted arc (a unit arc, or
     // the chain arc of the chain vertex it leads to), so the contracted rows
     // have the original degrees: offsets first, then the rows in parallel.
