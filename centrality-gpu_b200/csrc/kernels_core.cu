@@ -51,7 +51,7 @@ namespace {
 
 constexpr int kLight = 8;        // rows up to this many arcs: one thread, kCoreShort arcs in flight
 constexpr int kWarpRow = 1024;   // rows up to this many: a warp; longer: the CTA
-constexpr int kCtaQueue = 64;    // rows of a level the whole CTA takes one by one (a warp each past that)
+constexpr int kCtaQueue = 64;    // queue of the rows of a level the whole CTA takes one by one: the first ones
 
 // A vertex's record in global memory, one 32-byte sector: its key, its path
 // count (then q), its path count once more, its dependency.
@@ -96,7 +96,7 @@ struct Slot {
   int32_t *via;              // chains whose vertices wait for the backward sweep
   uint32_t *bits;            // shared memory: vertices that have their level
   int32_t *order, *ring;     // vertices by level; the buckets past their first entries
-  int32_t *rows;             // long rows of a level past the first ones
+  int32_t *rows;             // long rows of a level past the first ones (queue_row)
   int32_t *lv, *lx;          // level offsets into order; level exponents
   int64_t bcap;
   int32_t scap;              // entries of a bucket in shared memory
@@ -227,15 +227,17 @@ __device__ __forceinline__ void fwd_done(SH &sh, const CoreArgs &a, const Slot &
   if (e - 1023 > a.rescale_exp || e == 0x7ff) atomicMax(&sh.emax[L.m], e);
 }
 
-// Queues a long row of the level.
+// Queues a long row of the level, by its length alone: the CTA and a warp sum a
+// row in different orders, and the order of the queue is not the same twice. The
+// slot's list holds a warp's rows from the front and the CTA's from the back (its
+// end is the start of the ring); together they are no more than the level.
 template <int kBlock>
 __device__ __forceinline__ void queue_row(Shared<kBlock> &sh, const Slot &w, int m, int32_t v, int deg) {
   if (deg > kWarpRow) {
     const int at = atomicAdd(&sh.ncq[m], 1);
-    if (at < kCtaQueue) {
-      sh.cq[at] = v;
-      return;
-    }
+    if (at < kCtaQueue) sh.cq[at] = v;
+    else w.ring[-1 - at] = v;
+    return;
   }
   const int at = atomicAdd(&sh.nwq[m], 1);
   if (at < Shared<kBlock>::kQueue) sh.wq[at] = v;
@@ -244,7 +246,7 @@ __device__ __forceinline__ void queue_row(Shared<kBlock> &sh, const Slot &w, int
 
 // The queued rows of a level, the very long ones by the whole CTA, the others by
 // a warp each: row(v, head, first arc, step) sums arcs, done(v, head, sums)
-// takes the result in one thread. Two sums, in a fixed order.
+// takes the result in one thread. Two sums, in an order that the row's length fixes.
 template <int kBlock, class Row, class Done>
 __device__ __forceinline__ void long_rows(Shared<kBlock> &sh, const Slot &w, const View &g, int nc, int nw, Row row,
                                           Done done) {
@@ -255,7 +257,9 @@ __device__ __forceinline__ void long_rows(Shared<kBlock> &sh, const Slot &w, con
     const bool all = r < nc;
     const int at = all ? r : (r - nc) * kWarps + warp;
     const bool on = all || at < nw;
-    const int32_t v = !on ? 0 : all ? sh.cq[at] : at < Shared<kBlock>::kQueue ? sh.wq[at] : w.rows[at];
+    const int32_t v = !on                                                 ? 0
+                      : at < (all ? kCtaQueue : Shared<kBlock>::kQueue) ? (all ? sh.cq : sh.wq)[at]
+                                                                        : (all ? w.ring[-1 - at] : w.rows[at]);
     const Head h = head_of(g, v);
     double x = 0.0, y = 0.0;
     if (on) row(h, all ? tid : lane, all ? kBlock : 32, x, y);
@@ -357,7 +361,7 @@ __device__ int core_bfs(Shared<kBlock> &sh, const CoreArgs &a, const Slot &w, Vi
       else queue_row(sh, w, m, v, h.deg);
     }
     __syncthreads();
-    const int nw = sh.nwq[m], nc = min(sh.ncq[m], kCtaQueue);
+    const int nw = sh.nwq[m], nc = sh.ncq[m];
     if (nw | nc) {
       long_rows(sh, w, g, nc, nw,
                 [&](const Head &h, int j0, int step, double &x, double &) { x = fwd_arcs(sh, a, w, g, L, h, Arcs{}, j0, step); },
@@ -569,7 +573,7 @@ __device__ void core_sweep(Shared<kBlock> &sh, const CoreArgs &a, const Slot &w,
       bwd_done(a, w, h.reach, v, s, q, in);
     }
     __syncthreads();
-    const int nw = sh.nwq[m], nc = min(sh.ncq[m], kCtaQueue);
+    const int nw = sh.nwq[m], nc = sh.ncq[m];
     if (nw | nc) {
       long_rows(sh, w, g, nc, nw,
                 [&](const Head &h, int j0, int step, double &x, double &y) { bwd_arcs(w, g, h, Arcs{}, j0, step, l, x, y); },
