@@ -78,7 +78,7 @@ struct bc_plan {
   std::vector<int64_t> src_at, core_at, item_at;
   int32_t *tsrc = nullptr;
   bcg::CoreArgs core{};
-  int core_slots = 0, core_block = 256, core_grid = 0;
+  int core_slots = 0, core_block = 256;
   int slots = 0;  // workspace slots of the per-source kernel; slot `slots` is the row export's
   int32_t *ws_i = nullptr, *epochs = nullptr;
   double *ws_f = nullptr;
@@ -525,6 +525,20 @@ bool core_takes(const bc_bccs *B, int32_t b, std::vector<int32_t> &dist, std::ve
   return connected;
 }
 
+// The small-BCC schedule of a plan, laid out before any of it is allocated.
+struct TileLayout {
+  std::vector<bcg::TileItem> items;
+  std::vector<bc_plan::TileLaunch> tl;
+  std::vector<int64_t> off, pairs;  // [n_bcc] slice of each BCC (-1: none) and its pairs of arcs
+  std::vector<int32_t> size;
+  int64_t total = 0, slots = 0, tcap = 2, p_rows = 1, tcap_P = 0;
+  bool listed = false;  // items hold places of a source list
+  int64_t bytes(int64_t n_bcc, int64_t sources) const {
+    return std::max<int64_t>(total, 16) + 12 * n_bcc + (int64_t)sizeof(bcg::TileItem) * (int64_t)items.size() +
+           4 * slots * tcap + (listed ? 4 * sources : 8 * p_rows * std::max<int64_t>(tcap_P, 1));
+  }
+};
+
 // Work items, staged slices and warp workspace of the small-BCC schedule.
 // Launches: the warp class, then the CTA class in buckets by sources in
 // flight per SM (from each BCC's own shared-memory need): 256-thread CTAs at
@@ -534,19 +548,22 @@ bool core_takes(const bc_bccs *B, int32_t b, std::vector<int32_t> &dist, std::ve
 // 1024-thread CTA per SM; CTAs of eight groups, where they fit, which leaves the
 // warp class the BCCs with too many levels for the groups' tables. Each bucket's
 // items are contiguous.
-// With a source list (PLAIN plans: src, each BCC's sources from list[b] on)
-// the items hold places in it, and contributions go straight into the
-// fixed-point counters, so that BC is bit for bit what the per-source kernel
-// gives.
-int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, const std::vector<int32_t> &ecc_of,
-                bc_plan *p, const std::vector<int32_t> *src = nullptr, const std::vector<int64_t> *list = nullptr) {
-  int rc = BCGPU_OK;
-  auto first_of = [&](int32_t b) { return src ? (*list)[(size_t)b] : 0; };
+// With a source list (PLAIN plans: each BCC's sources from list[b] on) the
+// items hold places in it, and contributions go straight into the fixed-point
+// counters.
+int plan_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, const std::vector<int32_t> &ecc_of,
+               const std::vector<int64_t> *list, TileLayout *out) {
+  auto first_of = [&](int32_t b) { return list ? (*list)[(size_t)b] : 0; };
   auto sources_of = [&](int32_t b) {
-    return src ? (*list)[(size_t)b + 1] - (*list)[(size_t)b] : B->vtx_off[b + 1] - B->vtx_off[b];
+    return list ? (*list)[(size_t)b + 1] - (*list)[(size_t)b] : B->vtx_off[b + 1] - B->vtx_off[b];
   };
-  std::vector<int64_t> off((size_t)B->n_bcc, -1);
-  std::vector<int32_t> size((size_t)B->n_bcc, 0);
+  TileLayout &t = *out;
+  t = TileLayout{};
+  t.listed = list != nullptr;
+  t.off.assign((size_t)B->n_bcc, -1);
+  t.size.assign((size_t)B->n_bcc, 0);
+  t.pairs.assign((size_t)B->n_bcc, 0);
+  std::vector<int32_t> &size = t.size;
   std::vector<int8_t> bucket((size_t)B->n_bcc, -1);
   // bucket k -> class: 0 warp, 1 / 2 CTA (4+ / 3 per SM), 3 four groups, 4 CTA-512, 5 two groups, 6 CTA-1024,
   // 7 eight groups of 128, 8 of 64, 9 of 32
@@ -555,12 +572,12 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
                                         bcg::kTileCta512, bcg::kTileCta1024x2, bcg::kTileCta1024, bcg::kTileCta1024x8,
                                         bcg::kTileCta512x8, bcg::kTileCta256x8};
   const int64_t lim = (int64_t)bcg::tile_smem_limit(ctx->device);
-  std::vector<int64_t> per((size_t)B->n_bcc, 0), pairs((size_t)B->n_bcc, 0);
+  std::vector<int64_t> per((size_t)B->n_bcc, 0);
   for (int32_t b = 0; b < B->n_bcc; ++b) {
     if (cls[b] < 0) continue;
     const int64_t nb = B->vtx_off[b + 1] - B->vtx_off[b];
-    pairs[b] = slice_pairs(B, b);
-    size[b] = (int32_t)bcg::TileSlice::bytes(nb, pairs[b]);
+    t.pairs[b] = slice_pairs(B, b);
+    size[b] = (int32_t)bcg::TileSlice::bytes(nb, t.pairs[b]);
     if (cls[b] == bcg::kTileWarp) { bucket[b] = 0; continue; }
     per[b] = bcg::kTileSmPerSm / ((int64_t)bcg::tile_smem_bytes(bcg::kTileCta, nb, size[b]) + bcg::kTileReserved);
     bucket[b] = (int8_t)(per[b] >= 4 ? 1 : per[b] == 3 ? 2 : per[b] == 2 ? 4 : 6);
@@ -601,11 +618,11 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
   promote(7, [&](int32_t b) { return cls[b] != bcg::kTileWarp && per[b] <= 7 && !grouped(b); });
   promote(3, [&](int32_t b) { return cls[b] != bcg::kTileWarp && per[b] <= 3 && !grouped(b); });  // four, not at most three
   promote(5, [&](int32_t b) { return cls[b] != bcg::kTileWarp && per[b] <= 1 && bucket[b] == 6; });  // two instead of one
-  int64_t total = 0, p_rows = 1;
+  int warp_grid = 1;
   for (int k = 0; k < kBuckets; ++k) {
     bc_plan::TileLaunch T;
     T.cls = kBucketCls[k];
-    T.i0 = (int64_t)p->h_titems.size();
+    T.i0 = (int64_t)t.items.size();
     int64_t nmax = 0, smax = 0, sources = 0;
     for (int32_t b = 0; b < B->n_bcc; ++b) {
       if (bucket[b] != k) continue;
@@ -622,31 +639,43 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
     if (per_sm < 1) return fail(ctx, BCGPU_ECUDA, "small-BCC schedule: no CTA fits an SM");
     T.grid = ctx->sms * per_sm;
     const int groups = bcg::tile_groups(T.cls);
-    if (T.cls != bcg::kTileWarp) p_rows = std::max<int64_t>(p_rows, (int64_t)T.grid * groups);
+    if (T.cls == bcg::kTileWarp) {
+      warp_grid = T.grid;
+      t.tcap = std::max<int64_t>(nmax + 2, 2);
+    } else {
+      t.p_rows = std::max<int64_t>(t.p_rows, (int64_t)T.grid * groups);
+      t.tcap_P = std::max(t.tcap_P, nmax);
+    }
     const int32_t per_item = bcg::tile_item_sources(T.cls, T.grid, sources);
     for (int32_t b = 0; b < B->n_bcc; ++b) {
       if (bucket[b] != k) continue;
       const int64_t l0 = first_of(b), l1 = l0 + sources_of(b);
-      off[b] = total;
-      total += size[b];
+      t.off[b] = t.total;
+      t.total += size[b];
       for (int64_t s0 = l0; s0 < l1; s0 += per_item)
-        p->h_titems.push_back({b, (int32_t)s0, (int32_t)std::min<int64_t>(l1, s0 + per_item), 0});
+        t.items.push_back({b, (int32_t)s0, (int32_t)std::min<int64_t>(l1, s0 + per_item), 0});
     }
-    T.i1 = (int64_t)p->h_titems.size();
-    if (T.cls == bcg::kTileWarp) p->tcap = nmax + 2;
-    p->tl.push_back(T);
+    T.i1 = (int64_t)t.items.size();
+    t.tl.push_back(T);
   }
+  t.slots = (int64_t)warp_grid * bcg::kTileWarps;
+  return BCGPU_OK;
+}
+
+// Uploads what plan_tiles laid out (src: the source list of listed items).
+int build_tiles(const bc_bccs *B, TileLayout &t, const std::vector<int32_t> *src, bc_plan *p) {
+  int rc = BCGPU_OK;
   // slices: row offsets in pairs (uint16 when narrow, else int32), neighbours
   // (uint16, a row's spare place the vertex itself), 16-byte aligned parts; bit 0
   // of a narrow slice's offset set
-  std::vector<unsigned char> blob((size_t)std::max<int64_t>(total, 16), 0);
-  std::vector<int64_t> off_flag(off);  // what the kernels read: offset | narrow
+  std::vector<unsigned char> blob((size_t)std::max<int64_t>(t.total, 16), 0);
+  std::vector<int64_t> off_flag(t.off);  // what the kernels read: offset | narrow
 #pragma omp parallel for schedule(dynamic, 16) if (B->n_bcc > 16)
   for (int32_t b = 0; b < B->n_bcc; ++b) {
-    if (off[b] < 0) continue;  // no item
+    if (t.off[b] < 0) continue;  // no item
     const int64_t vo = B->vtx_off[b], nb = B->vtx_off[b + 1] - vo;
-    const bool narrow = bcg::TileSlice::narrow(pairs[b]);
-    unsigned char *base = blob.data() + off[b];
+    const bool narrow = bcg::TileSlice::narrow(t.pairs[b]);
+    unsigned char *base = blob.data() + t.off[b];
     uint16_t *C = reinterpret_cast<uint16_t *>(base + bcg::TileSlice::col_at(nb, narrow));
     int64_t at = 0;
     for (int64_t v = 0; v <= nb; ++v) {
@@ -658,20 +687,17 @@ int build_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, c
     }
     if (narrow) off_flag[b] |= 1;
   }
+  p->h_titems = std::move(t.items);
   p->n_titems = (int64_t)p->h_titems.size();
-  int warp_grid = 1;
-  for (const auto &T : p->tl) {
-    if (T.cls == bcg::kTileWarp) warp_grid = T.grid;
-    else p->tcap_P = std::max<int64_t>(p->tcap_P, T.nmax);
-  }
-  const int64_t slots = (int64_t)warp_grid * bcg::kTileWarps;
-  p->tcap = std::max<int64_t>(p->tcap, 2);
+  p->tl = std::move(t.tl);
+  p->tcap = t.tcap;
+  p->tcap_P = t.tcap_P;
   if ((rc = upload(p, &p->slices, blob.data(), (int64_t)blob.size())) ||
       (rc = upload(p, &p->slice_off, off_flag.data(), B->n_bcc)) ||
-      (rc = upload(p, &p->slice_bytes, size.data(), B->n_bcc)) ||
-      (rc = upload(p, &p->titems, p->h_titems.data(), p->n_titems)) || (rc = dalloc(p, &p->tws_lv, slots * p->tcap)) ||
+      (rc = upload(p, &p->slice_bytes, t.size.data(), B->n_bcc)) ||
+      (rc = upload(p, &p->titems, p->h_titems.data(), p->n_titems)) || (rc = dalloc(p, &p->tws_lv, t.slots * p->tcap)) ||
       (rc = src ? upload(p, &p->tsrc, src->data(), (int64_t)src->size())
-                : dalloc(p, &p->tws_P, p_rows * std::max<int64_t>(p->tcap_P, 1))) ||
+                : dalloc(p, &p->tws_P, t.p_rows * std::max<int64_t>(p->tcap_P, 1))) ||
       (rc = alloc_acc(p, B->n_packed)))
     return rc;
   if (src) return BCGPU_OK;  // the plan's units are its per-source items
@@ -715,7 +741,6 @@ int build_core(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &on, con
   CK(ctx, bcg::core_contract(p->row, p->col, p->vtx_off, n_plain, p->reach, chain_off, p->chain_start, p->chain_len,
                              p->chain_l, p->chain_r, d_on, B->n_bcc, B->n_packed, row_off, rows, xcol, xk, xcid, ctab, vchain,
                              ctx->stream));
-  p->core_slots = (int)std::min<int64_t>(p->core_grid, (int64_t)src.size());
   const int64_t n = p->core_slots, rec = a.shape.rec_bytes();
   std::vector<int32_t> ep((size_t)n, 1);
   if ((rc = dalloc(p, &a.rec, n * rec)) || (rc = dalloc(p, &a.ws, n * a.shape.rest_bytes())) ||
@@ -728,6 +753,226 @@ int build_core(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &on, con
   a.next = p->counter; a.acc = p->acc; a.err = p->err;
   a.rescale_exp = ctx->opts.rescale_exp > 0 ? ctx->opts.rescale_exp : 900;
   return BCGPU_OK;
+}
+
+// The per-source items of a plan, laid out before any of it is allocated: the
+// kernel each BCC's items run on, the kernels' lists, and what they take.
+struct SourceLayout {
+  bool plain = false;             // PLAIN plan: a row-export slot is allocated whatever runs
+  bool listed = false;            // the sources fit a source list
+  std::vector<int8_t> small;      // [n_bcc] small-BCC class, -1: not on the small-BCC kernels
+  std::vector<int32_t> small_ecc;
+  std::vector<int8_t> core;       // [n_bcc] on the contracted kernel
+  std::vector<int32_t> src;       // the small-BCC kernels' source list, BCC b's from list[b] on
+  std::vector<int64_t> list;
+  std::vector<bcg::CoreSource> csrc;   // the contracted kernel's
+  std::vector<bcg::PlainItem> rest;    // the whole-BCC kernel's items
+  std::vector<int64_t> src_at, core_at, item_at;  // what lies before each item in each list
+  TileLayout tiles;
+  bcg::CoreArgs::CoreShape shape{};
+  int64_t ncore = 0;              // core vertices of the BCCs on the contracted kernel
+  int core_block = 256, core_grid = 0;  // its CTAs; as many as fit the device
+  int64_t ws_n = 0;               // rows' capacity in the whole-BCC kernel
+  int64_t slot() const { return row_bytes() + 2 * (int64_t)sizeof(int32_t); }  // rows and two epochs
+  int64_t row_bytes() const { return ws_n * (bcg::kWsIntRows * 4 + bcg::kWsDblRows * 8); }
+  int64_t core_slot() const { return shape.rec_bytes() + shape.rest_bytes() + (int64_t)sizeof(int32_t); }
+  int64_t core_tables(const bc_bccs *B) const {  // as build_core allocates them
+    return 21 * (int64_t)B->n_bcc + 8 + (int64_t)sizeof(bcg::CoreSource) * (int64_t)csrc.size() +
+           (int64_t)sizeof(bcg::CoreRow) * ncore + 12 * B->n_arcs + 16 * B->n_chains + 4 * B->n_packed;
+  }
+};
+
+// The source lists by what small and core say.
+void split_sources(const bc_bccs *B, const std::vector<bcg::PlainItem> &items, SourceLayout &L) {
+  L.src.clear();
+  L.csrc.clear();
+  L.rest.clear();
+  L.src_at.clear();
+  L.core_at.clear();
+  L.item_at.clear();
+  L.list.assign((size_t)B->n_bcc + 1, 0);
+  L.ncore = 0;
+  for (int32_t b = 0; b < B->n_bcc; ++b)
+    if (L.core[(size_t)b]) L.ncore += B->n_plain[b];
+  auto mark = [&] {
+    L.src_at.push_back((int64_t)L.src.size());
+    L.core_at.push_back((int64_t)L.csrc.size());
+    L.item_at.push_back((int64_t)L.rest.size());
+  };
+  for (const auto &it : items) {
+    mark();
+    const bool t = L.small[(size_t)it.bcc] >= 0;
+    if (!t && !L.core[(size_t)it.bcc]) {
+      L.rest.push_back(it);
+      continue;
+    }
+    auto add = [&](int32_t s) {
+      if (t) L.src.push_back(s);
+      else L.csrc.push_back({it.bcc, s});
+    };
+    if (it.own) add(it.src);
+    for (int32_t c = it.c0; c < it.c1; ++c)
+      for (int32_t k = 0; k < B->chain_len[c]; ++k) add(B->chain_start[c] + k);
+    if (t) L.list[(size_t)it.bcc + 1] = (int64_t)L.src.size();
+  }
+  mark();
+  for (int32_t b = 0; b < B->n_bcc; ++b) L.list[(size_t)b + 1] = std::max(L.list[(size_t)b + 1], L.list[(size_t)b]);
+}
+
+// The BCCs of the items on the contracted kernel: those it takes, if its slot is
+// no larger than the whole-BCC kernel's (long chains in a BCC of few chain
+// vertices are not worth their buckets).
+// Its CTAs: as wide as its levels are (core vertices over the depth seen
+// from local vertex 0, and half as much again), between 64 and 512 threads,
+// as many as fit. Narrow levels leave a wide CTA's warps idle, and wide
+// ones make more sources in flight miss L2 more often: kernel ms for 64 /
+// 128 / 256 / 512 threads, 80x80 grid (width 37) 14.9 / 17.1 / 24.3 / -,
+// 512x512 grid (241) 320 / 171 / 143 / 123, R-MAT 14 (1,009) 135 / 114 / 107
+// / 91. plain_ctas_per_sm 4, 8 or 16 asks for 256, 128 or 64 threads.
+void route_core(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> &items,
+                const std::vector<int32_t> &ecc0, const std::vector<char> &conn0, SourceLayout &L) {
+  L.core.assign((size_t)B->n_bcc, 0);
+  L.shape = {4, 2, 0, 2, 3};
+  int levels = 1;  // the deepest core's
+  if (L.listed) {
+    std::vector<int32_t> dist, queue;
+    std::vector<char> seen((size_t)B->n_bcc, 0);
+    for (const auto &it : items) {
+      const int32_t b = it.bcc;
+      if (seen[(size_t)b] || L.small[(size_t)b] >= 0) continue;
+      seen[(size_t)b] = 1;
+      int32_t ecc = ecc0.empty() ? -1 : ecc0[(size_t)b];
+      if (!core_takes(B, b, dist, queue, &ecc, !conn0.empty() && conn0[(size_t)b])) continue;
+      int kmax = 0;
+      for (int64_t c = B->chain_off[b]; c < B->chain_off[b + 1]; ++c) kmax = std::max(kmax, B->chain_len[c]);
+      bcg::CoreArgs::CoreShape h = L.shape;
+      h.cap = std::max<int64_t>(h.cap, (B->n_plain[b] + 3) / 4 * 4);  // 16-byte parts of shared memory
+      h.bcap = std::max<int64_t>(h.bcap, 2 * (B->chain_off[b + 1] - B->chain_off[b]) + 2);
+      h.ccap = std::max(h.ccap, B->chain_off[b + 1] - B->chain_off[b]);
+      h.tcap = std::max(h.tcap, 2 * ecc + kmax + 3);
+      h.ring = std::max(h.ring, kmax + 3);
+      if (h.rec_bytes() + h.rest_bytes() > std::max<int64_t>(L.row_bytes(), 1 << 16) || h.smem_bytes() > kCoreBits) continue;
+      levels = std::max(levels, ecc);
+      L.shape = h;
+      L.core[(size_t)b] = 1;
+    }
+  }
+  if (ctx->opts.plain_ctas_per_sm) {
+    L.core_block = 1024 / ctx->opts.plain_ctas_per_sm;
+  } else {
+    L.core_block = 64;
+    while (L.core_block < 512 && 2 * L.core_block * (int64_t)levels < 3 * L.shape.cap) L.core_block *= 2;
+  }
+  L.core_grid = ctx->sms * bcg::core_ctas_per_sm(L.core_block, L.shape);
+  if (L.core_grid < 1) std::fill(L.core.begin(), L.core.end(), 0);
+}
+
+// Slots of the two per-source kernels that keep their rows in global memory.
+struct SourceSlots {
+  int grid = 0, block = 1024;  // whole-BCC kernel: CTAs were all items its own (less by memory only), and their threads
+  int64_t whole = 0, core = 0;  // slots of each; the row-export slot is not among them
+};
+
+// What fits `room` bytes, tables and the row-export slot included, at least one
+// whole-BCC slot where that kernel has items. Four 256-thread CTAs per SM (four
+// sources in flight) when their rows fit, else two of 512, else one of 1024 per
+// SM; with plain_ctas_per_sm 8 or 16, CTAs of 128 or 64 threads are tried first.
+// Of two kernels that cannot both have what they would, each gets half.
+SourceSlots fit_slots(const bc_ctx *ctx, const bc_bccs *B, const SourceLayout &L, int64_t room) {
+  SourceSlots r;
+  room -= (int64_t)sizeof(bcg::PlainItem) * std::max<int64_t>((int64_t)L.rest.size(), 1);
+  if (!L.src.empty()) room -= L.tiles.bytes(B->n_bcc, (int64_t)L.src.size());
+  if (L.plain || !L.rest.empty()) room -= L.slot();
+  const int64_t core_want = std::min<int64_t>(L.core_grid, (int64_t)L.csrc.size());
+  int64_t whole_room = room;
+  if (core_want) {
+    room -= L.core_tables(B);
+    const int64_t most = (int64_t)ctx->sms * std::max(4, ctx->opts.plain_ctas_per_sm);
+    const int64_t whole_want = std::min<int64_t>(most, (int64_t)L.rest.size()) * L.slot();
+    const int64_t half = std::max(room / 2, room - core_want * L.core_slot());
+    const int64_t shared = std::min(whole_want, std::max(half, L.rest.empty() ? 0 : L.slot()));
+    r.core = std::max<int64_t>(0, std::min(core_want, (room - shared) / L.core_slot()));
+    whole_room = L.rest.empty() ? whole_room : room - r.core * L.core_slot();
+  }
+  const int first = ctx->opts.plain_ctas_per_sm > 4 ? 1024 / ctx->opts.plain_ctas_per_sm : 256;
+  for (int block : {64, 128, 256, 512, 1024}) {
+    if (block < first) continue;
+    const int want = ctx->sms * (1024 / block);
+    r.grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, whole_room / L.slot()));
+    r.block = block;
+    if (r.grid == want) break;
+  }
+  r.whole = std::min<int64_t>(r.grid, (int64_t)L.rest.size());  // items take a slot each
+  return r;
+}
+
+// Device bytes of the items with these slots (the counters not among them).
+int64_t source_bytes(const bc_bccs *B, const SourceLayout &L, const SourceSlots &r) {
+  return (int64_t)sizeof(bcg::PlainItem) * std::max<int64_t>((int64_t)L.rest.size(), 1) +
+         (L.src.empty() ? 0 : L.tiles.bytes(B->n_bcc, (int64_t)L.src.size())) +
+         (r.core ? L.core_tables(B) + r.core * L.core_slot() : 0) + (r.whole || L.plain ? (r.whole + 1) * L.slot() : 0);
+}
+
+// Lays out the items (see SourceLayout); which kernel takes which BCC is settled
+// up to what fits the device memory (settle_sources).
+int lay_out_sources(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> &items, bool plain,
+                    const std::vector<int32_t> &ecc0, const std::vector<char> &conn0, SourceLayout &L) {
+  L.plain = plain;
+  int64_t nb_max = 0, nb_items = 0, sources = 0;
+  for (int32_t b = 0; b < B->n_bcc; ++b) nb_max = std::max(nb_max, B->vtx_off[b + 1] - B->vtx_off[b]);
+  for (const auto &it : items) {
+    nb_items = std::max(nb_items, B->vtx_off[it.bcc + 1] - B->vtx_off[it.bcc]);
+    sources += it.own ? 1 : 0;
+    for (int32_t c = it.c0; c < it.c1; ++c) sources += B->chain_len[c];
+  }
+  L.ws_n = (plain ? nb_max : nb_items) + 2;
+  L.listed = !items.empty() && sources < INT32_MAX;
+  // PLAIN: items of the BCCs that fit shared memory go to the small-BCC
+  // kernels (sources of an item: its own vertex, then its chains'). Their path
+  // counts stay below 2^1000 and need no rescaling, whatever the threshold.
+  // Rows in shared memory instead of L2, and a BFS per chain vertex instead of
+  // a merge and a double listing: a chain-endpoint call on a BCC of 1,494
+  // vertices went from 1.95 to 0.66 ms, 1,194 sources.
+  L.small.assign((size_t)B->n_bcc, -1);
+  if (plain && L.listed) route_tiles(ctx, B, std::vector<char>((size_t)B->n_bcc, 0), L.small, L.small_ecc, true);
+  route_core(ctx, B, items, ecc0, conn0, L);
+  split_sources(B, items, L);
+  return L.src.empty() ? BCGPU_OK : plan_tiles(ctx, B, L.small, L.small_ecc, &L.list, &L.tiles);
+}
+
+// Takes back what does not fit `room` bytes, for the whole-BCC kernel, which fits
+// any plan that is accepted: the small-BCC kernels, if their slices leave no room
+// for the slots the others need; the contracted kernel, if its tables leave it
+// less than half the sources in flight that the whole-BCC kernel would have (it
+// takes a source in 0.35 to 0.5 of the time, both with all their CTAs resident:
+// the figures in kernels_core.cu).
+SourceSlots settle_sources(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> &items,
+                           const std::vector<int32_t> &ecc0, const std::vector<char> &conn0, int64_t room,
+                           SourceLayout &L) {
+  const int64_t others = L.csrc.empty() && L.rest.empty() ? 0 : L.slot();
+  if (!L.src.empty() && source_bytes(B, L, SourceSlots{}) + others > room) {
+    std::fill(L.small.begin(), L.small.end(), -1);
+    route_core(ctx, B, items, ecc0, conn0, L);
+    split_sources(B, items, L);
+  }
+  SourceSlots r = fit_slots(ctx, B, L, room);
+  if (!L.csrc.empty() && r.core < std::min<int64_t>(L.core_grid, (int64_t)L.csrc.size())) {
+    SourceLayout alone = L;
+    std::fill(alone.core.begin(), alone.core.end(), 0);
+    split_sources(B, items, alone);
+    const SourceSlots w = fit_slots(ctx, B, alone, room);
+    if (2 * r.core < w.whole || source_bytes(B, L, r) > room) {
+      L = std::move(alone);
+      r = w;
+    }
+  }
+  if (source_bytes(B, L, r) > room && L.rest.size() < items.size()) {  // slices, lists and one slot do not fit
+    std::fill(L.small.begin(), L.small.end(), -1);
+    std::fill(L.core.begin(), L.core.end(), 0);
+    split_sources(B, items, L);
+    r = fit_slots(ctx, B, L, room);
+  }
+  return r;
 }
 
 // Source orders of the BCCs in multi-source passes, computed on one host
@@ -792,9 +1037,6 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
   p->h_n_plain.assign(B->n_plain, B->n_plain + B->n_bcc);
   p->h_chain_start.assign(B->chain_start, B->chain_start + B->n_chains);
   p->h_chain_len.assign(B->chain_len, B->chain_len + B->n_chains);
-  int64_t nb_max = 0;
-  for (int32_t b = 0; b < B->n_bcc; ++b) nb_max = std::max(nb_max, B->vtx_off[b + 1] - B->vtx_off[b]);
-
   // BATCHED: which BCCs take multi-source passes (the others: per-source items)
   std::vector<char> on;
   std::vector<int32_t> ecc0;  // eccentricity of each BCC's local vertex 0, -1 unknown (the batched plan reuses it)
@@ -878,6 +1120,12 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
     for (int32_t b = 0; b < B->n_bcc; ++b) skip[b] |= n_tile ? tile[b] >= 0 : 0;
     plain_items(B, items, &skip);
   }
+  const bool sources = !items.empty() || p->mode == BCGPU_MODE_PLAIN;
+  SourceLayout L;
+  TileLayout tiles;
+  if (sources && (rc = lay_out_sources(ctx, B, items, p->mode == BCGPU_MODE_PLAIN, ecc0, conn0, L))) return bail(rc);
+  if (n_tile && (rc = plan_tiles(ctx, B, tile, tile_ecc, nullptr, &tiles))) return bail(rc);
+  HOST_MARK("lay out sources");
   if (p->mode == BCGPU_MODE_BATCHED && n_on > 0) {
     if ((rc = free_limit())) return bail(rc);
     bcg::BatchedConfig cfg;
@@ -909,9 +1157,8 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
     p->unit_aux.assign(1, 0);
     p->unit_visits.assign(1, 0);
   }
-  if (!items.empty() || p->mode == BCGPU_MODE_PLAIN) {
+  if (sources) {
     p->n_items = (int64_t)items.size();
-    int64_t nb_plain = 0;
     for (size_t i = 0; i < items.size(); ++i) {
       const auto &it = items[i];
       int64_t src = it.own ? 1 : 0, aux = it.own ? 0 : 1;
@@ -921,7 +1168,6 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
         if (B->chain_r[c] != prev) { ++aux; prev = B->chain_r[c]; }
       }
       const int64_t nb = B->vtx_off[it.bcc + 1] - B->vtx_off[it.bcc];
-      nb_plain = std::max(nb_plain, nb);
       const int64_t arcs = B->row[B->vtx_off[it.bcc + 1]] - B->row[B->vtx_off[it.bcc]];
       p->unit_sources.push_back(p->unit_sources.back() + src);
       p->unit_teps.push_back(p->unit_teps.back() + src * arcs);
@@ -929,131 +1175,46 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
       p->unit_aux.push_back(p->unit_aux.back() + aux);
       p->unit_visits.push_back(p->unit_visits.back() + src * nb);
     }
-    // PLAIN: items of the BCCs that fit shared memory go to the small-BCC
-    // kernels (sources of an item: its own vertex, then its chains'). Their path
-    // counts stay below 2^1000 and need no rescaling, whatever the threshold.
-    // Rows in shared memory instead of L2, and a BFS per chain vertex instead of
-    // a merge and a double listing: a chain-endpoint call on a BCC of 1,494
-    // vertices went from 1.95 to 0.66 ms, 1,194 sources.
-    const bool listed = p->unit_sources.back() - p->unit_sources[(size_t)p->n_bat] < INT32_MAX;
-    std::vector<int8_t> small((size_t)B->n_bcc, -1), core((size_t)B->n_bcc, 0);
-    std::vector<int32_t> small_ecc;
-    if (p->mode == BCGPU_MODE_PLAIN && p->n_items > 0 && listed)
-      route_tiles(ctx, B, std::vector<char>((size_t)B->n_bcc, 0), small, small_ecc, true);
-    p->ws_n = (p->mode == BCGPU_MODE_PLAIN ? nb_max : nb_plain) + 2;
-    const int64_t per_slot = p->ws_n * (bcg::kWsIntRows * 4 + bcg::kWsDblRows * 8);
-    // Four 256-thread CTAs per SM (four sources in flight) when their rows
-    // fit the budget, else two of 512, else one of 1024 per SM; with
-    // plain_ctas_per_sm 8 or 16, CTAs of 128 or 64 threads are tried first.
-    // Where every item is a small BCC's, the slot of the row export is all there
-    // is to hold: a few of those are allocated without asking what is free.
-    const bool all_small = p->mode == BCGPU_MODE_PLAIN &&
-                           std::none_of(items.begin(), items.end(), [&](const auto &it) { return small[it.bcc] < 0; });
-    if (!all_small || 2 * per_slot > kUnasked) {
+    p->ws_n = L.ws_n;
+    // Where every item is a small BCC's, the slices and the slot of the row export
+    // are all there is to hold: a little of that is allocated without asking.
+    const bool all_small = L.csrc.empty() && L.rest.empty();
+    if (!all_small || source_bytes(B, L, SourceSlots{}) + L.slot() > kUnasked) {
       if ((rc = free_limit())) return bail(rc);
     } else if (limit <= 0) {
-      limit = INT64_MAX;
+      limit = INT64_MAX / 2;
     }
-    const int64_t avail = limit - p->device_bytes - 64 * (int64_t)ctx->sms;
-    if (avail < 2 * per_slot) return bail(fail(ctx, BCGPU_ENOMEM, "workspace for the largest BCC exceeds the limit"));
-    int grid = 0;
-    const int first = ctx->opts.plain_ctas_per_sm > 4 ? 1024 / ctx->opts.plain_ctas_per_sm : 256;
-    for (int block : {64, 128, 256, 512, 1024}) {
-      if (block < first) continue;
-      const int want = ctx->sms * (1024 / block);
-      grid = (int)std::min<int64_t>(want, avail / per_slot - 1);
-      p->block = block;
-      if (grid == want) break;
-    }
-    p->grid = std::max(1, grid);
-    // the others: the contracted kernel, if its slot is no larger than the
-    // whole-BCC kernel's (long chains in a BCC of few chain vertices are not
-    // worth their buckets)
-    bcg::CoreArgs::CoreShape &shape = p->core.shape;
-    shape = {4, 2, 0, 2, 3};
-    int levels = 1;  // the deepest core's
-    if (listed && p->n_items > 0) {
-      std::vector<int32_t> dist, queue;
-      std::vector<char> seen((size_t)B->n_bcc, 0);
-      for (const auto &it : items) {
-        const int32_t b = it.bcc;
-        if (seen[b] || small[b] >= 0) continue;
-        seen[b] = 1;
-        int32_t ecc = ecc0.empty() ? -1 : ecc0[b];
-        if (!core_takes(B, b, dist, queue, &ecc, !conn0.empty() && conn0[b])) continue;
-        int kmax = 0;
-        for (int64_t c = B->chain_off[b]; c < B->chain_off[b + 1]; ++c) kmax = std::max(kmax, B->chain_len[c]);
-        bcg::CoreArgs::CoreShape h = shape;
-        levels = std::max(levels, ecc);
-        h.cap = std::max<int64_t>(h.cap, (B->n_plain[b] + 3) / 4 * 4);  // 16-byte parts of shared memory
-        h.bcap = std::max<int64_t>(h.bcap, 2 * (B->chain_off[b + 1] - B->chain_off[b]) + 2);
-        h.ccap = std::max(h.ccap, B->chain_off[b + 1] - B->chain_off[b]);
-        h.tcap = std::max(h.tcap, 2 * ecc + kmax + 3);
-        h.ring = std::max(h.ring, kmax + 3);
-        if (h.rec_bytes() + h.rest_bytes() > std::max<int64_t>(per_slot, 1 << 16) ||
-            h.smem_bytes() > kCoreBits)
-          continue;
-        shape = h;
-        core[b] = 1;
-      }
-    }
-    // Its CTAs: as wide as its levels are (core vertices over the depth seen
-    // from local vertex 0, and half as much again), between 64 and 512 threads,
-    // as many as fit. Narrow levels leave a wide CTA's warps idle, and wide
-    // ones make more sources in flight miss L2 more often: kernel ms for 64 /
-    // 128 / 256 / 512 threads, 80x80 grid (width 37) 14.9 / 17.1 / 24.3 / -,
-    // 512x512 grid (241) 320 / 171 / 143 / 123, R-MAT 14 (1,009) 135 / 114 / 107
-    // / 91. plain_ctas_per_sm 4, 8 or 16 asks for 256, 128 or 64 threads.
-    if (ctx->opts.plain_ctas_per_sm) {
-      p->core_block = 1024 / ctx->opts.plain_ctas_per_sm;
-    } else {
-      p->core_block = 64;
-      while (p->core_block < 512 && 2 * p->core_block * (int64_t)levels < 3 * shape.cap) p->core_block *= 2;
-    }
-    p->core_grid = (int)std::min<int64_t>((int64_t)ctx->sms * bcg::core_ctas_per_sm(p->core_block, shape),
-                                          avail / (shape.rec_bytes() + shape.rest_bytes()));
-    if (p->core_grid < 1) std::fill(core.begin(), core.end(), 0);
-    std::vector<int32_t> src;
-    std::vector<bcg::CoreSource> csrc;
-    std::vector<int64_t> list((size_t)B->n_bcc + 1, 0);
-    std::vector<bcg::PlainItem> rest;
-    for (const auto &it : items) {
-      p->src_at.push_back((int64_t)src.size());
-      p->core_at.push_back((int64_t)csrc.size());
-      p->item_at.push_back((int64_t)rest.size());
-      const bool t = small[it.bcc] >= 0;
-      if (!t && !core[it.bcc]) {
-        rest.push_back(it);
-        continue;
-      }
-      auto add = [&](int32_t s) {
-        if (t) src.push_back(s);
-        else csrc.push_back({it.bcc, s});
-      };
-      if (it.own) add(it.src);
-      for (int32_t c = it.c0; c < it.c1; ++c)
-        for (int32_t k = 0; k < B->chain_len[c]; ++k) add(B->chain_start[c] + k);
-      if (t) list[(size_t)it.bcc + 1] = (int64_t)src.size();
-    }
-    p->src_at.push_back((int64_t)src.size());
-    p->core_at.push_back((int64_t)csrc.size());
-    p->item_at.push_back((int64_t)rest.size());
-    for (int32_t b = 0; b < B->n_bcc; ++b) list[(size_t)b + 1] = std::max(list[(size_t)b + 1], list[(size_t)b]);
-    if (!src.empty() && (rc = build_tiles(ctx, B, small, small_ecc, p, &src, &list))) return bail(rc);
-    p->h_items = std::move(items);
-    if ((rc = upload(p, &p->items, rest.data(), (int64_t)rest.size()))) return bail(rc);
     if ((rc = alloc_acc(p, B->n_packed))) return bail(rc);
-    if (!csrc.empty() && (rc = build_core(ctx, B, core, csrc, p))) return bail(rc);
-    p->slots = (int)std::min<int64_t>(p->grid, (int64_t)rest.size());  // items take a slot each
+    // Two slots of rows beside all the items, on the whole-BCC kernel, are the least
+    // that a plan is accepted with; what runs elsewhere has to fit the same limit.
+    int64_t room = limit - p->device_bytes;
+    if (room - (int64_t)sizeof(bcg::PlainItem) * std::max<int64_t>(p->n_items, 1) - 64 * (int64_t)ctx->sms <
+        2 * L.row_bytes())
+      return bail(fail(ctx, BCGPU_ENOMEM, "workspace for the largest BCC exceeds the limit"));
+    if (n_tile) room = std::max(room - tiles.bytes(B->n_bcc, 0), 2 * L.slot() + (int64_t)sizeof(bcg::PlainItem) * p->n_items);
+    const SourceSlots slots = settle_sources(ctx, B, items, ecc0, conn0, room, L);
+    p->grid = slots.grid;
+    p->block = slots.block;
+    p->slots = (int)slots.whole;
+    p->core_slots = (int)slots.core;
+    p->core_block = L.core_block;
+    p->core.shape = L.shape;
+    p->src_at = std::move(L.src_at);
+    p->core_at = std::move(L.core_at);
+    p->item_at = std::move(L.item_at);
+    p->h_items = std::move(items);
+    if (!L.src.empty() && (rc = build_tiles(B, L.tiles, &L.src, p))) return bail(rc);
+    if ((rc = upload(p, &p->items, L.rest.data(), (int64_t)L.rest.size()))) return bail(rc);
+    if (!L.csrc.empty() && (rc = build_core(ctx, B, L.core, L.csrc, p))) return bail(rc);
     if (p->slots || p->mode == BCGPU_MODE_PLAIN) {
-      const int64_t slots = p->slots + 1;  // + the row-export slot
-      if ((rc = dalloc(p, &p->ws_i, slots * bcg::kWsIntRows * p->ws_n)) ||
-          (rc = dalloc(p, &p->ws_f, slots * bcg::kWsDblRows * p->ws_n)) || (rc = dalloc(p, &p->epochs, 2 * slots)))
+      const int64_t n = p->slots + 1;  // + the row-export slot
+      if ((rc = dalloc(p, &p->ws_i, n * bcg::kWsIntRows * p->ws_n)) ||
+          (rc = dalloc(p, &p->ws_f, n * bcg::kWsDblRows * p->ws_n)) || (rc = dalloc(p, &p->epochs, 2 * n)))
         return bail(rc);
-      if (cudaMemsetAsync(p->ws_f, 0, sizeof(double) * (size_t)(slots * bcg::kWsDblRows * p->ws_n), ctx->stream) !=
+      if (cudaMemsetAsync(p->ws_f, 0, sizeof(double) * (size_t)(n * bcg::kWsDblRows * p->ws_n), ctx->stream) !=
           cudaSuccess)  // row records: stamp 0, unvisited
         return bail(cuda_fail(ctx, cudaGetLastError(), "cudaMemsetAsync"));
-      std::vector<int32_t> ep((size_t)(2 * slots), 1);
+      std::vector<int32_t> ep((size_t)(2 * n), 1);
       CK(ctx, cudaMemcpyAsync(p->epochs, ep.data(), sizeof(int32_t) * ep.size(), cudaMemcpyHostToDevice, ctx->stream));
       p->h2d_bytes += (int64_t)(sizeof(int32_t) * ep.size());
     }
@@ -1061,7 +1222,7 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
     CK(ctx, cudaStreamSynchronize(ctx->stream));
   }
   HOST_MARK("plain items+ws");
-  if (n_tile && (rc = build_tiles(ctx, B, tile, tile_ecc, p))) return bail(rc);
+  if (n_tile && (rc = build_tiles(B, tiles, nullptr, p))) return bail(rc);
   CK(ctx, cudaStreamSynchronize(ctx->stream));
   HOST_MARK("tiles+sync");
   return BCGPU_OK;
