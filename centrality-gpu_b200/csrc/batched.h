@@ -16,6 +16,7 @@ struct BatchedConfig {
   bool delta_fp32c = true;  // FP32 two-sum compensated dependencies (else FP64)
   int sms = 148;
   int64_t limit_bytes = 0;  // device bytes available to the plan's workspace
+  int64_t merge_bytes = 0;  // device bytes it may take, tables included, to run several passes as one
   int rescale_exp = 900;    // rescale a level's path counts above 2^rescale_exp
   unsigned long long wait_ns = 60ull * 1000 * 1000 * 1000;  // limit of one device-side wait
   cudaMemPool_t pool = nullptr;  // device memory from this pool, ordered on the plan's stream (null: cudaMalloc)

@@ -1133,6 +1133,10 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
     cfg.delta_fp32c = ctx->opts.delta == BCGPU_DELTA_FP32C;
     cfg.sms = ctx->sms;
     cfg.limit_bytes = limit - p->device_bytes;
+    // running passes together is for what the other schedules leave: all they would hold
+    cfg.merge_bytes = cfg.limit_bytes - (n_tile ? tiles.bytes(B->n_bcc, 0) : 0);
+    if (sources || n_tile) cfg.merge_bytes -= (int64_t)acc_bytes(B->n_packed);
+    if (sources) cfg.merge_bytes -= source_bytes(B, L, fit_slots(ctx, B, L, INT64_MAX / 2)) + 64 * (int64_t)ctx->sms;
     cfg.rescale_exp = ctx->opts.rescale_exp;
     cfg.wait_ns = wait_ns(ctx);
     cfg.pool = ctx->pool;

@@ -1802,15 +1802,14 @@ int batched_build(const bc_bccs *B, const BatchedConfig &cfg, const int64_t *row
            w * 32 * (tcap + 2) * 4 + nch * w * 32 * 8;
   };
   const int64_t need = need_of(W);
+  auto workspace_of = [&](int64_t w) {  // every byte of it, as allocated below
+    return n * (w * 32 * (4 + 8 + qb + 8) + (int64_t)(tcap + 2) * w * 4 + w * 4 + 8 + w * 8) + (4 * ((int64_t)tcap + 3) + 2) * 4 +
+           w * 32 * (8 + 4 + ((int64_t)tcap + 2) * 4 + 4) + (int64_t)sizeof(Ctrl) +
+           std::max<int64_t>(P->n_batches, 1) * 4 + std::max<int64_t>(nch, 1) * w * (32 * 8 + 4);
+  };
   if (need > cfg.limit_bytes)
     return bail(BCGPU_ENOMEM, "batched workspace " + std::to_string(need >> 20) + " MiB exceeds the limit " +
                                   std::to_string(cfg.limit_bytes >> 20) + " MiB (lower the batch width)");
-  // passes run as one: as many as the rule allows, the plan will run and the
-  // workspace fits; a pass has to end on a whole group of words
-  const int64_t filled = std::min(P->n_batches, cfg.fill_end) - std::max<int64_t>(0, cfg.fill_begin);
-  P->merge = W * 32 == width ? (int)std::max<int64_t>(1, std::min<int64_t>(merge_passes(n, width), filled)) : 1;
-  while (P->merge > 1 && need_of((int64_t)P->merge * W) > cfg.limit_bytes) --P->merge;
-  const int64_t WA = (int64_t)P->merge * W;  // words a row is allocated
   P->pool = cfg.pool;
   P->stream = stream;
   auto alloc = [&](void **p, int64_t bytes) -> bool {
@@ -1829,23 +1828,6 @@ int batched_build(const bc_bccs *B, const BatchedConfig &cfg, const int64_t *row
   Args &a = P->args;
   void *p = nullptr;
   bool ok = true;
-  ok &= alloc(&p, n * WA * 32 * 4); a.d = (int32_t *)p;
-  ok &= ok && alloc(&p, n * WA * 32 * 8); a.sig = (double *)p;
-  ok &= ok && alloc(&p, n * WA * 32 * qb); a.q = p;
-  ok &= ok && alloc(&p, (int64_t)(tcap + 2) * n * WA * 4); a.lm = (uint32_t *)p;
-  ok &= ok && alloc(&p, n * WA * 4); a.seen = (uint32_t *)p;
-  ok &= ok && alloc(&p, n * 4); a.lmin = (int32_t *)p;
-  ok &= ok && alloc(&p, n * 4); a.armed = (int32_t *)p;
-  ok &= ok && alloc(&p, (4 * ((int64_t)tcap + 3) + 2) * 4); a.wq = (int *)p;
-  ok &= ok && alloc(&p, n * WA * 8); a.bcpart = (double *)p;
-  ok &= ok && alloc(&p, n * WA * 32 * 8); a.cdep = (double *)p;
-  ok &= ok && alloc(&p, WA * 32 * 8); a.wsrc = (double *)p;
-  ok &= ok && alloc(&p, WA * 32 * 4); a.schain = (int32_t *)p;
-  ok &= ok && alloc(&p, WA * 32 * (tcap + 2) * 4); a.X = (int32_t *)p;
-  ok &= ok && alloc(&p, WA * 32 * 4); a.rexp = (int32_t *)p;
-  ok &= ok && alloc(&p, sizeof(Ctrl)); a.ctrl = (Ctrl *)p;
-  ok &= ok && alloc(&p, (int64_t)std::max<int64_t>(P->n_batches, 1) * 4); a.redo = (int *)p;
-  HOST_MARK("b: ws alloc");
   // tables
   auto upload = [&](const void **dst, const void *src, int64_t bytes) -> bool {
     if (!alloc(&p, bytes)) return false;
@@ -1907,8 +1889,32 @@ int batched_build(const bc_bccs *B, const BatchedConfig &cfg, const int64_t *row
   }
   ok = ok && upload((const void **)&a.seeds, seeds.data(), (int64_t)seeds.size() * (int64_t)sizeof(Seed));
   ok = ok && upload((const void **)&a.arms, arms.data(), (int64_t)arms.size() * (int64_t)sizeof(int2));
+  // Passes run as one: as many as the rule allows, the plan will run and, with the
+  // tables above, fit what the rest of the plan leaves; a pass has to end on a
+  // whole group of words.
+  const int64_t filled = std::min(P->n_batches, cfg.fill_end) - std::max<int64_t>(0, cfg.fill_begin);
+  P->merge = W * 32 == width ? (int)std::max<int64_t>(1, std::min<int64_t>(merge_passes(n, width), filled)) : 1;
+  while (P->merge > 1 && P->bytes + workspace_of((int64_t)P->merge * W) > cfg.merge_bytes) --P->merge;
+  const int64_t WA = (int64_t)P->merge * W;  // words a row is allocated
+  ok &= ok && alloc(&p, n * WA * 32 * 4); a.d = (int32_t *)p;
+  ok &= ok && alloc(&p, n * WA * 32 * 8); a.sig = (double *)p;
+  ok &= ok && alloc(&p, n * WA * 32 * qb); a.q = p;
+  ok &= ok && alloc(&p, (int64_t)(tcap + 2) * n * WA * 4); a.lm = (uint32_t *)p;
+  ok &= ok && alloc(&p, n * WA * 4); a.seen = (uint32_t *)p;
+  ok &= ok && alloc(&p, n * 4); a.lmin = (int32_t *)p;
+  ok &= ok && alloc(&p, n * 4); a.armed = (int32_t *)p;
+  ok &= ok && alloc(&p, (4 * ((int64_t)tcap + 3) + 2) * 4); a.wq = (int *)p;
+  ok &= ok && alloc(&p, n * WA * 8); a.bcpart = (double *)p;
+  ok &= ok && alloc(&p, n * WA * 32 * 8); a.cdep = (double *)p;
+  ok &= ok && alloc(&p, WA * 32 * 8); a.wsrc = (double *)p;
+  ok &= ok && alloc(&p, WA * 32 * 4); a.schain = (int32_t *)p;
+  ok &= ok && alloc(&p, WA * 32 * (tcap + 2) * 4); a.X = (int32_t *)p;
+  ok &= ok && alloc(&p, WA * 32 * 4); a.rexp = (int32_t *)p;
+  ok &= ok && alloc(&p, sizeof(Ctrl)); a.ctrl = (Ctrl *)p;
+  ok &= ok && alloc(&p, (int64_t)std::max<int64_t>(P->n_batches, 1) * 4); a.redo = (int *)p;
   ok = ok && alloc(&p, std::max<int64_t>(nch, 1) * WA * 32 * 8); a.hacc = (double *)p;
   ok = ok && alloc(&p, std::max<int64_t>(nch, 1) * WA * 4); a.hmask = (uint32_t *)p;
+  HOST_MARK("b: ws alloc");
   if (!ok) return bail(BCGPU_ENOMEM, "cudaMalloc or upload of the batched workspace failed");
   cudaError_t e = cudaMemsetAsync(a.ctrl, 0, sizeof(Ctrl), stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(a.redo, 0, (size_t)std::max<int64_t>(P->n_batches, 1) * 4, stream);

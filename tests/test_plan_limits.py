@@ -61,3 +61,38 @@ for extra in (-1, 0, rows, 3 * rows, 10 * rows, 40 * rows, 150 * rows, 600 * row
     least = res.pop("least")
     assert res.pop("-1") == 3, least  # BCGPU_ENOMEM
     assert all(v <= 0 for v in res.values()), (least, res)
+
+
+@pytest.mark.parametrize("width,delta", [(128, "P.DELTA_FP32C"), (256, "P.DELTA_FP64")])
+def test_merged_passes_give_way_to_the_rest_of_the_plan(stub_dir, width, delta):  # noqa: F811
+    """Multi-source passes (an R-MAT BCC) beside per-source items (a grid too deep
+    for them) and small BCCs: once a limit is accepted, every larger one is, and
+    what passes run as one take stays within it."""
+    res = run_stub(stub_dir, f"""
+n, us, vs = 0, [], []
+for k, u, v in (G.gen_rmat(12, 16, chain_frac=0.2, chain_hi=8, seed=2), G.gen_grid(90, leaves=50, seed=3),
+                G.pack_graphs(G.gen_ba_batch(6, 60, 300, seed=7))[:3]):
+    us.append(n + u)
+    vs.append(n + v)
+    n += k
+d = decomp(n, np.concatenate(us), np.concatenate(vs))
+got = []
+for i in range(28):
+    limit = int(4e6 * 1.2 ** i)
+    ctx = P.Context(mode=P.MODE_BATCHED, plain_core=1500, batch_width={width}, delta={delta}, workspace_limit=limit)
+    held = []
+    def build():
+        plan = ctx.plan(d)
+        held.append(plan.device_bytes)
+        plan.close()
+    r = raises(build)
+    got.append([limit, r[0] if r else 0, held[0] if held else 0])
+    ctx.close()
+out["got"] = got
+""")["got"]
+    first = next(i for i, g in enumerate(res) if g[1] == 0)
+    assert 0 < first < 20 and all(code == 3 for _, code, _ in res[:first])
+    assert all(code == 0 for _, code, _ in res[first:]), res
+    least = res[first][2]
+    assert all(held <= max(limit, least) for limit, _, held in res[first:]), res
+    assert res[-1][2] > 2 * least  # with room, passes run as one and more sources are in flight
