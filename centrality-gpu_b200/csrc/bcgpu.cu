@@ -857,6 +857,8 @@ void route_core(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem>
       L.core[(size_t)b] = 1;
     }
   }
+  L.core_grid = 0;
+  if (std::find(L.core.begin(), L.core.end(), 1) == L.core.end()) return;
   if (ctx->opts.plain_ctas_per_sm) {
     L.core_block = 1024 / ctx->opts.plain_ctas_per_sm;
   } else {

@@ -52,6 +52,11 @@ __device__ __forceinline__ void wait_while_equal_probe(const unsigned int *word,
   wait_while_equal(word, 0u, limit_ns, err, [] { return false; });
 }
 
+// Shared memory of a CTA on sm_100, static and dynamic. A kernel's limit of the
+// dynamic part belongs to the function, in every thread of the process, so it is
+// always set to all there is, never to what one launch needs.
+constexpr int kSmemPerCta = 227 * 1024;
+
 // Default limit of a device-side wait (bc_opts.wait_limit_ms = 0).
 constexpr unsigned long long kDefaultWaitNs = 60ull * 1000 * 1000 * 1000;
 

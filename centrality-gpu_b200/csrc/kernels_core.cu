@@ -767,13 +767,20 @@ const void *core_fn(int block) {
     default: return nullptr;
   }
 }
+cudaError_t allow_smem(int block) {
+  const size_t fixed = block == 64    ? sizeof(Shared<64>)
+                       : block == 128 ? sizeof(Shared<128>)
+                       : block == 256 ? sizeof(Shared<256>)
+                                      : sizeof(Shared<512>);
+  return cudaFuncSetAttribute(core_fn(block), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta - (int)fixed);
+}
 }  // namespace
 
 int core_ctas_per_sm(int block, const CoreArgs::CoreShape &shape) {
   const void *fn = core_fn(block);
   int n = 0;
   if (!fn) return 0;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem_bytes()) != cudaSuccess ||
+  if (allow_smem(block) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, (size_t)shape.smem_bytes()) != cudaSuccess) {
     cudaGetLastError();
     return 0;
@@ -785,7 +792,7 @@ cudaError_t launch_core(const CoreArgs &a, int block, int grid, cudaStream_t str
   const void *fn = core_fn(block);
   if (!fn) return cudaErrorInvalidValue;
   const size_t smem = (size_t)a.shape.smem_bytes();
-  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_smem(block);
   if (e != cudaSuccess) return e;
   CoreArgs args = a;
   void *params[] = {&args};

@@ -866,18 +866,20 @@ const void *tile_fn(int cls) {
          : cls == kTileCta512x8  ? reinterpret_cast<const void *>(tile_cta_kernel<512, 64>)
                                  : reinterpret_cast<const void *>(tile_cta_kernel<256, 32>);
 }
+cudaError_t allow_smem(int cls) {
+  return cudaFuncSetAttribute(tile_fn(cls), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta);
+}
 }  // namespace
 
 int tile_ctas_per_sm(int cls, size_t smem) {
   int n = 0;
-  if (cudaFuncSetAttribute(tile_fn(cls), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return 0;
+  if (allow_smem(cls) != cudaSuccess) return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_fn(cls), block_of(cls), smem) != cudaSuccess) return 0;
   return n;
 }
 
 cudaError_t launch_tile(int cls, const TileArgs &a, int grid, size_t smem, cudaStream_t stream) {
-  cudaError_t e = cudaFuncSetAttribute(tile_fn(cls), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_smem(cls);
   if (e != cudaSuccess) return e;
   switch (cls) {
     case kTileWarp: tile_warp_kernel<<<grid, kThreads, smem, stream>>>(a); break;
