@@ -21,9 +21,9 @@ TWO_KERNELS = """
 def two_kernels():
     rng = np.random.default_rng(5)
     n, us, vs = 0, [], []
-    for size, chain in ((9000, 0), (9000, 70)):
+    for size, chain in ((14000, 0), (14000, 70)):
         i = np.arange(size)
-        u, v = np.concatenate([i, rng.integers(0, size, 9000)]), np.concatenate([(i + 1) % size, rng.integers(0, size, 9000)])
+        u, v = np.concatenate([i, rng.integers(0, size, size)]), np.concatenate([(i + 1) % size, rng.integers(0, size, size)])
         path = np.concatenate([[0], size + np.arange(chain), [size // 2]])
         us += [n + u, n + path[:-1]]
         vs += [n + v, n + path[1:]]
