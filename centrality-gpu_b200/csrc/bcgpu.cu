@@ -1165,22 +1165,6 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
   }
   if (sources) {
     p->n_items = (int64_t)items.size();
-    for (size_t i = 0; i < items.size(); ++i) {
-      const auto &it = items[i];
-      int64_t src = it.own ? 1 : 0, aux = it.own ? 0 : 1;
-      int32_t prev = -1;
-      for (int32_t c = it.c0; c < it.c1; ++c) {
-        src += B->chain_len[c];
-        if (B->chain_r[c] != prev) { ++aux; prev = B->chain_r[c]; }
-      }
-      const int64_t nb = B->vtx_off[it.bcc + 1] - B->vtx_off[it.bcc];
-      const int64_t arcs = B->row[B->vtx_off[it.bcc + 1]] - B->row[B->vtx_off[it.bcc]];
-      p->unit_sources.push_back(p->unit_sources.back() + src);
-      p->unit_teps.push_back(p->unit_teps.back() + src * arcs);
-      p->unit_bfs.push_back(p->unit_bfs.back() + (it.own ? 1 : 0));
-      p->unit_aux.push_back(p->unit_aux.back() + aux);
-      p->unit_visits.push_back(p->unit_visits.back() + src * nb);
-    }
     p->ws_n = L.ws_n;
     // Where every item is a small BCC's, the slices and the slot of the row export
     // are all there is to hold: a little of that is allocated without asking.
@@ -1205,6 +1189,25 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
     p->core_slots = (int)slots.core;
     p->core_block = L.core_block;
     p->core.shape = L.shape;
+    for (size_t i = 0; i < items.size(); ++i) {
+      const auto &it = items[i];
+      int64_t src = it.own ? 1 : 0, aux = it.own ? 0 : 1;
+      int32_t prev = -1;
+      for (int32_t c = it.c0; c < it.c1; ++c) {
+        src += B->chain_len[c];
+        if (B->chain_r[c] != prev) { ++aux; prev = B->chain_r[c]; }
+      }
+      const int64_t nb = B->vtx_off[it.bcc + 1] - B->vtx_off[it.bcc];
+      const int64_t arcs = B->row[B->vtx_off[it.bcc + 1]] - B->row[B->vtx_off[it.bcc]];
+      // the whole-BCC kernel merges chain sources from its ends' BFS; the others
+      // run one for every source
+      const bool merged = L.item_at[i + 1] > L.item_at[i];
+      p->unit_sources.push_back(p->unit_sources.back() + src);
+      p->unit_teps.push_back(p->unit_teps.back() + src * arcs);
+      p->unit_bfs.push_back(p->unit_bfs.back() + (merged ? (it.own ? 1 : 0) : src));
+      p->unit_aux.push_back(p->unit_aux.back() + (merged ? aux : 0));
+      p->unit_visits.push_back(p->unit_visits.back() + src * nb);
+    }
     p->src_at = std::move(L.src_at);
     p->core_at = std::move(L.core_at);
     p->item_at = std::move(L.item_at);

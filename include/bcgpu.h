@@ -127,8 +127,9 @@ typedef struct bc_bccs {
 
 typedef struct bc_stats {
   int64_t sources;        /* sources whose dependencies were accumulated */
-  int64_t bfs_sources;    /* of which ran a forward BFS (the others were merged from chain endpoints) */
-  int64_t aux_bfs;        /* extra forward-only BFS runs for chain endpoints */
+  int64_t bfs_sources;    /* of which ran a forward BFS (the others were merged from chain endpoints,
+                             which the whole-BCC per-source kernel does) */
+  int64_t aux_bfs;        /* extra forward-only BFS runs for chain endpoints (that kernel's) */
   int64_t teps_edges;     /* sum over sources of the arcs of the source's BCC (TEPS numerator) */
   double kernel_ms;       /* device time of the BC kernels (CUDA events) */
   double total_ms;        /* device time of the whole call incl. copies */
