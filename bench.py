@@ -280,10 +280,10 @@ def traffic_per_source(mode, workload):
 
 
 def plain_sample(P, d, device, stream, waves, batched_gteps, whole=False):
-    """Times the plain FP64 schedule (one source per CTA) on `waves` full
-    waves of its work items, taken from two places in the largest BCC's item
-    list (or on all its items when `whole`), with CUDA events; returns its TEPS
-    and the batched/plain ratio."""
+    """Times the plain FP64 schedule (one source per CTA) on `waves` times as many
+    of its work items (a vertex and the chains it owns) as CTAs are resident, taken
+    from two places in the largest BCC's item list (or on all its items when
+    `whole`), with CUDA events; returns its TEPS and the batched/plain ratio."""
     import torch
     pctx = P.Context(mode=P.MODE_PLAIN, device=device, stream=stream.cuda_stream)
     pplan = pctx.plan(d)
@@ -313,7 +313,7 @@ def plain_sample(P, d, device, stream, waves, batched_gteps, whole=False):
     return {"value": g, "unit": "GTEPS", "dtype": "f64", "items": sum(b - a for a, b in picks), "sources": int(src),
             "ms": ms, "resident_ctas": slots, "batched_over_plain": batched_gteps / g,
             "sample": "every plain work item (the whole workload)" if whole else
-                      f"{waves} full waves of plain work items ({slots} resident CTAs) at 25% and 75% of the item list"}
+                      f"plain work items, {waves} times the {slots} resident CTAs, at 25% and 75% of the item list"}
 
 
 def run_reference(args):
@@ -364,8 +364,8 @@ def main():
                     help="--impl reference: seconds of CPU work per step (its sources are sized to it)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--plain-waves", type=int, default=6,
-                    help="batched runs: also time the plain FP64 schedule on this many full waves of its work "
-                         "items (one item per resident CTA), the denominator of batched vs plain (0 = skip)")
+                    help="batched runs: also time the plain FP64 schedule on this many times as many work items as "
+                         "CTAs are resident, the denominator of batched vs plain (0 = skip)")
     ap.add_argument("--graph", type=int, choices=[0, 1], default=1,
                     help="1: every step is one launch of a CUDA graph of the step's device work, recorded "
                          "(stream capture, nothing runs) before the warm-up; 0: the work is enqueued directly")

@@ -1503,7 +1503,12 @@ extern "C" int bc_plan_tile_launches(const bc_plan *p, int32_t *cls, int32_t *gr
   }
   return n;
 }
-extern "C" int bc_plan_concurrency(const bc_plan *p) { return !p ? 0 : p->mode == BCGPU_MODE_BATCHED ? 1 : p->grid; }
+
+extern "C" int bc_plan_concurrency(const bc_plan *p) {
+  if (!p || p->mode == BCGPU_MODE_BATCHED) return p ? 1 : 0;
+  const int slots = std::max(p->core_slots, p->slots);
+  return slots ? slots : p->grid;
+}
 
 extern "C" int64_t bc_plan_unit_sources(const bc_plan *p, int64_t begin, int64_t end, int64_t *out, int64_t cap) {
   if (!p) return -BCGPU_EINVAL;

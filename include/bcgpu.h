@@ -245,9 +245,13 @@ int64_t bc_plan_device_bytes(const bc_plan *plan);
  * up to cap entries; returns the number of launches (negative error code on
  * failure). Introspection for tests and tools; no reference counterpart. */
 int bc_plan_tile_launches(const bc_plan *plan, int32_t *cls, int32_t *grid, int32_t cap);
-/* Work units that run at once: PLAIN, the resident CTAs (one item each);
- * BATCHED, 1 (one pass at a time over the whole GPU). No reference
- * counterpart: the reference launches one source at a time. */
+/* How much a range of units should hold to fill the GPU. PLAIN: the resident
+ * CTAs of the kernel its items run on -- one source each of the contracted
+ * per-source kernel's, one item each (its own vertex and its chains) of the
+ * whole-BCC kernel's, the larger number when a plan uses both; where every item
+ * runs on the small-BCC kernels, which take sources of many items together, the
+ * CTAs that plain_ctas_per_sm asks for. BATCHED: 1 (passes take the whole GPU).
+ * No reference counterpart: the reference launches one source at a time. */
 int bc_plan_concurrency(const bc_plan *plan);
 
 /* Batch-width autotuner (no reference counterpart: the reference has one

@@ -1,5 +1,5 @@
 """What a plan says of its per-source work, on the stand-in runtime: the BFS runs
-of each kernel that items go to."""
+of each kernel that items go to, and the CTAs of it that are resident."""
 import pytest
 
 from test_host_plumbing import run_stub, stub_dir  # noqa: F401
@@ -40,3 +40,18 @@ ctx.close()
     assert sources > res["own"]
     assert (bfs, aux > 0) == ((res["own"], True) if merged else (sources, False))
     assert (res["first"][1] == res["first"][0]) == (not merged)
+
+
+def test_concurrency_is_of_the_kernel_that_runs(stub_dir):  # noqa: F811
+    """With 16 CTAs an SM asked for (the stand-in device has 148, and says that four
+    CTAs of any kernel fit): the contracted kernel's own, or the whole-BCC kernel's."""
+    res = run_stub(stub_dir, RING + """
+for name, size, chains, length in (("contracted", 14000, 4, 9), ("whole", 14000, 4, 70)):
+    d = decomp(*ring(size, size, chains, length, 1))
+    ctx = P.Context(mode=P.MODE_PLAIN, plain_ctas_per_sm=16)
+    plan = ctx.plan(d)
+    out[name] = plan.concurrency
+    plan.close()
+    ctx.close()
+""")
+    assert res == {"contracted": 148 * 4, "whole": 148 * 16}
