@@ -837,7 +837,7 @@ int tile_class(int64_t n, int64_t slice_bytes, size_t lim) {
   if (n > kTileMaxVertices) return -1;
   if (n <= kTileGroups32 && fits(kTileCta256x8)) return kTileCta256x8;
   if (n <= kTileGroups64 && fits(kTileCta512x8)) return kTileCta512x8;
-  if (n <= kTileWarpMaxVertices) return fits(kTileWarp) ? kTileWarp : -1;
+  if (n <= kTileWarpMaxVertices) return -1;  // the warp class takes more shared memory still
   const int64_t per = kTileSmPerSm / ((int64_t)tile_smem_bytes(kTileCta, n, slice_bytes) + kTileReserved);
   if (per <= 7 && fits(kTileCta1024x8)) return kTileCta1024x8;
   if (per >= 4) return kTileCta;

@@ -47,14 +47,13 @@ static_assert(kMaxVertices <= kAccMaxAdds, "one call's sources must fit the fixe
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
-// The small-BCC kernels' part, in place of the rows: slice, items, level offsets.
+// The small-BCC kernels' part, in place of the rows: slice and items.
 constexpr int64_t kOffSlice = 0;
 constexpr int64_t kBytesSlice = 256 * 1024;  // more than a CTA's shared memory
 constexpr int64_t kOffTileItems = kOffSlice + kBytesSlice;
 constexpr int64_t kBytesTileItems = kMaxVertices * (int64_t)sizeof(TileItem);
 constexpr int64_t kOffTileMeta = kOffTileItems + kBytesTileItems;  // slice_off, slice_bytes
-constexpr int64_t kOffTileLv = kOffTileMeta + 256;
-constexpr int64_t kBytesTileLv = kOffRow - kOffTileLv;
+static_assert(kOffTileMeta + 256 <= kOffRow, "the small-BCC kernels' part fits the rows' place");
 
 struct Layout {
   int32_t *ws_i;
@@ -237,8 +236,6 @@ cudaError_t enqueue(unsigned char *base, const Layout &L, int cls, size_t smem, 
     a.src_hi = nsrc;
     a.next_item = L.counter;
     a.acc = L.acc;
-    a.ws_lv = reinterpret_cast<int32_t *>(base + kOffTileLv);
-    a.cap = n + 2;
     a.nmax = n;
     a.slice_max = (int32_t)TileSlice::bytes(n, slice_pair(m, n));
     a.wait_ns = kDefaultWaitNs;
@@ -301,8 +298,7 @@ extern "C" int bc_begin_free_noalloc(bc_ctx *ctx, const int32_t *R, const int32_
     g_acc[dev] = false;
   }
   const Layout L = layout(base, n);
-  // the small-BCC kernels where the BCC fits; their level offsets have to fit
-  // the array too
+  // the small-BCC kernels where the BCC fits
   const int64_t slice = TileSlice::bytes(n, slice_pair(m, n));
   int cls = m <= INT32_MAX / 4 ? tile_class(n, slice, tile_smem_limit(dev)) : -1;
   size_t smem = 0;
@@ -311,7 +307,6 @@ extern "C" int bc_begin_free_noalloc(bc_ctx *ctx, const int32_t *R, const int32_
     smem = tile_smem_bytes(cls, n, slice);
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
       grid = sms * tile_ctas_per_sm(cls, smem);
-    if (cls == kTileWarp) grid = (int)std::min<int64_t>(grid, kBytesTileLv / (4 * kTileWarps * (int64_t)(n + 2)));
     if (grid < 1) cls = -1;
   }
   const bool timing = time_s != nullptr;

@@ -35,7 +35,7 @@ constexpr int kTileWarps = 8;          // warps per CTA
 constexpr int kTileMaxLevels = 1024;   // BFS levels the CTA class records (routing keeps BCCs below)
 constexpr int kTileGroupMaxLevels = 256;  // the same for the grouped classes
 constexpr int kGroupLongQueue = 256;      // long-row queues of a group in the grouped classes
-constexpr int64_t kTileWarpMaxVertices = 640;  // BCCs of up to this many vertices take the warp class
+constexpr int64_t kTileWarpMaxVertices = 640;  // largest BCCs for the warp class: those too deep for groups of 32
 constexpr int64_t kTileGroups32 = 640, kTileGroups64 = 1200;  // largest BCCs for groups of 32, of 64 threads
 constexpr int64_t kTileSmPerSm = 228 * 1024, kTileReserved = 1024;  // shared memory per SM, per-CTA reserve
 constexpr int32_t kTileMaxVertices = 65535;  // neighbour ids are 16-bit in the slice
@@ -81,8 +81,11 @@ struct TileArgs {
 };
 
 // Class of a lone BCC of n vertices with a slice of slice_bytes, as the plan's
-// buckets (bcgpu.cu build_tiles) would have it, or -1 if none fits lim bytes of
-// shared memory. The classes of several groups hold fewer levels than the others.
+// buckets (bcgpu.cu plan_tiles) would have it were it not too deep for the classes
+// of several groups, which hold fewer levels than the others, or -1 if none fits
+// lim bytes of shared memory. Never the warp class: eight groups of a warp take
+// less shared memory (96 bytes a vertex, not 160), and where that is not so, below
+// 90 vertices, no graph without repeated edges is too large for them.
 int tile_class(int64_t n, int64_t slice_bytes, size_t lim);
 // Sources per work item of a launch of class cls with `grid` resident CTAs and
 // `sources` in all.
