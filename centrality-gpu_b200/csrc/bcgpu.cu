@@ -418,20 +418,25 @@ bool mirrored(const bc_bccs *B, int32_t b) {
 // just its two chain neighbours. With mirrored arcs a BFS from a chain vertex
 // then gives the rows that the merge of the chain's ends gives.
 bool chains_are_paths(const bc_bccs *B, int32_t b) {
-  const int64_t vo = B->vtx_off[b];
+  const int64_t vo = B->vtx_off[b], c0 = B->chain_off[b], c1 = B->chain_off[b + 1];
   std::vector<char> held((size_t)(B->vtx_off[b + 1] - vo), 0);
-  for (int64_t c = B->chain_off[b]; c < B->chain_off[b + 1]; ++c) {
+  int bad = 0;
+#pragma omp parallel for schedule(static) reduction(| : bad) if (held.size() >= (size_t)kParallelBfs)
+  for (int64_t c = c0; c < c1; ++c) {
     const int32_t st = B->chain_start[c], k = B->chain_len[c];
-    if (B->chain_l[c] == B->chain_r[c]) return false;
-    for (int32_t j = 0; j < k; ++j) {
+    bad |= B->chain_l[c] == B->chain_r[c];
+    for (int32_t j = 0; j < k && !bad; ++j) {
       const int32_t prev = j == 0 ? B->chain_l[c] : st + j - 1, next = j == k - 1 ? B->chain_r[c] : st + j + 1;
       const int64_t e0 = B->row[vo + st + j], e1 = B->row[vo + st + j + 1];
-      if (e1 - e0 != 2 || held[(size_t)(st + j)]++) return false;
+      if (e1 - e0 != 2 || __atomic_exchange_n(&held[(size_t)(st + j)], 1, __ATOMIC_RELAXED)) {
+        bad = 1;
+        break;
+      }
       const int32_t x = B->col[e0], y = B->col[e0 + 1];
-      if (!((x == prev && y == next) || (x == next && y == prev))) return false;
+      bad |= !((x == prev && y == next) || (x == next && y == prev));
     }
   }
-  return true;
+  return !bad;
 }
 
 // Pairs of arcs in BCC b's slice: a row of an odd number has a spare place.
@@ -510,6 +515,29 @@ void route_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<char> &on, std
 // 28 KB more): cores of up to 1.5 million vertices.
 constexpr int64_t kCoreBits = 190 * 1024;
 
+// Whether contraction leaves little enough of a BCC: without chains the
+// contracted kernel is the slower one (half as many sources in flight, and its
+// tables to build). Kernel time of the whole-BCC kernel over its: no chains (every
+// free-source call) 512x512 grid 0.44, 400x400 0.80, 250x250 0.95, R-MAT 13 0.66,
+// random of 20,000 vertices 0.79; a share of core vertices of 0.77 to 0.78: R-MAT
+// 13 1.02, random 0.96 to 1.06; 0.66 to 0.69: 1.13 to 1.22; 0.4 grids 2.8 to 3.0.
+// In a deep BCC the whole-BCC kernel sweeps every level once more for each chain
+// source: grids of a share of 0.95 1.13 to 1.44, of 0.91 1.22 to 1.74.
+bool contracts(int64_t ncore, int64_t nb, bool deep) { return deep ? 32 * ncore <= 31 * nb : 4 * ncore <= 3 * nb; }
+// Few sources of a BCC with rows for a whole CTA wait for those rows, not for a
+// place on the GPU, and the contracted kernel's CTAs are wider there. Calls of
+// 1 / 64 / 256 / 512 sources, whole-BCC / contracted kernel, ms: R-MAT 13 5.1 /
+// 6.2 / 7.0 / 8.9 and 4.2 / 4.7 / 6.6 / 10.7, R-MAT 15 21 / 27 / 31 / 42 and 16 /
+// 19 / 28 / 49; on R-MAT 18, of 3.5 million vertices, the tables cost more: 1 / 64 /
+// 256 sources 154-173 / 181-201 / 259-282 and 217 / 246 / 324.
+bool hub_bound(const bc_bccs *B, int32_t b, int64_t sources) {
+  const int64_t vo = B->vtx_off[b], nb = B->vtx_off[b + 1] - vo;
+  if (sources > 256 || nb > 1 << 19) return false;
+  for (int64_t k = vo; k < vo + nb; ++k)
+    if (B->row[k + 1] - B->row[k] > 1024) return true;
+  return false;
+}
+
 // Whether the contracted per-source kernel takes BCC b, by its shape: what
 // mirrored(), chains_are_paths() and a BFS say (the kernel's level tables, its
 // closed forms and a chain source's two ways into the core rest on them), and
@@ -524,6 +552,20 @@ bool core_takes(const bc_bccs *B, int32_t b, std::vector<int32_t> &dist, std::ve
   if (*ecc < 0) *ecc = bcc_ecc0(B, b, dist, queue, nb >= kParallelBfs, &connected);
   return connected;
 }
+
+// Host memory for n values, not cleared: the threads that fill it touch it first.
+template <typename T>
+struct RawList {
+  std::unique_ptr<T[]> at;
+  int64_t n = 0;
+  void resize(int64_t count) {
+    at.reset(new T[(size_t)count]);
+    n = count;
+  }
+  bool empty() const { return n == 0; }
+  int64_t size() const { return n; }
+  const T *data() const { return at.get(); }
+};
 
 // The small-BCC schedule of a plan, laid out before any of it is allocated.
 struct TileLayout {
@@ -663,7 +705,7 @@ int plan_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &cls, co
 }
 
 // Uploads what plan_tiles laid out (src: the source list of listed items).
-int build_tiles(const bc_bccs *B, TileLayout &t, const std::vector<int32_t> *src, bc_plan *p) {
+int build_tiles(const bc_bccs *B, TileLayout &t, const RawList<int32_t> *src, bc_plan *p) {
   int rc = BCGPU_OK;
   // slices: row offsets in pairs (uint16 when narrow, else int32), neighbours
   // (uint16, a row's spare place the vertex itself), 16-byte aligned parts; bit 0
@@ -716,7 +758,7 @@ int build_tiles(const bc_bccs *B, TileLayout &t, const std::vector<int32_t> *src
 
 // The contracted per-source kernel's tables (filled on the device), source
 // list and workspace, for the BCCs with on[b] set.
-int build_core(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &on, const std::vector<bcg::CoreSource> &src,
+int build_core(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &on, const RawList<bcg::CoreSource> &src,
                bc_plan *p) {
   int rc = BCGPU_OK;
   bcg::CoreArgs &a = p->core;
@@ -763,9 +805,9 @@ struct SourceLayout {
   std::vector<int8_t> small;      // [n_bcc] small-BCC class, -1: not on the small-BCC kernels
   std::vector<int32_t> small_ecc;
   std::vector<int8_t> core;       // [n_bcc] on the contracted kernel
-  std::vector<int32_t> src;       // the small-BCC kernels' source list, BCC b's from list[b] on
+  RawList<int32_t> src;           // the small-BCC kernels' source list, BCC b's from list[b] on
   std::vector<int64_t> list;
-  std::vector<bcg::CoreSource> csrc;   // the contracted kernel's
+  RawList<bcg::CoreSource> csrc;       // the contracted kernel's
   std::vector<bcg::PlainItem> rest;    // the whole-BCC kernel's items
   std::vector<int64_t> src_at, core_at, item_at;  // what lies before each item in each list
   TileLayout tiles;
@@ -784,44 +826,52 @@ struct SourceLayout {
 
 // The source lists by what small and core say.
 void split_sources(const bc_bccs *B, const std::vector<bcg::PlainItem> &items, SourceLayout &L) {
-  L.src.clear();
-  L.csrc.clear();
-  L.rest.clear();
-  L.src_at.clear();
-  L.core_at.clear();
-  L.item_at.clear();
+  const int64_t n = (int64_t)items.size();
+  L.src_at.assign((size_t)n + 1, 0);
+  L.core_at.assign((size_t)n + 1, 0);
+  L.item_at.assign((size_t)n + 1, 0);
   L.list.assign((size_t)B->n_bcc + 1, 0);
+  L.rest.clear();
   L.ncore = 0;
   for (int32_t b = 0; b < B->n_bcc; ++b)
     if (L.core[(size_t)b]) L.ncore += B->n_plain[b];
-  auto mark = [&] {
-    L.src_at.push_back((int64_t)L.src.size());
-    L.core_at.push_back((int64_t)L.csrc.size());
-    L.item_at.push_back((int64_t)L.rest.size());
-  };
-  for (const auto &it : items) {
-    mark();
-    const bool t = L.small[(size_t)it.bcc] >= 0;
-    if (!t && !L.core[(size_t)it.bcc]) {
+  for (int64_t i = 0; i < n; ++i) {
+    const auto &it = items[(size_t)i];
+    const bool t = L.small[(size_t)it.bcc] >= 0, core = !t && L.core[(size_t)it.bcc];
+    int64_t k = it.own ? 1 : 0;
+    if (t || core)
+      for (int32_t c = it.c0; c < it.c1; ++c) k += B->chain_len[c];
+    else
       L.rest.push_back(it);
-      continue;
-    }
+    L.src_at[(size_t)i + 1] = L.src_at[(size_t)i] + (t ? k : 0);
+    L.core_at[(size_t)i + 1] = L.core_at[(size_t)i] + (core ? k : 0);
+    L.item_at[(size_t)i + 1] = (int64_t)L.rest.size();
+    if (t) L.list[(size_t)it.bcc + 1] = L.src_at[(size_t)i + 1];
+  }
+  for (int32_t b = 0; b < B->n_bcc; ++b) L.list[(size_t)b + 1] = std::max(L.list[(size_t)b + 1], L.list[(size_t)b]);
+  L.src.resize(L.src_at.back());
+  L.csrc.resize(L.core_at.back());
+#pragma omp parallel for schedule(static) if (L.src.n + L.csrc.n >= kParallelBfs)
+  for (int64_t i = 0; i < n; ++i) {
+    const auto &it = items[(size_t)i];
+    const bool t = L.small[(size_t)it.bcc] >= 0;
+    if (!t && !L.core[(size_t)it.bcc]) continue;
+    int64_t at = t ? L.src_at[(size_t)i] : L.core_at[(size_t)i];
     auto add = [&](int32_t s) {
-      if (t) L.src.push_back(s);
-      else L.csrc.push_back({it.bcc, s});
+      if (t) L.src.at[(size_t)at] = s;
+      else L.csrc.at[(size_t)at] = {it.bcc, s};
+      ++at;
     };
     if (it.own) add(it.src);
     for (int32_t c = it.c0; c < it.c1; ++c)
       for (int32_t k = 0; k < B->chain_len[c]; ++k) add(B->chain_start[c] + k);
-    if (t) L.list[(size_t)it.bcc + 1] = (int64_t)L.src.size();
   }
-  mark();
-  for (int32_t b = 0; b < B->n_bcc; ++b) L.list[(size_t)b + 1] = std::max(L.list[(size_t)b + 1], L.list[(size_t)b]);
 }
 
-// The BCCs of the items on the contracted kernel: those it takes, if its slot is
-// no larger than the whole-BCC kernel's (long chains in a BCC of few chain
-// vertices are not worth their buckets).
+// The BCCs of the items on the contracted kernel: those it takes, if enough of
+// their vertices are on chains and its slot is no larger than the whole-BCC
+// kernel's (long chains in a BCC of few chain vertices are not worth their
+// buckets).
 // Its CTAs: as wide as its levels are (core vertices over the depth seen
 // from local vertex 0, and half as much again), between 64 and 512 threads,
 // as many as fit. Narrow levels leave a wide CTA's warps idle, and wide
@@ -834,28 +884,60 @@ void route_core(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem>
   L.core.assign((size_t)B->n_bcc, 0);
   L.shape = {4, 2, 0, 2, 3};
   int levels = 1;  // the deepest core's
-  if (L.listed) {
-    std::vector<int32_t> dist, queue;
-    std::vector<char> seen((size_t)B->n_bcc, 0);
-    for (const auto &it : items) {
-      const int32_t b = it.bcc;
-      if (seen[(size_t)b] || L.small[(size_t)b] >= 0) continue;
-      seen[(size_t)b] = 1;
-      int32_t ecc = ecc0.empty() ? -1 : ecc0[(size_t)b];
-      if (!core_takes(B, b, dist, queue, &ecc, !conn0.empty() && conn0[(size_t)b])) continue;
-      int kmax = 0;
-      for (int64_t c = B->chain_off[b]; c < B->chain_off[b + 1]; ++c) kmax = std::max(kmax, B->chain_len[c]);
-      bcg::CoreArgs::CoreShape h = L.shape;
-      h.cap = std::max<int64_t>(h.cap, (B->n_plain[b] + 3) / 4 * 4);  // 16-byte parts of shared memory
-      h.bcap = std::max<int64_t>(h.bcap, 2 * (B->chain_off[b + 1] - B->chain_off[b]) + 2);
-      h.ccap = std::max(h.ccap, B->chain_off[b + 1] - B->chain_off[b]);
-      h.tcap = std::max(h.tcap, 2 * ecc + kmax + 3);
-      h.ring = std::max(h.ring, kmax + 3);
-      if (h.rec_bytes() + h.rest_bytes() > std::max<int64_t>(L.row_bytes(), 1 << 16) || h.smem_bytes() > kCoreBits) continue;
-      levels = std::max(levels, ecc);
-      L.shape = h;
-      L.core[(size_t)b] = 1;
+  auto size_of = [&](int32_t b) { return B->vtx_off[b + 1] - B->vtx_off[b]; };
+  std::vector<int32_t> bccs, ecc((size_t)B->n_bcc, -1);
+  std::vector<char> takes((size_t)B->n_bcc, 0), hubs((size_t)B->n_bcc, 0);
+  for (size_t i = 0; L.listed && i < items.size();) {  // a BCC's items are next to each other
+    const int32_t b = items[i].bcc;
+    int64_t sources = 0;
+    for (; i < items.size() && items[i].bcc == b; ++i) {
+      sources += items[i].own ? 1 : 0;
+      for (int32_t c = items[i].c0; c < items[i].c1; ++c) sources += B->chain_len[c];
     }
+    if (L.small[(size_t)b] >= 0) continue;
+    hubs[(size_t)b] = hub_bound(B, b, sources);
+    if (hubs[(size_t)b] || contracts(B->n_plain[b], size_of(b), true)) bccs.push_back(b);
+  }
+  auto big = [&](int32_t b) { return size_of(b) >= kParallelBfs; };
+  auto look = [&](int32_t b, std::vector<int32_t> &dist, std::vector<int32_t> &queue) {
+    if (!ecc0.empty()) ecc[(size_t)b] = ecc0[(size_t)b];
+    takes[(size_t)b] = core_takes(B, b, dist, queue, &ecc[(size_t)b], !conn0.empty() && conn0[(size_t)b]);
+  };
+  {
+    std::vector<int32_t> dist, queue;
+    for (int32_t b : bccs)
+      if (big(b)) look(b, dist, queue);  // one BCC at a time, its loops in parallel
+  }
+  int nomem = 0;  // no exception leaves a parallel region
+#pragma omp parallel reduction(| : nomem) if (bccs.size() > 1)
+  {
+    std::vector<int32_t> dist, queue;
+#pragma omp for schedule(dynamic, 1)
+    for (size_t i = 0; i < bccs.size(); ++i) {
+      if (big(bccs[i])) continue;
+      try {
+        look(bccs[i], dist, queue);
+      } catch (const std::bad_alloc &) {
+        nomem = 1;
+      }
+    }
+  }
+  if (nomem) throw std::bad_alloc();
+  for (int32_t b : bccs) {
+    if (!takes[(size_t)b]) continue;
+    if (!hubs[(size_t)b] && !contracts(B->n_plain[b], size_of(b), 2 * ecc[(size_t)b] > kBatchedMaxLevels)) continue;
+    int kmax = 0;
+    for (int64_t c = B->chain_off[b]; c < B->chain_off[b + 1]; ++c) kmax = std::max(kmax, B->chain_len[c]);
+    bcg::CoreArgs::CoreShape h = L.shape;
+    h.cap = std::max<int64_t>(h.cap, (B->n_plain[b] + 3) / 4 * 4);  // 16-byte parts of shared memory
+    h.bcap = std::max<int64_t>(h.bcap, 2 * (B->chain_off[b + 1] - B->chain_off[b]) + 2);
+    h.ccap = std::max(h.ccap, B->chain_off[b + 1] - B->chain_off[b]);
+    h.tcap = std::max(h.tcap, 2 * ecc[(size_t)b] + kmax + 3);
+    h.ring = std::max(h.ring, kmax + 3);
+    if (h.rec_bytes() + h.rest_bytes() > std::max<int64_t>(L.row_bytes(), 1 << 16) || h.smem_bytes() > kCoreBits) continue;
+    levels = std::max(levels, ecc[(size_t)b]);
+    L.shape = h;
+    L.core[(size_t)b] = 1;
   }
   L.core_grid = 0;
   if (std::find(L.core.begin(), L.core.end(), 1) == L.core.end()) return;
@@ -959,13 +1041,16 @@ SourceSlots settle_sources(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg:
   }
   SourceSlots r = fit_slots(ctx, B, L, room);
   if (!L.csrc.empty() && r.core < std::min<int64_t>(L.core_grid, (int64_t)L.csrc.size())) {
-    SourceLayout alone = L;
-    std::fill(alone.core.begin(), alone.core.end(), 0);
-    split_sources(B, items, alone);
-    const SourceSlots w = fit_slots(ctx, B, alone, room);
-    if (2 * r.core < w.whole || source_bytes(B, L, r) > room) {
-      L = std::move(alone);
+    const int64_t held = source_bytes(B, L, r);
+    const std::vector<int8_t> core = L.core;
+    std::fill(L.core.begin(), L.core.end(), 0);
+    split_sources(B, items, L);
+    const SourceSlots w = fit_slots(ctx, B, L, room);
+    if (2 * r.core < w.whole || held > room) {
       r = w;
+    } else {
+      L.core = core;
+      split_sources(B, items, L);
     }
   }
   if (source_bytes(B, L, r) > room && L.rest.size() < items.size()) {  // slices, lists and one slot do not fit

@@ -24,7 +24,7 @@ def test_bfs_runs_by_kernel(stub_dir, size, length, merged):  # noqa: F811
     """A BCC in shared memory, one on the contracted kernel, and one with chains too
     long for that: only the last merges its chain sources."""
     res = run_stub(stub_dir, RING + f"""
-d = decomp(*ring({size}, {size}, 4, {length}, 1))
+d = decomp(*ring({size}, {size}, {400 if size > 1000 else 4}, {length}, 1))
 a = d.arrays()
 ctx = P.Context(mode=P.MODE_PLAIN)
 plan = ctx.plan(d)
@@ -44,14 +44,59 @@ ctx.close()
 
 def test_concurrency_is_of_the_kernel_that_runs(stub_dir):  # noqa: F811
     """With 16 CTAs an SM asked for (the stand-in device has 148, and says that four
-    CTAs of any kernel fit): the contracted kernel's own, or the whole-BCC kernel's."""
+    CTAs of any kernel fit): the contracted kernel's own, or the whole-BCC kernel's, which
+    takes the BCCs with chains too long for that one and those with few chains: a
+    seventh of a ring's vertices have no chord."""
     res = run_stub(stub_dir, RING + """
-for name, size, chains, length in (("contracted", 14000, 4, 9), ("whole", 14000, 4, 70)):
-    d = decomp(*ring(size, size, chains, length, 1))
+for name, chains, length in (("contracted", 400, 9), ("long chains", 80, 70), ("few chains", 10, 9)):
+    d = decomp(*ring(14000, 14000, chains, length, 1))
     ctx = P.Context(mode=P.MODE_PLAIN, plain_ctas_per_sm=16)
     plan = ctx.plan(d)
     out[name] = plan.concurrency
     plan.close()
     ctx.close()
 """)
-    assert res == {"contracted": 148 * 4, "whole": 148 * 16}
+    assert res == {"contracted": 148 * 4, "long chains": 148 * 16, "few chains": 148 * 16}
+
+
+@pytest.mark.parametrize("sub_p,contracted", [(0.0, False), (0.02, True)])
+def test_deep_bccs_with_any_chains_are_contracted(stub_dir, sub_p, contracted):  # noqa: F811
+    """A grid of 130 x 130 with no vertex on a chain, and with one in eleven."""
+    res = run_stub(stub_dir, f"""
+d = decomp(*G.gen_grid(130, delete_frac=0.0, sub_p={sub_p}, leaves=0, seed=3))
+a = d.arrays()
+out["share"] = int(a["n_plain"][0]) / int(a["n_packed"])
+ctx = P.Context(mode=P.MODE_PLAIN, plain_ctas_per_sm=16)
+plan = ctx.plan(d)
+out["concurrency"] = plan.concurrency
+plan.close()
+ctx.close()
+""")
+    assert (res["share"] > 0.97) == (not contracted) and res["share"] > 0.8
+    assert res["concurrency"] == 148 * (4 if contracted else 16)
+
+
+@pytest.mark.parametrize("sources,contracted", [(256, True), (257, False)])
+def test_few_sources_of_a_bcc_with_hubs_are_contracted(stub_dir, sources, contracted):  # noqa: F811
+    """A free-source call has no chains: only up to 256 sources of a BCC with a row
+    of more than 1,024 arcs go to the contracted kernel, which allocates tables."""
+    res = run_stub(stub_dir, f"""
+L.stub_cudart_mallocs.restype = C.c_longlong
+rng = np.random.default_rng(3)
+n = 16000
+i = np.arange(n)
+counts = []
+for hub in (1500, 1000):
+    a = decomp(n, *G.simple_edges(n, np.concatenate([i, rng.integers(0, n, n), np.zeros(hub, int)]),
+                                  np.concatenate([(i + 1) % n, rng.integers(0, n, n), rng.permutation(n)[:hub]]))).arrays()
+    assert a["n_bcc"] == 1 and int(a["n_packed"]) == n
+    src = np.arange({sources}, dtype=np.int32)
+    ctx = P.Context(mode=P.MODE_PLAIN)
+    m0 = L.stub_cudart_mallocs()
+    P.begin_gpu_free(ctx, a["row"].astype(np.int32), a["col"].astype(np.int32), n, len(a["col"]), src,
+                     a["reach"].astype(np.int32), np.zeros(n, np.float32))
+    counts.append(L.stub_cudart_mallocs() - m0)
+    ctx.close()
+out["more"] = counts[0] - counts[1]
+""")
+    assert (res["more"] > 0) == contracted

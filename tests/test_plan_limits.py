@@ -24,6 +24,7 @@ def two_kernels():
     for size, chain in ((14000, 0), (14000, 70)):
         i = np.arange(size)
         u, v = np.concatenate([i, rng.integers(0, size, size)]), np.concatenate([(i + 1) % size, rng.integers(0, size, size)])
+        size, u, v = G.subdivide(size, u, v, 0.2, 1, 4, rng)
         path = np.concatenate([[0], size + np.arange(chain), [size // 2]])
         us += [n + u, n + path[:-1]]
         vs += [n + v, n + path[1:]]
