@@ -1330,7 +1330,7 @@ int create_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem>
   bc_plan *p = nullptr;
   int rc;
   try {
-    const bcg::SmallTeam team(B ? B->n_packed : 0, B ? B->n_arcs : 0);
+    const bcg::SmallTeam team(B ? B->n_packed : 0, B ? B->n_arcs : 0, bcg::kTeamVertices);
     rc = validate(ctx, B);
     if (rc == BCGPU_OK) {
       const cudaError_t e = cudaSetDevice(ctx->device);

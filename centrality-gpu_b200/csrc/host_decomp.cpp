@@ -1132,7 +1132,7 @@ extern "C" int bc_decompose(const bc_graph *g, bc_decomp **out) {
   if (!D) return BCGPU_ENOMEM;
   int rc;
   try {
-    const bcg::SmallTeam team(g->n, (int64_t)g->col.size());
+    const bcg::SmallTeam team(g->n, (int64_t)g->col.size(), bcg::kTeamVertices);
     rc = decompose(g, D);
   } catch (const std::bad_alloc &) {
     rc = BCGPU_ENOMEM;
