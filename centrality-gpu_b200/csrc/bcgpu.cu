@@ -16,6 +16,7 @@
 #include "tile.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <chrono>
 #include <cstdio>
@@ -166,6 +167,26 @@ int guard(bc_ctx *ctx, F &&body) {
     return fail(ctx, BCGPU_ENOMEM, "host allocation failed");
   }
 }
+
+// A host allocation that throws on a thread of a parallel region, which no
+// exception may leave: remembered, and thrown again once the region has ended.
+class TeamAlloc {
+ public:
+  template <class F>
+  void run(F &&body) {
+    try {
+      body();
+    } catch (const std::bad_alloc &) {
+      failed_ = true;
+    }
+  }
+  void check() const {
+    if (failed_) throw std::bad_alloc();
+  }
+
+ private:
+  std::atomic<bool> failed_{false};
+};
 
 // Device memory from the context's pool, ordered on its stream. When the
 // pool cannot grow, its unused reserve is trimmed once and the allocation
@@ -326,20 +347,24 @@ int bcc_ecc0(const bc_bccs *B, int32_t b, std::vector<int32_t> &dist, std::vecto
     size_t reached = 1;
     while (true) {
       next.clear();
+      TeamAlloc host;
 #pragma omp parallel
       {
         std::vector<int32_t> mine;
 #pragma omp for schedule(dynamic, 256) nowait
         for (size_t i = 0; i < frontier.size(); ++i) {
           const int32_t x = frontier[i];
-          for (int64_t e = B->row[vo + x]; e < B->row[vo + x + 1]; ++e) {
-            const int32_t y = B->col[e];
-            if (dist[y] < 0 && __sync_bool_compare_and_swap(&dist[y], -1, lev + 1)) mine.push_back(y);
-          }
+          host.run([&] {
+            for (int64_t e = B->row[vo + x]; e < B->row[vo + x + 1]; ++e) {
+              const int32_t y = B->col[e];
+              if (dist[y] < 0 && __sync_bool_compare_and_swap(&dist[y], -1, lev + 1)) mine.push_back(y);
+            }
+          });
         }
 #pragma omp critical
-        next.insert(next.end(), mine.begin(), mine.end());
+        host.run([&] { next.insert(next.end(), mine.begin(), mine.end()); });
       }
+      host.check();
       if (next.empty()) {
         *connected = reached == (size_t)nb;
         return lev;
@@ -472,27 +497,30 @@ void route_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<char> &on, std
                                         bcg::kTileMaxVertices);
   std::vector<int64_t> bytes((size_t)B->n_bcc, 0);
   std::vector<int8_t> want((size_t)B->n_bcc, -1);
+  TeamAlloc host;
 #pragma omp parallel
   {
     std::vector<int32_t> dist, queue;
-#pragma omp for schedule(dynamic, 16)
-    for (int32_t b = 0; b < B->n_bcc; ++b) {
-      if (on[b]) continue;
+    auto route = [&](int32_t b) {
       const int64_t vo = B->vtx_off[b], nb = B->vtx_off[b + 1] - vo;
-      if (nb > cap) continue;
+      if (nb > cap) return;
       bytes[b] = bcg::TileSlice::bytes(nb, slice_pairs(B, b));
       const int c = nb <= bcg::kTileWarpMaxVertices ? bcg::kTileWarp : bcg::kTileCta;
-      if (bcg::tile_smem_bytes(fit_cls(c), nb, bytes[b]) > lim) continue;
+      if (bcg::tile_smem_bytes(fit_cls(c), nb, bytes[b]) > lim) return;
       int64_t maxdeg = 1;
       for (int64_t k = vo; k < vo + nb; ++k) maxdeg = std::max(maxdeg, B->row[k + 1] - B->row[k]);
-      if (strict && !(mirrored(B, b) && chains_are_paths(B, b))) continue;
+      if (strict && !(mirrored(B, b) && chains_are_paths(B, b))) return;
       bool connected = true;
       const int ecc = bcc_ecc0(B, b, dist, queue, false, &connected);
       ecc_of[b] = ecc;
-      if (strict && !connected) continue;
+      if (strict && !connected) return;
       if ((2.0 * ecc + 1.0) * std::log2((double)std::max<int64_t>(maxdeg, 2)) <= 1000.0) want[b] = (int8_t)c;
-    }
+    };
+#pragma omp for schedule(dynamic, 16)
+    for (int32_t b = 0; b < B->n_bcc; ++b)
+      if (!on[b]) host.run([&] { route(b); });
   }
+  host.check();
   for (int c : {bcg::kTileWarp, bcg::kTileCta}) {
     std::vector<int32_t> cand;
     for (int32_t b = 0; b < B->n_bcc; ++b)
@@ -908,21 +936,15 @@ void route_core(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem>
     for (int32_t b : bccs)
       if (big(b)) look(b, dist, queue);  // one BCC at a time, its loops in parallel
   }
-  int nomem = 0;  // no exception leaves a parallel region
-#pragma omp parallel reduction(| : nomem) if (bccs.size() > 1)
+  TeamAlloc host;
+#pragma omp parallel if (bccs.size() > 1)
   {
     std::vector<int32_t> dist, queue;
 #pragma omp for schedule(dynamic, 1)
-    for (size_t i = 0; i < bccs.size(); ++i) {
-      if (big(bccs[i])) continue;
-      try {
-        look(bccs[i], dist, queue);
-      } catch (const std::bad_alloc &) {
-        nomem = 1;
-      }
-    }
+    for (size_t i = 0; i < bccs.size(); ++i)
+      if (!big(bccs[i])) host.run([&] { look(bccs[i], dist, queue); });
   }
-  if (nomem) throw std::bad_alloc();
+  host.check();
   for (int32_t b : bccs) {
     if (!takes[(size_t)b]) continue;
     if (!hubs[(size_t)b] && !contracts(B->n_plain[b], size_of(b), 2 * ecc[(size_t)b] > kBatchedMaxLevels)) continue;
@@ -1150,13 +1172,15 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
         for (int32_t b = 0; b < B->n_bcc; ++b)
           if (big(b)) route(b, dist, queue, true);  // one BCC at a time, its levels in parallel
       }
+      TeamAlloc host;
 #pragma omp parallel
       {
         std::vector<int32_t> dist, queue;
 #pragma omp for schedule(dynamic, 1)
         for (int32_t b = 0; b < B->n_bcc; ++b)
-          if (!big(b)) route(b, dist, queue, false);
+          if (!big(b)) host.run([&] { route(b, dist, queue, false); });
       }
+      host.check();
     }
     for (char x : on) n_on += x;
   }
