@@ -268,10 +268,12 @@ def save_sample(P, d, arrs, plan, args, device, stream, width, tile_max):
 
 
 def traffic_per_source(mode, workload):
-    """DRAM bytes per source of the dominant kernel from the committed ncu
-    summary (profiles/<kernel>_<workload>.md, line 'traffic_bytes_per_source: X')."""
+    """DRAM bytes per source of the dominant kernel from the committed ncu summary
+    of that kernel as it is (profiles/<kernel>_<workload>.md, line
+    'traffic_bytes_per_source: X'); none, no figure. PLAIN plans of the workloads with
+    chains run on the contracted per-source kernel."""
     import re
-    name = ("batched_kernel" if mode == "batched" else "plain_kernel") + f"_{workload}.md"
+    name = ("batched_kernel" if mode == "batched" else "core_kernel") + f"_{workload}.md"
     f = ROOT / "profiles" / name
     if not f.exists():
         return None, None
@@ -549,6 +551,8 @@ def main():
                 "traffic": tps * sources / args.steps if tps else None,
                 "traffic_source": f"ncu dram__bytes_read.sum+dram__bytes_write.sum per source ({tsrc}) x sources "
                                   f"per launch" if tps else None,
+                # the share of the measured copy bandwidth that traffic is
+                "dram_frac": tps * sources / args.steps / (avg_launch_ms * 1e-3) / 1e9 / peak if tps else None,
                 "alg_bytes_per_launch": alg_bytes / args.steps, "avg_launch_ms": avg_launch_ms}
 
     # end to end through the public API with host buffers (uploads + download inside)
