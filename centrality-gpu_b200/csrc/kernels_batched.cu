@@ -77,12 +77,17 @@ constexpr int kHeavyDeg = BCGPU_BATCHED_HEAVY_DEG;
 // 32.1 for 128, 55.8 / 31.3 for 512).
 constexpr int kHeavyDegSmall = 512;
 constexpr int kSmallCore = 16384;  // cores below this many vertices use kHeavyDegSmall
-// On large cores a level has enough other rows to hide a longer one behind, and a
-// chunked row costs a partial sum in memory and its combine. Two passes of 512, rows
-// up to 1024 / 2048 arcs on a warp: R-MAT 17 (55,000 core vertices) 22.3 / 23.1 ms,
-// R-MAT 18 46.4 / 51.1, R-MAT 19 87.9 / 87.9, R-MAT 20 (430,000) 139.8 / 132.8.
-constexpr int kHeavyDegLarge = 2 * kHeavyDeg;
-constexpr int kLargeCore = 1 << 18;  // cores from this many vertices on use kHeavyDegLarge
+// Where rows of up to twice that length are as many as the warps in flight, a warp
+// each keeps them all busy, and a chunked row's partial sum in memory and its
+// combine are saved; where they are few, a level waits for them. Two passes of 512
+// at 20% and 60% of the source order, rows up to 1024 / 2048 arcs on a warp, by rows
+// of 1025 to 2048 arcs: 4,845 (R-MAT 20) 167 and 143 / 159 and 135 ms, 5,985 (R-MAT
+// 21, 12 edges a vertex) 275 and 222 / 264 and 213, 4,843 (R-MAT 20 of 24) 216 and
+// 169 / 216 and 171; 989 (R-MAT 20 of 8) 94 and 80 / 107 and 92, 460 and 362
+// (skewed random, 34 and 37 million arcs) 87 and 180 / 106 and 219; R-MAT 17 and 18
+// (two passes in the middle) 22.3 and 46.4 / 23.1 and 51.1, R-MAT 19 even.
+constexpr int kHeavyDegMany = 2 * kHeavyDeg;
+constexpr int64_t kManyRows = 4096;  // rows of kHeavyDeg to kHeavyDegMany arcs that make them many
 #ifndef BCGPU_BATCHED_CHUNK
 #define BCGPU_BATCHED_CHUNK 2048
 #endif
@@ -716,7 +721,7 @@ struct RowLane {
     return lane < (int)(len_j >> 16) ? (uint32_t)ldg(a.hcol + rb + at_j + lane) : 0u;
   }
 };
-static_assert(kHeavyDegLarge < 1 << 16, "a light row's length takes 16 bits");
+static_assert(kHeavyDegMany < 1 << 16, "a light row's length takes 16 bits");
 
 // Heavy-row chunk tasks of a phase: each CTA's first task is its own index;
 // later ones in a fixed stride (BCGPU_BATCHED_HEAVY_DYN 0) or from the
@@ -1664,7 +1669,16 @@ int batched_build(const bc_bccs *B, const BatchedConfig &cfg, const int64_t *row
     HOST_MARK("b: chains");
     // contracted rows: unit arcs first, then chain arcs
     hvo.push_back((int64_t)hrow.size());
-    const int heavy_deg = npl < kSmallCore ? kHeavyDegSmall : npl < kLargeCore ? kHeavyDeg : kHeavyDegLarge;
+    int heavy_deg = kHeavyDegSmall;
+    if (npl >= kSmallCore) {
+      int64_t longer = 0;
+#pragma omp parallel for schedule(static) reduction(+ : longer)
+      for (int32_t x = 0; x < npl; ++x) {
+        const int64_t deg = B->row[vo + x + 1] - B->row[vo + x];
+        longer += deg > kHeavyDeg && deg <= kHeavyDegMany;
+      }
+      heavy_deg = longer < kManyRows ? kHeavyDeg : kHeavyDegMany;
+    }
     // Every arc of a core vertex becomes one contracted arc (a unit arc, or
     // the chain arc of the chain vertex it leads to), so the contracted rows
     // have the original degrees: offsets first, then the rows in parallel.
