@@ -445,15 +445,23 @@ bool mirrored(const bc_bccs *B, int32_t b) {
 bool chains_are_paths(const bc_bccs *B, int32_t b) {
   const int64_t vo = B->vtx_off[b], c0 = B->chain_off[b], c1 = B->chain_off[b + 1];
   std::vector<char> held((size_t)(B->vtx_off[b + 1] - vo), 0);
+  const bool team = held.size() >= (size_t)kParallelBfs;  // else no locked exchanges: 8 us for 1,200 chain vertices
+  auto take = [&](int32_t v) {
+    char &h = held[(size_t)v];
+    if (team) return __atomic_exchange_n(&h, 1, __ATOMIC_RELAXED) != 0;
+    const bool was = h != 0;
+    h = 1;
+    return was;
+  };
   int bad = 0;
-#pragma omp parallel for schedule(static) reduction(| : bad) if (held.size() >= (size_t)kParallelBfs)
+#pragma omp parallel for schedule(static) reduction(| : bad) if (team)
   for (int64_t c = c0; c < c1; ++c) {
     const int32_t st = B->chain_start[c], k = B->chain_len[c];
     bad |= B->chain_l[c] == B->chain_r[c];
     for (int32_t j = 0; j < k && !bad; ++j) {
       const int32_t prev = j == 0 ? B->chain_l[c] : st + j - 1, next = j == k - 1 ? B->chain_r[c] : st + j + 1;
       const int64_t e0 = B->row[vo + st + j], e1 = B->row[vo + st + j + 1];
-      if (e1 - e0 != 2 || __atomic_exchange_n(&held[(size_t)(st + j)], 1, __ATOMIC_RELAXED)) {
+      if (e1 - e0 != 2 || take(st + j)) {
         bad = 1;
         break;
       }
@@ -540,7 +548,7 @@ void route_tiles(bc_ctx *ctx, const bc_bccs *B, const std::vector<char> &on, std
 }
 
 // Shared memory for a bit per core vertex at most (a CTA of 512 threads needs
-// 28 KB more): cores of up to 1.5 million vertices.
+// 28 KB more): cores of up to 1.5 million vertices; from 700,000 on one CTA an SM.
 constexpr int64_t kCoreBits = 190 * 1024;
 
 // Whether contraction leaves little enough of a BCC: without chains the
@@ -804,13 +812,14 @@ int build_core(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &on, con
   bcg::CoreSource *list = nullptr;
   if ((rc = upload(p, &n_plain, B->n_plain, B->n_bcc)) || (rc = upload(p, &chain_off, B->chain_off, B->n_bcc + 1)) ||
       (rc = upload(p, &d_on, on.data(), B->n_bcc)) || (rc = upload(p, &list, src.data(), (int64_t)src.size())) ||
-      (rc = upload(p, &row_off, off.data(), B->n_bcc)) || (rc = dalloc(p, &rows, ncore)) || (rc = dalloc(p, &xcol, B->n_arcs)) || (rc = dalloc(p, &xk, B->n_arcs)) ||
+      (rc = upload(p, &row_off, off.data(), B->n_bcc)) || (rc = dalloc(p, &rows, ncore)) ||
+      (rc = dalloc(p, &xcol, B->n_arcs)) || (rc = dalloc(p, &xk, B->n_arcs)) ||
       (rc = dalloc(p, &xcid, B->n_arcs)) || (rc = dalloc(p, &ctab, B->n_chains)) ||
       (rc = dalloc(p, &vchain, B->n_packed)))
     return rc;
   CK(ctx, bcg::core_contract(p->row, p->col, p->vtx_off, n_plain, p->reach, chain_off, p->chain_start, p->chain_len,
-                             p->chain_l, p->chain_r, d_on, B->n_bcc, B->n_packed, row_off, rows, xcol, xk, xcid, ctab, vchain,
-                             ctx->stream));
+                             p->chain_l, p->chain_r, d_on, B->n_bcc, B->n_packed, row_off, rows, xcol, xk, xcid, ctab,
+                             vchain, ctx->stream));
   const int64_t n = p->core_slots, rec = a.shape.rec_bytes();
   std::vector<int32_t> ep((size_t)n, 1);
   if ((rc = dalloc(p, &a.rec, n * rec)) || (rc = dalloc(p, &a.ws, n * a.shape.rest_bytes())) ||
@@ -819,7 +828,8 @@ int build_core(bc_ctx *ctx, const bc_bccs *B, const std::vector<int8_t> &on, con
   CK(ctx, cudaMemsetAsync(a.rec, 0, (size_t)(n * rec), ctx->stream));  // key 0: unvisited
   CK(ctx, cudaStreamSynchronize(ctx->stream));                         // ep goes out of scope
   a.row = p->row; a.vtx_off = p->vtx_off; a.n_plain = n_plain; a.reach = p->reach; a.chain_off = chain_off;
-  a.rows = rows; a.row_off = row_off; a.xcol = xcol; a.xk = xk; a.xcid = xcid; a.ctab = ctab; a.vchain = vchain; a.src = list;
+  a.rows = rows; a.row_off = row_off; a.xcol = xcol; a.xk = xk; a.xcid = xcid; a.ctab = ctab; a.vchain = vchain;
+  a.src = list;
   a.next = p->counter; a.acc = p->acc; a.err = p->err;
   a.rescale_exp = ctx->opts.rescale_exp > 0 ? ctx->opts.rescale_exp : 900;
   return BCGPU_OK;
@@ -956,7 +966,8 @@ void route_core(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem>
     h.ccap = std::max(h.ccap, B->chain_off[b + 1] - B->chain_off[b]);
     h.tcap = std::max(h.tcap, 2 * ecc[(size_t)b] + kmax + 3);
     h.ring = std::max(h.ring, kmax + 3);
-    if (h.rec_bytes() + h.rest_bytes() > std::max<int64_t>(L.row_bytes(), 1 << 16) || h.smem_bytes() > kCoreBits) continue;
+    if (h.rec_bytes() + h.rest_bytes() > std::max<int64_t>(L.row_bytes(), 1 << 16) || h.smem_bytes() > kCoreBits)
+      continue;
     levels = std::max(levels, ecc[(size_t)b]);
     L.shape = h;
     L.core[(size_t)b] = 1;
@@ -1290,7 +1301,8 @@ int build_plan(bc_ctx *ctx, const bc_bccs *B, const std::vector<bcg::PlainItem> 
     if (room - (int64_t)sizeof(bcg::PlainItem) * std::max<int64_t>(p->n_items, 1) - 64 * (int64_t)ctx->sms <
         2 * L.row_bytes())
       return bail(fail(ctx, BCGPU_ENOMEM, "workspace for the largest BCC exceeds the limit"));
-    if (n_tile) room = std::max(room - tiles.bytes(B->n_bcc, 0), 2 * L.slot() + (int64_t)sizeof(bcg::PlainItem) * p->n_items);
+    const int64_t least = 2 * L.slot() + (int64_t)sizeof(bcg::PlainItem) * p->n_items;
+    if (n_tile) room = std::max(room - tiles.bytes(B->n_bcc, 0), least);
     const SourceSlots slots = settle_sources(ctx, B, items, ecc0, conn0, room, L);
     p->grid = slots.grid;
     p->block = slots.block;

@@ -23,7 +23,7 @@
 //   lm[t][v][w] bitmask of the slots that reach v at level t: the frontier of
 //               the forward phase and the successor test of the backward phase
 // Forward: level-synchronous pull. A core vertex still unseen by some slot
-// scans its row once per 32-slot word: a unit arc to u hits the slots in
+// scans its row once per 128 slots: a unit arc to u hits the slots in
 // lm[t][u], a chain arc of length k+1 hits those in lm[t-k][u]; the hits'
 // path counts are summed (the reference's per-source atomicCAS/atomicAdd BFS,
 // Codes/kernels_free.cu:286-362).
@@ -34,13 +34,14 @@
 // themselves: a closed form in prefix sums of reach+1 along the chain and the
 // two ends' path counts, evaluated for every (vertex, slot) in one parallel
 // phase between the forward and the backward sweeps.
-// Chain vertices: one warp per (chain, 32-slot word) evaluates every chain
-// vertex's dependency for the 32 slots from the endpoint columns.
+// Chain vertices: one warp per chain evaluates every chain vertex's dependency
+// from the endpoint columns, two neighbouring slots a lane.
 // Path counts carry a per-(slot, level) power-of-two base X so deep graphs do
 // not overflow FP64: a level is rescaled when its largest count passes
 // 2^rescale_exp (900 by default).
-// BC: per (vertex, word) FP64 partials, summed over words in fixed order ->
-// deterministic (the reference uses FP32 atomics, Codes/kernels_free.cu:423-426).
+// BC: FP64 partials per vertex and 128 slots, summed in fixed order: the same bits
+// on every run of the same unit ranges (the reference uses FP32 atomics,
+// Codes/kernels_free.cu:423-426). Passes that run as one are summed as one.
 // The whole GPU works on one batch at a time: a cooperative persistent kernel
 // with a grid barrier whose waits are bounded (error flag, no hang).
 #include "accum.cuh"
@@ -184,8 +185,10 @@ struct Args {
   uint32_t *seen;   // [n_cap][W]
   int32_t *lmin;    // [n_cap] first level on which some slot reached the vertex
   int32_t *armed;   // [n_cap] first level on which some slot can reach the vertex (a neighbour was reached)
-  int *wq;          // [4*(tcap+3)+2] work counters: light rows forward (t), backward (tcap+3+lev); heavy chunks (2*(tcap+3)+t, 3*(tcap+3)+lev); chain in-flow (4*(tcap+3)); chain vertices (4*(tcap+3)+1)
-  double *bcpart;   // [n_cap][W] BC partials of the core vertices
+  // [4*(tcap+3)+2] work counters: light rows forward (t), backward (tcap+3+lev); heavy chunks (2*(tcap+3)+t,
+  // 3*(tcap+3)+lev); chain in-flow (4*(tcap+3)); chain vertices (4*(tcap+3)+1)
+  int *wq;
+  double *bcpart;   // [n_cap][W] BC partials of the core vertices (a light row's 128 slots in their first word)
   double *cdep;     // [n_cap][W][32] dependency a core vertex receives from its chains' vertices
   double *wsrc;     // [B] reach(source)+1 of each slot of the pass
   int32_t *schain;  // [B] chain of each slot's source (-1: a core vertex; kNoSlot: no slot)

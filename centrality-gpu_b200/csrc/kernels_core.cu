@@ -37,7 +37,8 @@
 // finds them: with 16 CTAs at different points of the kernel, instruction
 // fetches were a quarter of the stalls. Against the whole-BCC kernel: an 80x80
 // grid 31.2 -> 14.9 ms (14,867 sources), 2,870 sources of a 512x512 grid 356 ->
-// 123 ms, 7,867 sources of R-MAT 14 with 20% chains 233 -> 91 ms.
+// 123 ms, 7,867 sources of R-MAT 14 with 20% chains 233 -> 91 ms. Without chains to
+// contract it is the slower of the two (bcgpu.cu contracts()).
 #include "accum.cuh"
 #include "common.cuh"
 #include "core.h"
@@ -686,8 +687,8 @@ __global__ void chain_table_kernel(const int64_t *vtx_off, const int64_t *chain_
 __global__ void __launch_bounds__(256) contract_kernel(const int64_t *row, const int32_t *col, const int64_t *vtx_off,
                                                        const int32_t *n_plain, const int32_t *reach, const int8_t *on,
                                                        int32_t n_bcc, int64_t n_packed, const int4 *ctab,
-                                                       const int32_t *vchain, const int64_t *row_off, CoreRow *rows, int32_t *xcol, int32_t *xk,
-                                                       int32_t *xcid) {
+                                                       const int32_t *vchain, const int64_t *row_off, CoreRow *rows,
+                                                       int32_t *xcol, int32_t *xk, int32_t *xcid) {
   const int lane = threadIdx.x & 31;
   const uint32_t below = (1u << lane) - 1;
   for (int64_t v = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n_packed;
@@ -752,8 +753,8 @@ cudaError_t core_contract(const int64_t *row, const int32_t *col, const int64_t 
   const int blocks = (int)std::min<int64_t>((n_packed + 7) / 8, 148 * 8);
   chain_table_kernel<<<blocks, 256, 0, stream>>>(vtx_off, chain_off, chain_start, chain_len, chain_l, chain_r, on, n_bcc,
                                                  ctab, vchain);
-  contract_kernel<<<blocks, 256, 0, stream>>>(row, col, vtx_off, n_plain, reach, on, n_bcc, n_packed, ctab, vchain, row_off, rows,
-                                              xcol, xk, xcid);
+  contract_kernel<<<blocks, 256, 0, stream>>>(row, col, vtx_off, n_plain, reach, on, n_bcc, n_packed, ctab, vchain,
+                                              row_off, rows, xcol, xk, xcid);
   return cudaGetLastError();
 }
 

@@ -49,7 +49,9 @@ typedef struct bc_opts {
   int32_t batch_width;   /* sources per batched pass: multiple of 32, <= 1024; 0 = 512
                             (bc_autotune_width measures the best width for a graph) */
   void *stream;          /* cudaStream_t to launch on; NULL = a stream owned by the context */
-  int64_t workspace_limit; /* device bytes the context may hold; 0 = 80% of free memory */
+  int64_t workspace_limit; /* device bytes a plan may hold; 0 = 80% of free memory. A plan is
+                            accepted from two slots of rows of its largest BCC beside the graph
+                            on; more lets it run more sources and passes at once */
   int32_t rescale_exp;   /* BATCHED: rescale a level's path counts above 2^rescale_exp; 0 = 900.
                             Lower values only exercise the scaling path (tests). */
   int32_t plain_core;    /* BATCHED: BCCs whose core (the vertices off degree-2 chains) has fewer
@@ -63,20 +65,22 @@ typedef struct bc_opts {
                             the work directly on every run. The stream must be capturable
                             (not the legacy NULL stream). */
   int32_t plain_ctas_per_sm; /* per-source schedule: CTAs (sources in flight) per SM; 0 = four
-                            256-thread CTAs, fewer and larger when their rows do not fit the
-                            workspace budget; 8 or 16 = that many CTAs of 128 or 64 threads
-                            (more sources in flight for deep, narrow BCCs), with the same
-                            fallback; other values are rejected */
+                            256-thread CTAs on the whole BCC, fewer and larger when their rows
+                            do not fit the workspace budget, and 64 to 512 threads by the width
+                            of the levels on contracted BCCs; 4, 8 or 16 = that many CTAs of
+                            256, 128 or 64 threads (more sources in flight for deep, narrow
+                            BCCs), with the same fallback; other values are rejected */
   int32_t lazy_tables;   /* 1 (default): a one-shot bc_run_bccs_units call builds the multi-source
                             slot, seed and arming tables of the passes it runs only (and the
                             source order up to the last of them); 0 = of every pass (the same
-                            BC, bit for bit) */
+                            BC, bit for bit, unless device memory limits how many passes
+                            run as one) */
   int32_t tile_max;      /* BATCHED: BCCs routed away from multi-source passes run on the
                             small-BCC schedule (a CTA per range of sources of one BCC, its CSR
-                            slice staged in shared memory by a bulk copy, one warp per source)
-                            when they have at most tile_max vertices, fit shared memory and
-                            cannot overflow FP64 path counts; the others use the per-source
-                            schedule. 0 = as large as shared memory allows, -1 = off.
+                            slice staged in shared memory by a bulk copy, a warp, a group of
+                            threads or the CTA per source) when they have at most tile_max
+                            vertices, fit shared memory and cannot overflow FP64 path counts;
+                            the others use the per-source schedule. 0 = as large as shared memory allows, -1 = off.
                             No reference counterpart (one source per CTA for every BCC,
                             Codes/begin_gpupgm.cu:52-65). */
   int32_t wait_limit_ms; /* limit of one device-side wait (the multi-source kernel's grid
